@@ -236,3 +236,32 @@ def test_device_matrix_rejects_bad_layout(pkg):
         pkg.mst_device(d.data_ptr(), 12, 10)
     with pytest.raises(pkg.TchError, match="aligned"):
         pkg.neighbors_device(d.data_ptr() + 2, 16, 10, 3)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [33, 255, 1023, 1024, 1025, 2056, 3001])
+@pytest.mark.parametrize("order", ["random", "falling", "equal", "few"])
+def test_gpu_neighbors_block_edges(pkg, n, order):
+    """Row lengths around the kernel's 1 024-column blocks, rows whose every
+    value is a new minimum, all-equal rows and rows of few distinct values (the
+    column decides), the padding set to 0; k at both ends of its range."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(n)
+    if order == "random":
+        H = rng.integers(0, 65536, size=(n, n))
+    elif order == "falling":
+        H = np.broadcast_to(65535 - np.arange(n), (n, n)).copy()
+    elif order == "equal":
+        H = np.full((n, n), 65535)
+    else:
+        H = rng.integers(0, 3, size=(n, n))
+    H = H.astype(np.uint16)
+    ld = (n + 7) // 8 * 8
+    full = np.zeros((n, ld), np.uint16)
+    full[:, :n] = H
+    np.fill_diagonal(full[:, :n], 0)
+    d = torch.from_numpy(full.view(np.int16)).cuda()
+    for k in (1, 10, 32):
+        idx, dist = pkg.neighbors_device(d.data_ptr(), ld, n, k)
+        wi, wd = oracle.neighbors(H, k)
+        assert (idx == wi).all() and (dist == wd).all()
