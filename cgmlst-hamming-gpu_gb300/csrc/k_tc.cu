@@ -5,7 +5,7 @@
 // Operands (Fp4Operands): packed e2m1 rows [presence | one-hot | zeros], two
 // elements per byte, 0 or +1.0 in the `pos` copy, which is read as A, and 0
 // or +1.0 / -1.0 (one-hot part) in the `neg` copy, which is read as B.  One
-// output tile (128 rows i x 224 columns j) is
+// output tile (256 rows i x 240 columns j) is
 //
 //   D = pos_i . neg_j^T  =  P Pt - O Ot
 //
@@ -19,19 +19,40 @@
 // have no negate bit, hence the second operand copy with the one-hot sign in
 // the data.
 //
-// CTA = 10 warps, one CTA per SM, persistent over the stripe's tiles (upper
-// triangle only, or every tile of a rectangle):
-//   warp 0    TMA producer   5-stage ring of (A 128 x 128 B, B 224 x 128 B)
-//   warp 1    MMA issuer     4 x tcgen05.mma (K = 64 elements) per stage into
-//                            one of two 224-column TMEM accumulators
+// A CTA pair (cluster of two, tcgen05 cta_group::2) per tile, 10 warps per
+// CTA, one CTA per SM, persistent over the stripe's tiles (upper triangle
+// only, or every tile of a rectangle):
+//   warp 0    TMA producer   7-stage ring of (A 128 x 128 B, B 120 x 128 B): each
+//                            CTA its 128 rows of A and its half of the columns'
+//                            rows, completing on the first CTA's barrier
+//   warp 1    MMA issuer     (first CTA) 4 x tcgen05.mma (M 256, N 240, K = 64
+//                            elements) per stage into one of two 240-column
+//                            accumulators in both CTAs' TMEM
 //   warps 2-9 epilogue       two per TMEM lane quarter, one per column half:
-//                            tcgen05.ld 16 columns -> int -> minus the dense
-//                            rare counts (16-byte loads issued before the TMEM
-//                            read) -> u16 -> 32-byte stores from registers
-// TMEM: accumulators at columns 0 and 256, the scale factors (1.0, written
+//                            tcgen05.ld 32 columns x 16 rows -> u16 pairs -> quad
+//                            transpose -> minus the dense rare counts (loaded
+//                            while the MMAs run) -> 16-byte stores
+// TMEM: accumulators at columns 0 and 240, the scale factors (1.0, written
 // once by the epilogue warps before the first MMA) in columns 480-511.
-// Tiles are visited in raster groups of 8 row blocks, column-major inside a
-// group, so that the CTAs running at the same time share A and B tiles in L2.
+// Tiles are visited in raster groups of row blocks, column-major inside a
+// group, so that the pairs running at the same time share A and B tiles in L2.
+//
+// What bounds it: a stage's MMAs take 480 cycles (16 384 MACs per cycle and
+// SM, the probe's rate) and its operands 496 (31 KB per CTA at the 64 bytes a
+// cycle that an SM takes in from L2), so the pass runs at both limits inside a
+// tile (503 cycles per stage measured) plus about 1.9 us per tile, half of it
+// the tile's rare counts coming in.  One CTA per tile (128 x 224) takes 44 KB
+// for 448 cycles of MMAs and stops at 0.61 of the probe's rate: 8.46 ms for the
+// triangle of 63 005 long-tail profiles at tau 1 024, 6.24 ms in pairs (0.83).
+// Three more things were needed to get there, each measured on that triangle
+// (8.38 ms as a plain pair):
+//   - the next stage's barrier is looked at before a stage's MMAs are issued:
+//     a wait between two stages costs the issuing thread about 130 cycles that
+//     the tensor pipe then idles (8.38 -> 8.18);
+//   - the epilogue touches whole 64-byte row pieces (8.18 -> 7.60, below);
+//   - producer and issuer run under elect.sync (7.60 -> 6.27): under
+//     `lane == 0` an MMA takes 86 cycles to issue, as its descriptors move
+//     through vector registers.
 //
 // Every mbarrier wait is bounded (about 2 s of %globaltimer); on a timeout the
 // CTA records DEVERR_TIMEOUT, stops issuing work, drains what it issued,
@@ -39,6 +60,7 @@
 
 #include <cuda.h>
 #include <cudaTypedefs.h>
+#include <limits.h>
 
 #include "tc_ptx.cuh"
 #include "tch_internal.cuh"
@@ -46,30 +68,37 @@
 namespace tch {
 namespace {
 
-constexpr int BM = 128;             // tile rows (TMEM lanes)
-constexpr int BN = 224;             // tile columns (MMA N)
+constexpr int BM = 128;             // tile rows of one CTA (TMEM lanes)
+constexpr int PM = 2 * BM;          // tile rows of a CTA pair (MMA M)
+constexpr int BN = 240;             // tile columns (MMA N)
+constexpr int BH = BN / 2;          // column rows staged by each CTA of the pair
 constexpr int BK = 128;             // bytes of K per stage: one 128-byte swizzle row, 256 elements
-constexpr int STAGES = 5;
+constexpr int STAGES = 7;
 constexpr int A_BYTES = BM * BK;    // 16 KB
-constexpr int B_BYTES = BN * BK;    // 28 KB
-constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
+constexpr int B_BYTES = BH * BK;    // 15 KB
+constexpr int STAGE_BYTES = A_BYTES + B_BYTES;  // of one CTA
 constexpr int EPI_WARPS = 8;
 constexpr int THREADS = 64 + 32 * EPI_WARPS;
-constexpr int ACC_STRIDE = 256;     // TMEM columns from one accumulator to the next
+constexpr int ACC_STRIDE = BN;      // TMEM columns from one accumulator to the next
 constexpr int SF_COL = 480;         // 32 TMEM columns of scale factors
 constexpr int TMEM_COLS = 512;
-constexpr int CHUNK = 16;           // accumulator columns per tcgen05.ld
-constexpr int WARP_CHUNKS = BN / CHUNK / 2;  // chunks per epilogue warp (its column half)
-constexpr int GROUP_M = 8;          // row blocks per raster group (default; TCH_TC_GROUP overrides)
+constexpr int CHUNK = 32;           // accumulator columns per tcgen05.ld (16 lanes each)
+constexpr int CHUNKS = (BN + CHUNK - 1) / CHUNK;
+constexpr int WARP_CHUNKS = (CHUNKS + 1) / 2;  // chunks of the first column half (the second has the rest)
+// 128-row blocks per raster group (TCH_TC_GROUP overrides): 63 005 profiles, tau
+// 1 024: 4 -> 6.82 ms, 8 -> 6.31, 16 -> 6.24, 32 -> 6.40
+constexpr int GROUP_M = 16;
 constexpr int BAR_BYTES = 256;
 constexpr int SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + BAR_BYTES;
 static_assert(SMEM_BYTES <= 232448, "shared memory per CTA");
-static_assert(BN % (2 * CHUNK) == 0 && BN <= ACC_STRIDE && ACC_STRIDE + BN <= SF_COL, "TMEM layout");
+static_assert(BN % 16 == 0 && BN <= 256 && ACC_STRIDE + BN <= SF_COL && SF_COL + 32 <= TMEM_COLS, "TMEM layout");
+static_assert(ACC_STRIDE + CHUNKS * CHUNK <= TMEM_COLS, "the last chunk's loads stay inside TMEM");
+static_assert(BH % 8 == 0, "whole 8-row swizzle atoms per CTA");
 static_assert(A_BYTES % 1024 == 0 && B_BYTES % 1024 == 0, "stages stay 1024-byte aligned (128-byte swizzle)");
 
 using namespace ptx;
 
-// Row blocks per raster group: GROUP_M unless TCH_TC_GROUP gives another
+// 128-row blocks per raster group: GROUP_M unless TCH_TC_GROUP gives another
 // count in [1, 256].  Larger groups read the column side of the operand fewer
 // times (once per group) at the cost of a larger row-side working set.
 int group_row_blocks() {
@@ -82,8 +111,11 @@ int group_row_blocks() {
     return g;
 }
 
+// Row blocks of a pair (PM rows) per raster group, from the schedule's 128-row blocks.
+int pair_group(int group) { return std::max(1, (group > 0 ? std::min(group, 256) : group_row_blocks()) / 2); }
+
 // ---------------------------------------------------------------- tile order
-// Row block bi covers rows a_r0 + BM bi .. + BM of the A operand, column block
+// Row block bi covers rows a_r0 + PM bi .. + PM of the A operand, column block
 // bj columns c0 + BN bj .. + BN.  In a triangle (c0 = r0) the row block's
 // first column block is the one holding its first diagonal cell.
 struct TileSpace {
@@ -93,11 +125,11 @@ struct TileSpace {
 };
 
 __host__ __device__ __forceinline__ int first_col(const TileSpace& ts, int bi) {
-    return ts.rect ? 0 : (BM * bi) / BN;
+    return ts.rect ? 0 : (PM * bi) / BN;
 }
 // The last row block present in column block bj.
 __host__ __device__ __forceinline__ int last_row(const TileSpace& ts, int bj) {
-    const int r = ((bj + 1) * BN - 1) / BM;
+    const int r = ((bj + 1) * BN - 1) / PM;
     return ts.rect || r > ts.nbi - 1 ? ts.nbi - 1 : r;
 }
 
@@ -146,7 +178,7 @@ __device__ bool tile_coords(const TileSpace& ts, const GroupTable& gt, int t, in
 }
 
 // Tensor maps of every K chunk: A boxes (128 rows of the pos copy) and B
-// boxes (224 rows of the neg copy), and the 128-byte K blocks of each chunk.
+// boxes (BH rows of the neg copy), and the 128-byte K blocks of each chunk.
 struct TcMaps {
     CUtensorMap a[kMaxKChunks];
     CUtensorMap b[kMaxKChunks];
@@ -211,8 +243,35 @@ __device__ bool tile_coords_one_group(const TileSpace& ts, int t, int* bi_out, i
     return true;
 }
 
+// Lane quads transpose 4 x 4 words: lane c of a quad gives w[r] to lane r and
+// ends with word r from lane r of the quad, its own in place.
+__device__ __forceinline__ void quad_transpose(uint32_t (&w)[4], int c) {
+    constexpr unsigned ALL = 0xFFFFFFFFu;
+    const bool odd = c & 1, upper = c & 2;
+    const uint32_t s0 = __shfl_xor_sync(ALL, odd ? w[0] : w[1], 1);
+    const uint32_t s1 = __shfl_xor_sync(ALL, odd ? w[2] : w[3], 1);
+    if (odd) w[0] = s0, w[2] = s1;
+    else w[1] = s0, w[3] = s1;
+    const uint32_t t0 = __shfl_xor_sync(ALL, upper ? w[0] : w[2], 2);
+    const uint32_t t1 = __shfl_xor_sync(ALL, upper ? w[1] : w[3], 2);
+    if (upper) w[0] = t0, w[1] = t1;
+    else w[2] = t0, w[3] = t1;
+}
+
+// Two exact fp32 integers as u16 halves of a word (modulo 2^16): added to 1.5
+// x 2^23, an integer of magnitude below 2^22 stands in the low mantissa bits.
+// `bad` is set when one is not an integer.
+__device__ __forceinline__ uint32_t pack_u16(uint32_t v0, uint32_t v1, bool* bad) {
+    constexpr float kShift = 12582912.0f;
+    const float f0 = __uint_as_float(v0), f1 = __uint_as_float(v1);
+    const float x0 = __fadd_rn(f0, kShift), x1 = __fadd_rn(f1, kShift);
+    *bad |= (__fsub_rn(x0, kShift) != f0) | (__fsub_rn(x1, kShift) != f1);
+    return __byte_perm(__float_as_uint(x0), __float_as_uint(x1), 0x5410);
+}
+
 template <bool MULTI>
-__global__ void __launch_bounds__(THREADS, 1) tc_stripe_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
+    tc_stripe_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* stage_a = smem;
@@ -223,15 +282,17 @@ __global__ void __launch_bounds__(THREADS, 1) tc_stripe_kernel(const __grid_cons
     uint64_t* tfull = bars + 2 * STAGES;       // 2
     uint64_t* tempty = bars + 2 * STAGES + 2;  // 2
     uint64_t* drain = bars + 2 * STAGES + 4;   // 1
-    uint32_t* tmem_slot = (uint32_t*)(bars + 2 * STAGES + 5);
+    uint64_t* scales = bars + 2 * STAGES + 5;  // 1: the scale factors stand in both CTAs' TMEM
+    uint32_t* tmem_slot = (uint32_t*)(bars + 2 * STAGES + 6);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
 
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    // this CTA's tiles: every gridDim.x-th one (in a batch the CTAs then work
+    // this pair's tiles: every (gridDim.x / 2)-th one (in a batch the CTAs then work
     // on the same set's tiles at the same time, which keeps its operand in L2:
     // one contiguous range of tiles per CTA, split by work, measured 43.1 ms
     // against 34.1 ms on 512 sets)
-    const int t_begin = blockIdx.x, t_end = p.num_tiles, t_step = gridDim.x;
+    const int t_begin = blockIdx.x / 2, t_end = p.num_tiles, t_step = gridDim.x / 2;
+    const uint32_t rank = cluster_rank();  // 0: the CTA that issues the pair's MMAs
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; s++) {
@@ -240,9 +301,10 @@ __global__ void __launch_bounds__(THREADS, 1) tc_stripe_kernel(const __grid_cons
         }
         for (int a = 0; a < 2; a++) {
             mbar_init(&tfull[a], 1);
-            mbar_init(&tempty[a], EPI_WARPS);
+            mbar_init(&tempty[a], 2 * EPI_WARPS);  // both CTAs' epilogues
         }
         mbar_init(drain, 1);
+        mbar_init(scales, 8);  // four warps of each CTA
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         if (!MULTI)
@@ -252,28 +314,20 @@ __global__ void __launch_bounds__(THREADS, 1) tc_stripe_kernel(const __grid_cons
             }
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                      "r"(TMEM_COLS)
                      : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
     tc_fence_before();
-    __syncthreads();
+    __syncwarp();
+    cluster_sync();  // barriers initialised and TMEM allocated in both CTAs
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    // scale factors 1.0 in every lane of the 32 scale-factor columns, one
-    // epilogue warp per lane quarter, before any MMA reads them
-    if (warp >= 2 && warp < 6) {
-        tmem_fill32(tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + SF_COL, 0x01010101u * kUe8m0One);
-        tmem_wait_st();
-    }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
 
     if (warp == 0) {
         // ------------------------------------------------------------ producer
-        if (lane == 0) {
+        if (elect_one()) {
             int s = 0;
             uint32_t ph = 0;
             bool ok = true;
@@ -288,14 +342,14 @@ __global__ void __launch_bounds__(THREADS, 1) tc_stripe_kernel(const __grid_cons
                 const int* kbls = maps.kblocks;
                 if (!MULTI) {
                     if (!tile_coords(p.ts, p.gt, t, &bi, &bj)) break;
-                    y_a = p.r0 + bi * BM;
+                    y_a = p.r0 + bi * PM;
                     y_b = p.c0 + bj * BN;
                     kblocks = p.kblocks;
                 } else {
                     const int job = __ldg(p.tile_job + t);
                     const TcJob& jb = p.jobs[job];
                     if (!tile_coords_one_group(jb.ts, t - jb.tile0, &bi, &bj)) break;
-                    y_a = bi * BM;
+                    y_a = bi * PM;
                     y_b = bj * BN;
                     kblocks = jb.kblocks;
                     ma = p.jmaps + jb.map0;
@@ -306,13 +360,17 @@ __global__ void __launch_bounds__(THREADS, 1) tc_stripe_kernel(const __grid_cons
                         last_job = job;
                     }
                 }
+                y_a += (int)rank * BM;  // this CTA's half of the rows and of the columns
+                y_b += (int)rank * BH;
                 int ch = 0, kbl = 0;  // K chunk and block inside it
                 int kbl_end = kbls[0];
                 for (int kb = 0; kb < kblocks; kb++) {
                     if (!mbar_wait(&empty[s], ph ^ 1, abort_flag, p.err)) { ok = false; break; }
-                    mbar_expect_tx(&full[s], STAGE_BYTES);
-                    tma_load_2d(ma + ch, &full[s], stage_a + s * A_BYTES, kbl * BK, y_a);
-                    tma_load_2d(mb + ch, &full[s], stage_b + s * B_BYTES, kbl * BK, y_b);
+                    // both CTAs' loads complete on the issuing CTA's barrier
+                    if (rank == 0) mbar_expect_tx(&full[s], 2 * STAGE_BYTES);
+                    const uint32_t bar = peer_addr(&full[s], 0);
+                    tma_load_2d_pair(ma + ch, bar, stage_a + s * A_BYTES, kbl * BK, y_a);
+                    tma_load_2d_pair(mb + ch, bar, stage_b + s * B_BYTES, kbl * BK, y_b);
                     if (++kbl == kbl_end) {
                         kbl = 0;
                         if (++ch < kMaxKChunks) kbl_end = kbls[ch];
@@ -328,8 +386,8 @@ __global__ void __launch_bounds__(THREADS, 1) tc_stripe_kernel(const __grid_cons
                     if (!mbar_wait(&empty[s], ph ^ 1, abort_flag, p.err)) break;
                     if (++s == STAGES) s = 0, ph ^= 1;
                 }
-            } else {
-                // abort: let the loads already issued land before the CTA exits
+            } else if (rank == 0) {
+                // abort: let the loads already issued land before the pair exits
                 for (int q = 0; q < STAGES; q++)
                     if (issued[q]) {
                         const unsigned long long t0 = gtimer();
@@ -340,34 +398,41 @@ __global__ void __launch_bounds__(THREADS, 1) tc_stripe_kernel(const __grid_cons
         __syncwarp();
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
-            const uint32_t idesc = make_idesc_mx(kE2M1, 1, BM, BN);
+        if (rank == 0 && elect_one()) {
+            const uint32_t idesc = make_idesc_mx(kE2M1, 1, PM, BN);
             const uint32_t sf = tmem_base + SF_COL;
             int s = 0, acc = 0;
             uint32_t ph = 0, aph = 0;
-            bool ok = true;
+            bool ready = false;  // stage s is known to hold its operands
+            bool ok = mbar_wait(scales, 0, abort_flag, p.err);
+            tc_fence_after();
             for (int t = t_begin; ok && t < t_end; t += t_step) {
                 const int kblocks = MULTI ? p.jobs[__ldg(p.tile_job + t)].kblocks : p.kblocks;
                 if (!mbar_wait(&tempty[acc], aph ^ 1, abort_flag, p.err)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + (uint32_t)(acc * ACC_STRIDE);
                 for (int kb = 0; kb < kblocks; kb++) {
-                    if (!mbar_wait(&full[s], ph, abort_flag, p.err)) { ok = false; break; }
+                    if (!ready && !mbar_wait(&full[s], ph, abort_flag, p.err)) { ok = false; break; }
                     tc_fence_after();
                     const uint32_t a0 = smem_u32(stage_a + s * A_BYTES), b0 = smem_u32(stage_b + s * B_BYTES);
+                    // look at the next stage's barrier before this stage's MMAs are
+                    // issued: the look's latency then hides behind them instead of
+                    // leaving the tensor pipe idle between two stages
+                    const int sn = s + 1 == STAGES ? 0 : s + 1;
+                    ready = mbar_peek(&full[sn], sn ? ph : ph ^ 1);
 #pragma unroll
                     for (int k = 0; k < BK / 32; k++)
-                        tc_mma_mxf4(d_tmem, sw128_desc(a0 + 32 * k), sw128_desc(b0 + 32 * k), idesc, sf, sf,
-                                    (kb | k) ? 1u : 0u);
-                    tc_commit(&empty[s]);  // stage free once these MMAs have read it
+                        tc_mma_mxf4_pair(d_tmem, sw128_desc(a0 + 32 * k), sw128_desc(b0 + 32 * k), idesc, sf, sf,
+                                         (kb | k) ? 1u : 0u);
+                    tc_commit_pair(&empty[s]);  // stage free in both CTAs once these MMAs have read it
                     if (++s == STAGES) s = 0, ph ^= 1;
                 }
                 if (!ok) break;
-                tc_commit(&tfull[acc]);  // accumulator ready for the epilogue
+                tc_commit_pair(&tfull[acc]);  // accumulator ready for both epilogues
                 if (++acc == 2) acc = 0, aph ^= 1;
             }
             // every MMA issued by this thread has completed before TMEM is freed
-            tc_commit(drain);
+            tc_commit_pair_local(drain);
             const unsigned long long t0 = gtimer();
             while (!mbar_test(drain, 0) && gtimer() - t0 < WAIT_NS) {}
         }
@@ -376,15 +441,25 @@ __global__ void __launch_bounds__(THREADS, 1) tc_stripe_kernel(const __grid_cons
         // ------------------------------------------------------------ epilogue
         const int q = warp & 3;           // TMEM lanes [32 q, 32 q + 32) belong to this warp
         const int half = (warp - 2) / 4;  // column half of the tile
+        if (half == 0) {
+            // scale factors 1.0 in every lane of the 32 scale-factor columns, one
+            // warp per lane quarter; the first loads are under way meanwhile
+            tmem_fill32(tmem_base + ((uint32_t)(q * 32) << 16) + SF_COL, 0x01010101u * kUe8m0One);
+            tmem_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(peer_addr(scales, 0));
+        }
         int acc = 0;
         uint32_t aph = 0;
-        int bad = 0;
+        bool bad = false;
         for (int t = t_begin; t < t_end; t += t_step) {
             int bi, bj;
             int n = p.n, r0 = p.r0, c0 = p.c0, iend = p.r0 + p.rows, vec_store = p.vec_store;
             const uint16_t* rdense = p.rdense;
             uint16_t* out = p.out;
             size_t ldo = p.ldo, ldr = p.ldr;
+            const bool tri = MULTI || !p.ts.rect;
             if (!MULTI) {
                 if (!tile_coords(p.ts, p.gt, t, &bi, &bj)) break;
             } else {
@@ -401,64 +476,82 @@ __global__ void __launch_bounds__(THREADS, 1) tc_stripe_kernel(const __grid_cons
                 ldr = jb.ldr;
             }
             const bool dense = rdense != nullptr;
-            const int i = r0 + bi * BM + q * 32 + lane;  // this lane's row
+            // A chunk is 32 columns of the warp's 32 rows, in two passes of 16 rows.
+            // After the quad transpose a lane holds 8 consecutive columns (16
+            // bytes) of rows l / 4 and l / 4 + 8 of the pass, so one 16-byte access
+            // of the warp covers 64 bytes of 8 rows.  (With a row per lane, as
+            // 32x32b loads give it, each access touched 32 rows; the L1 then spent
+            // 7 700 of a tile's cycles on them, which the MMAs need to fetch
+            // operands: 8.18 ms against 7.60 on the 63 005-profile triangle.)
+            const int i0 = r0 + bi * PM + (int)rank * BM + q * 32;  // the warp's first row
             const int j0 = c0 + bj * BN;
-            const bool row_ok = i < iend;
-            const size_t orow = (size_t)(i - r0) * ldo;
-            const size_t rrow = (size_t)(i - r0) * ldr;
+            const int c_begin = half * WARP_CHUNKS, c_end = half ? CHUNKS : WARP_CHUNKS;
+            const int quad = lane & 3, lrow = lane >> 2;
+            // a chunk with no cell above the diagonal is skipped
+            const int j_min = tri ? i0 + 2 - CHUNK : INT_MIN;
+            // columns of this tile and set: [j0, j_end)
+            const int j_end = min(n, j0 + BN);
+            // the rare counts, fetched while the MMAs of the tile run; a row of the
+            // block is at least up(n - c0, 8) wide, so a live 16 bytes is in bounds
+            uint4 r4[WARP_CHUNKS][4];
+#pragma unroll
+            for (int cc = 0; cc < WARP_CHUNKS; cc++) {
+                const int cb = j0 + (c_begin + cc) * CHUNK, j = cb + 8 * quad;
+#pragma unroll
+                for (int g = 0; g < 4; g++) {
+                    const int i = i0 + 8 * g + lrow;
+                    r4[cc][g] = make_uint4(0, 0, 0, 0);
+                    if (dense && c_begin + cc < c_end && cb >= j_min && i < iend && j < j_end)
+                        r4[cc][g] = __ldg(reinterpret_cast<const uint4*>(rdense + (size_t)(i - r0) * ldr + (j - c0)));
+                }
+            }
             if (!mbar_wait(&tfull[acc], aph, abort_flag, p.err)) break;
             tc_fence_after();
             const uint32_t tbase = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * ACC_STRIDE);
-#pragma unroll 1
+#pragma unroll
             for (int cc = 0; cc < WARP_CHUNKS; cc++) {
-                const int c = half * WARP_CHUNKS + cc;
+                const int c = c_begin + cc;
                 const int cb = j0 + c * CHUNK;  // first column of the chunk
-                const bool live = row_ok && cb < n;
-                // this row's rare counts for the chunk (32 bytes), fetched before
-                // the accumulator read so the two overlap; a row of the block is
-                // at least up(n - c0, 16) wide, so a live chunk is in bounds
-                uint4 r4[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
-                if (dense && live) {
-                    const uint4* src = reinterpret_cast<const uint4*>(rdense + rrow + (size_t)(cb - c0));
-                    r4[0] = __ldg(src);
-                    r4[1] = __ldg(src + 1);
+                const bool skip = c >= c_end || cb < j_min || cb >= j_end;  // uniform over the warp
+                uint32_t v[2][16];
+                if (!skip) {
+                    tmem_ld_16x256b_x4(tbase + (uint32_t)(c * CHUNK), v[0]);
+                    tmem_ld_16x256b_x4(tbase + (16u << 16) + (uint32_t)(c * CHUNK), v[1]);
+                    tmem_wait_ld();
                 }
-                uint32_t v[16];
-                tmem_ld16(tbase + (uint32_t)(c * CHUNK), v);
-                tmem_wait_ld();
                 if (cc == WARP_CHUNKS - 1) {  // this warp's part of the accumulator is read: hand it back
                     tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(&tempty[acc]);
+                    if (lane == 0) mbar_arrive_cluster(peer_addr(&tempty[acc], 0));
                 }
-                uint32_t w[8];
+                if (skip) continue;
+                const int j = cb + 8 * quad;
 #pragma unroll
-                for (int e = 0; e < 8; e++) {
-                    const float f0 = __uint_as_float(v[2 * e]), f1 = __uint_as_float(v[2 * e + 1]);
-                    int x0 = __float2int_rn(f0), x1 = __float2int_rn(f1);
-                    bad |= (__int2float_rn(x0) != f0) | (__int2float_rn(x1) != f1);
-                    const uint4& r = r4[e / 4];
-                    const uint32_t rw = (e % 4 == 0) ? r.x : (e % 4 == 1) ? r.y : (e % 4 == 2) ? r.z : r.w;
-                    x0 -= (int)(rw & 0xFFFF);
-                    x1 -= (int)(rw >> 16);
-                    w[e] = (uint32_t)(x0 & 0xFFFF) | ((uint32_t)(x1 & 0xFFFF) << 16);
-                }
-                if (live) {
-                    uint16_t* dst = out + orow + (size_t)(cb - c0);
-                    if (cb + CHUNK <= n) {
-                        if (vec_store) {
-                            uint4* d4 = reinterpret_cast<uint4*>(dst);
-                            d4[0] = make_uint4(w[0], w[1], w[2], w[3]);
-                            d4[1] = make_uint4(w[4], w[5], w[6], w[7]);
-                        } else {
-                            uint32_t* d1 = reinterpret_cast<uint32_t*>(dst);
+                for (int g = 0; g < 4; g++) {  // rows 8 g + l / 4 of the warp's 32
+                    const int i = i0 + 8 * g + lrow;
+                    uint32_t w[4];
 #pragma unroll
-                            for (int e = 0; e < 8; e++) d1[e] = w[e];
-                        }
+                    for (int r = 0; r < 4; r++) {
+                        bool odd = false;
+                        w[r] = pack_u16(v[g / 2][4 * r + 2 * (g & 1)], v[g / 2][4 * r + 2 * (g & 1) + 1], &odd);
+                        bad |= odd && cb + 8 * r < j0 + BN;  // columns past BN are not this accumulator's
+                    }
+                    quad_transpose(w, quad);
+                    const uint4 rr = r4[cc][g];
+                    w[0] = __vsub2(w[0], rr.x);
+                    w[1] = __vsub2(w[1], rr.y);
+                    w[2] = __vsub2(w[2], rr.z);
+                    w[3] = __vsub2(w[3], rr.w);
+                    if (i >= iend || j >= j_end) continue;
+                    uint16_t* dst = out + (size_t)(i - r0) * ldo + (j - c0);
+                    if (vec_store && j + 8 <= n) {
+                        *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
                     } else {
 #pragma unroll
-                        for (int e = 0; e < CHUNK; e++)
-                            if (cb + e < n) dst[e] = (uint16_t)(w[e / 2] >> (16 * (e & 1)));
+                        for (int e = 0; e < 8; e += 2) {
+                            if (j + e + 1 < n) *reinterpret_cast<uint32_t*>(dst + e) = w[e / 2];
+                            else if (j + e < n) dst[e] = (uint16_t)w[e / 2];
+                        }
                     }
                 }
             }
@@ -467,11 +560,14 @@ __global__ void __launch_bounds__(THREADS, 1) tc_stripe_kernel(const __grid_cons
         if (bad) atomicOr(p.err, DEVERR_OVERFLOW);
     }
 
+    // neither CTA leaves (or frees TMEM) while the other may still use its
+    // barriers, its operand stages or its accumulators
     tc_fence_before();
-    __syncthreads();
+    __syncwarp();
+    cluster_sync();
     if (warp == 1) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS)
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS)
                      : "memory");
     }
 }
@@ -522,22 +618,22 @@ cudaError_t launch_one(const Fp4Operands& A, const Fp4Operands& B, const uint16_
     if ((a.ldo & 1) || ((uintptr_t)a.out & 3)) return cudaErrorInvalidValue;
     if (R && ((ldr & 7) || ((uintptr_t)R & 15))) return cudaErrorInvalidValue;
     TcMaps maps;
+    TcParams p;
     maps.n = ka.n;
     for (int c = 0; c < ka.n; c++) {
         const int wc = ka.width_of(c);
         if (wc <= 0 || (wc % BK)) return cudaErrorInvalidValue;
-        if (!make_map(&maps.a[c], ka.p[c], A.n_rows, wc, BM) || !make_map(&maps.b[c], kb.p[c], B.n_rows, wc, BN))
+        if (!make_map(&maps.a[c], ka.p[c], A.n_rows, wc, BM) || !make_map(&maps.b[c], kb.p[c], B.n_rows, wc, BH))
             return cudaErrorInvalidValue;
         maps.kblocks[c] = wc / BK;
     }
-    TcParams p;
     p.n = a.n;
     p.r0 = a.r0;
     p.c0 = a.rect ? 0 : a.r0;
     p.rows = a.rows;
     p.kblocks = A.kb / BK;
-    p.ts.gs = a.group > 0 ? std::min(a.group, 256) : group_row_blocks();
-    p.ts.nbi = (a.rows + BM - 1) / BM;
+    p.ts.gs = pair_group(a.group);
+    p.ts.nbi = (a.rows + PM - 1) / PM;
     p.ts.rect = a.rect ? 1 : 0;
     p.ts.nbj = (a.n - p.c0 + BN - 1) / BN;
     const long long tiles = tiles_in(p.ts, 0, p.ts.nbi);
@@ -564,7 +660,7 @@ cudaError_t launch_one(const Fp4Operands& A, const Fp4Operands& B, const uint16_
     p.jmaps = nullptr;
     p.tile_job = nullptr;
     if (p.num_tiles == 0) return cudaSuccess;
-    const int grid = std::min(p.num_tiles, std::max(num_sms, 1));
+    const int grid = 2 * std::min(p.num_tiles, std::max(num_sms / 2, 1));
     tc_stripe_kernel<false><<<grid, THREADS, SMEM_BYTES, st>>>(maps, p);
     return cudaGetLastError();
 }
@@ -599,10 +695,10 @@ cudaError_t tc_batch_prepare(const std::vector<TcBatchItem>& items, int num_sms,
         }
         for (int c = 0; c < ka.n; c++) {
             CUtensorMap m;
-            if (!make_map(&m, kb.p[c], A.n_rows, kb.width_of(c), BN)) return cudaErrorInvalidValue;
+            if (!make_map(&m, kb.p[c], A.n_rows, kb.width_of(c), BH)) return cudaErrorInvalidValue;
             mh.push_back(m);
         }
-        jb.ts.nbi = (it.n + BM - 1) / BM;
+        jb.ts.nbi = (it.n + PM - 1) / PM;
         jb.ts.nbj = (it.n + BN - 1) / BN;
         jb.ts.gs = jb.ts.nbi;
         jb.ts.rect = 0;
@@ -623,7 +719,7 @@ cudaError_t tc_batch_prepare(const std::vector<TcBatchItem>& items, int num_sms,
     plan->njobs = (int)jobs.size();
     plan->num_tiles = tile0;
     if (jobs.empty()) return cudaSuccess;
-    plan->grid = std::max(1, std::min(tile0, num_sms));
+    plan->grid = 2 * std::max(1, std::min(tile0, num_sms / 2));
     cudaError_t e = cudaMalloc(&plan->d_jobs, jobs.size() * sizeof(TcJob));
     if (e == cudaSuccess) e = cudaMalloc(&plan->d_maps, mh.size() * sizeof(CUtensorMap));
     if (e == cudaSuccess) e = cudaMalloc(&plan->d_tile_job, tile_job.size() * sizeof(int));
@@ -673,8 +769,7 @@ cudaError_t launch_tc_stripe(const Fp4Operands& ops, const Fp4Operands* bops, co
     const Fp4Operands& b = bops ? *bops : ops;
     // one launch covers at most MAX_GROUPS raster groups of rows; a taller
     // stripe runs as consecutive sub-stripes writing into the same output
-    const int group = a.group > 0 ? std::min(a.group, 256) : group_row_blocks();
-    const int max_rows = MAX_GROUPS * group * BM;
+    const int max_rows = MAX_GROUPS * pair_group(a.group) * PM;
     for (int done = 0; done < a.rows; done += max_rows) {
         StripeArgs s = a;
         s.r0 = a.r0 + done;

@@ -267,3 +267,28 @@ def test_k_chunked_operand(tch):
             tch.Solver.from_encoding(enc, kernel="tc_f4")
     finally:
         tch.set_max_chunk_bytes(0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [2, 119, 121, 129, 239, 240, 241, 255, 257, 481, 513, 737])
+def test_tile_edges(pkg, n):
+    """Sizes around the tile pass's 256 x 240 tiles (128 rows and 120 columns
+    per CTA), whole triangles and stripes from odd first rows, outputs with
+    16-byte rows and with rows that start between two 16-byte boundaries."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(n)
+    L = 61
+    A = rng.integers(0, 9, size=(n, L)).astype(np.uint64)
+    A[:, :20] = rng.integers(0, max(2, n // 3), size=(n, 20))
+    want = oracle.hamming(pkg.dense_ranks(A)[0])
+    with pkg.Solver.from_calls(A, tau=6) as s:
+        for r0, rows in ((0, n), (1, n - 1), (n // 3, n // 2), (n - 1, 1)):
+            for ldo in ((n - r0 + 7) // 8 * 8, (n - r0 + 7) // 8 * 8 + 2):
+                d = torch.full((max(rows, 1), ldo), -1, dtype=torch.int16, device="cuda:0")
+                s.stripe(r0, rows, d.data_ptr(), ldo, torch.cuda.current_stream().cuda_stream)
+                s.check()
+                got = d.cpu().numpy().view(np.uint16)
+                for r in range(min(rows, n - r0)):
+                    i = r0 + r
+                    np.testing.assert_array_equal(got[r, r + 1:n - r0], want[i, i + 1:])
+                    assert (got[r, n - r0:] == 0xFFFF).all()  # nothing past the row's last column
