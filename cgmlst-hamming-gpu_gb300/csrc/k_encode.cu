@@ -207,10 +207,11 @@ __global__ void group_fill_kernel(const uint16_t* __restrict__ x, int n, int L, 
 }
 
 // One CTA per rare group: rows are distinct, so a row's place is the number
-// of smaller rows in the group.  groups holds (first, end, locus) triples;
+// of smaller rows in the group.  groups holds (first, end, locus) triples; the
+// rows go to sorted16 when given, else to sorted;
 // mpos (optional, n x L) receives every row's own index in `sorted`.
 __global__ void group_sort_kernel(const uint64_t* __restrict__ groups, const uint32_t* __restrict__ members,
-                                  uint32_t* sorted, uint32_t* mpos, int L) {
+                                  uint32_t* sorted, uint16_t* sorted16, uint32_t* mpos, int L) {
     const uint64_t g0 = groups[3 * blockIdx.x], g1 = groups[3 * blockIdx.x + 1];
     const int locus = (int)groups[3 * blockIdx.x + 2];
     const uint32_t g = (uint32_t)(g1 - g0);
@@ -238,7 +239,8 @@ __global__ void group_sort_kernel(const uint64_t* __restrict__ groups, const uin
         for (int q = 0; q < 4; q++) {
             const uint32_t e = e0 + q * blockDim.x + threadIdx.x;
             if (e < g) {
-                sorted[g0 + r[q]] = mine[q];
+                if (sorted16) sorted16[g0 + r[q]] = (uint16_t)mine[q];
+                else sorted[g0 + r[q]] = mine[q];
                 if (mpos) mpos[(size_t)mine[q] * L + locus] = (uint32_t)(g0 + r[q]);
             }
         }
@@ -248,9 +250,10 @@ __global__ void group_sort_kernel(const uint64_t* __restrict__ groups, const uin
 // Partner runs of every row (one warp per row, loci in order): the members
 // after the row's own entry in each of its rare groups, when there are any.
 // Pass 0 writes each row's run count; pass 1 the runs' first members, their
-// exclusive item prefix within the row, and the row's item total.
+// piece prefix and end within the row, and the row's total (RareGroups; `piece`
+// members to a piece).
 __global__ void row_runs_kernel(const uint16_t* __restrict__ x, int n, int L, const uint64_t* __restrict__ cnt_off,
-                                const uint64_t* __restrict__ goff, const uint32_t* __restrict__ mpos, int pass,
+                                const uint64_t* __restrict__ goff, const uint32_t* __restrict__ mpos, int piece, int pass,
                                 uint32_t* count, const uint64_t* __restrict__ roff, uint32_t* rlo, uint32_t* rpre,
                                 uint32_t* rtot) {
     const int lane = threadIdx.x & 31;
@@ -270,7 +273,8 @@ __global__ void row_runs_kernel(const uint16_t* __restrict__ x, int n, int L, co
             }
             const unsigned has = __ballot_sync(0xFFFFFFFFu, len > 0);
             if (pass) {
-                uint32_t inc = len;  // inclusive warp scan of the run lengths
+                const uint32_t pieces = len ? (lo + len - 1) / piece - lo / piece + 1 : 0;
+                uint32_t inc = pieces;  // inclusive warp scan of the runs' pieces
 #pragma unroll
                 for (int d = 1; d < 32; d <<= 1) {
                     const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, inc, d);
@@ -279,14 +283,14 @@ __global__ void row_runs_kernel(const uint16_t* __restrict__ x, int n, int L, co
                 if (len) {
                     const uint64_t q = base + nrun + __popc(has & ((1u << lane) - 1u));
                     rlo[q] = lo;
-                    rpre[q] = items + inc - len;
+                    rpre[q] = (items + inc - pieces) << 3 | (lo + len - 1) % piece;
                 }
                 items += __shfl_sync(0xFFFFFFFFu, inc, 31);
             }
             nrun += __popc(has);
         }
         if (lane == 0) {
-            if (pass) rtot[i] = items;
+            if (pass) rtot[i] = items << 3;
             else count[i] = nrun;
         }
     }
@@ -406,6 +410,7 @@ struct TauRow {
     double r = 0, cells = 0;  // rare pairs, cells in rare groups
     double sq = 0;            // sum of squared counts of the alleles that are not frequent
     double kb = 0, mem = 0, t = 0;
+    double feature_t = 0;     // the estimate as the learned model's feature (its training rates)
     bool fits = false;
 };
 
@@ -455,10 +460,12 @@ std::vector<TauRow> tau_rows(const std::vector<uint32_t>& cnt_flat, const std::v
         if (dense) {  // ranks, own positions, group members, row runs (a stripe's counts come later)
             w.mem = (double)rows * w.kb + nl * 6.0 + 12.0 * w.cells + 12.0 * n;
             w.t = pairs * w.kb / m.gemm_rate + w.r / m.dense_rate;
+            w.feature_t = pairs * w.kb / m.feature_gemm_rate + w.r / m.feature_dense_rate;
             w.fits = w.mem <= (double)free_bytes && w.cells < 4.0e9;
         } else {
             w.mem = (double)rows * w.kb + 4.0 * (w.r + n + 1.0) + 2.0 * (double)n * (double)up((size_t)n, 8) / 4;
             w.t = pairs * w.kb / m.gemm_rate + w.r / m.rare_rate;
+            w.feature_t = pairs * w.kb / m.feature_gemm_rate + w.r / m.rare_rate;
             w.fits = w.mem <= (double)free_bytes && w.r < 4.0e9;
         }
         out.push_back(w);
@@ -512,7 +519,7 @@ void tau_features(const std::vector<TauRow>& rows, const std::vector<uint32_t>& 
                 t->feats.push_back((float)log1p(w.r));
                 t->feats.push_back((float)log1p(w.cells));
                 t->feats.push_back((float)log(pairs * w.kb));
-                t->feats.push_back((float)log(std::max(w.t, 1e-9)));
+                t->feats.push_back((float)log(std::max(w.feature_t, 1e-9)));
                 t->feats.push_back((float)(sub ? log((double)sub / std::max(n, 1)) : 0.0));
                 t->feats.push_back((float)log((double)grp));
             }
@@ -598,7 +605,7 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
     unsigned long long* keys = nullptr;
     uint32_t *cnts = nullptr, *nd = nullptr, *list_slots = nullptr, *cnt_flat = nullptr, *gfill = nullptr;
     uint32_t *members = nullptr, *sorted = nullptr, *row_count = nullptr, *base_d = nullptr, *mpos = nullptr;
-    uint16_t* rank_slot = nullptr;
+    uint16_t *rank_slot = nullptr, *sorted16 = nullptr;
     unsigned long long* list_keys = nullptr;
     uint64_t *cnt_off_d = nullptr, *goff_d = nullptr, *groups_d = nullptr, *start64 = nullptr;
     int32_t* col_d = nullptr;
@@ -771,7 +778,13 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
         // ---- 5: rare groups, sorted
         const size_t ngroups = groups.size() / 3;
         TCH_CK(e, dalloc(&members, n_members, &tmp_bytes));
-        TCH_CK(e, dalloc(&sorted, n_members, &tmp_bytes));
+        // row runs where they are used (triangle solves) and their packed prefix
+        // holds; two-byte members where every row index fits
+        const int piece = n <= 65536 ? 8 : 4;
+        const bool runs = dense_rare && !query_maps && n > 1 && (double)L * (n / piece + 2.0) < 536870912.0;
+        const bool narrow = runs && n <= 65536;
+        if (narrow) TCH_CK(e, dalloc(&sorted16, n_members + 8, &tmp_bytes));  // the last piece is loaded whole
+        else TCH_CK(e, dalloc(&sorted, n_members + 4, &tmp_bytes));
         TCH_CK(e, dalloc(&gfill, off_h[L], &tmp_bytes));
         TCH_CK(e, cudaMemset(gfill, 0, std::max<uint64_t>(off_h[L], 1) * 4));
         if (dense_rare) {  // cells in no rare group keep the sentinel: the rare counts skip them
@@ -785,16 +798,16 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
             TCH_CK(e, cudaGetLastError());
             for (size_t g0 = 0; g0 < ngroups; g0 += 65535) {
                 const unsigned gcount = (unsigned)std::min<size_t>(65535, ngroups - g0);
-                group_sort_kernel<<<gcount, 256>>>(groups_d + 3 * g0, members, sorted, mpos, L);
+                group_sort_kernel<<<gcount, 256>>>(groups_d + 3 * g0, members, sorted, sorted16, mpos, L);
                 TCH_CK(e, cudaGetLastError());
             }
         }
 
         mark("rare groups");
-        if (dense_rare && !query_maps && n > 1) {  // the partner runs of every row, for triangle solves
+        if (runs) {  // the partner runs of every row, for triangle solves
             TCH_CK(e, dalloc(&row_count, (size_t)n, &tmp_bytes));
             const int rgrid = (int)std::min<size_t>(((size_t)n + 7) / 8, (size_t)sms * 16);
-            row_runs_kernel<<<rgrid, 256>>>(out->x, n, L, cnt_off_d, goff_d, mpos, 0, row_count, nullptr, nullptr,
+            row_runs_kernel<<<rgrid, 256>>>(out->x, n, L, cnt_off_d, goff_d, mpos, piece, 0, row_count, nullptr, nullptr,
                                             nullptr, nullptr);
             TCH_CK(e, cudaGetLastError());
             std::vector<uint32_t> rc_h((size_t)n);
@@ -808,7 +821,7 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
             TCH_CK(e, dalloc(&out->rpre, std::max<uint64_t>(acc, 1), &out->bytes));
             TCH_CK(e, dalloc(&out->rtot, (size_t)n, &out->bytes));
             TCH_CK(e, cudaMemcpy(out->roff, roff_h.data(), ((size_t)n + 1) * 8, cudaMemcpyHostToDevice));
-            row_runs_kernel<<<rgrid, 256>>>(out->x, n, L, cnt_off_d, goff_d, mpos, 1, nullptr, out->roff, out->rlo,
+            row_runs_kernel<<<rgrid, 256>>>(out->x, n, L, cnt_off_d, goff_d, mpos, piece, 1, nullptr, out->roff, out->rlo,
                                             out->rpre, out->rtot);
             TCH_CK(e, cudaGetLastError());
             mark("row runs");
@@ -820,8 +833,9 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
             out->cnt_off = cnt_off_d;
             out->goff = goff_d;
             out->members = sorted;
+            out->members16 = sorted16;
             out->mpos = mpos;
-            out->bytes += ((size_t)L + 1) * 8 + (off_h[L] + 1) * 8 + n_members * 4 + (size_t)n * L * 4;
+            out->bytes += ((size_t)L + 1) * 8 + (off_h[L] + 1) * 8 + n_members * (narrow ? 2 : 4) + (size_t)n * L * 4;
             if (query_maps) {  // what new profiles need to be encoded like these
                 out->slot_ids = reinterpret_cast<uint64_t*>(slot_ids);
                 out->col = col_d;
@@ -834,6 +848,7 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
             cnt_off_d = nullptr;
             goff_d = nullptr;
             sorted = nullptr;
+            sorted16 = nullptr;
             mpos = nullptr;
             goto done;
         }
@@ -878,12 +893,12 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
     }
 done:
     cudaFree(err_d); cudaFree(nd); cudaFree(cnt_off_d); cudaFree(cnt_flat); cudaFree(col_d); cudaFree(base_d);
-    cudaFree(goff_d); cudaFree(members); cudaFree(sorted); cudaFree(gfill); cudaFree(groups_d); cudaFree(row_count);
+    cudaFree(goff_d); cudaFree(members); cudaFree(sorted); cudaFree(sorted16); cudaFree(gfill); cudaFree(groups_d); cudaFree(row_count);
     cudaFree(start64); cudaFree(mpos); cudaFree(slot_ids);
     return 0;
 fail:
     cudaFree(err_d); cudaFree(nd); cudaFree(cnt_off_d); cudaFree(cnt_flat); cudaFree(col_d); cudaFree(base_d);
-    cudaFree(goff_d); cudaFree(members); cudaFree(sorted); cudaFree(gfill); cudaFree(groups_d); cudaFree(row_count);
+    cudaFree(goff_d); cudaFree(members); cudaFree(sorted); cudaFree(sorted16); cudaFree(gfill); cudaFree(groups_d); cudaFree(row_count);
     cudaFree(start64); cudaFree(keys); cudaFree(cnts); cudaFree(rank_slot); cudaFree(list_keys); cudaFree(list_slots);
     cudaFree(mpos); cudaFree(slot_ids);
     free_device_encoding(out);
@@ -898,6 +913,7 @@ void free_device_encoding(DeviceEncoding* d) {
     cudaFree(d->cnt_off);
     cudaFree(d->goff);
     cudaFree(d->members);
+    cudaFree(d->members16);
     cudaFree(d->mpos);
     cudaFree(d->roff);
     cudaFree(d->rlo);
@@ -916,6 +932,7 @@ void free_device_encoding(DeviceEncoding* d) {
     d->start = d->js = nullptr;
     d->cnt_off = d->goff = nullptr;
     d->members = d->mpos = nullptr;
+    d->members16 = nullptr;
 }
 
 }  // namespace tch

@@ -9,15 +9,22 @@
 // into a u16 block laid out like the output, which the tensor-core epilogue
 // subtracts with 16-byte loads: no pair list is ever materialised.
 //
-// One CTA per stripe row (persistent over the rows).  The counters of the
-// row's columns sit in shared memory as u16 pairs (65536 columns per pass),
-// each partner adds 1 with a shared atomic, and the finished row is written
-// out with coalesced 16-byte stores.  The partner runs of up to 2048 loci are
+// A CTA per stripe row (persistent over the rows).  The counters of the row's
+// columns sit in shared memory as u16 pairs (65 536 columns per pass), each
+// partner adds 1 with a shared atomic, and the finished row is written out with
+// coalesced 16-byte stores.  Triangle solves read the rows' partner runs as the
+// encoder laid them out (rare_runs_kernel); where there are none (queries, and
+// stripes wider than one pass) the runs of up to 2048 loci are found per locus,
 // laid end to end by a block-wide scan of their lengths and cut into 32 equal
-// parts, one per warp, so every warp of the CTA has the same number of
-// partners whatever the group sizes are; a warp walks its part run by run
-// with its lanes on consecutive members (coalesced loads, up to eight in
-// flight per lane).
+// parts, one per warp (rare_dense_kernel, rare_query_kernel).
+//
+// What bounds rare_runs_kernel: the shared atomics.  Random columns put 3.4
+// lanes of a warp on one bank, so an atomic takes 3.4 of the L1's data cycles,
+// and with the member loads and the run cursor those are 75-79 % busy (ncu,
+// 12 011 x 5 000 founders); at the margin it counts 2.0e12 pairs/s, of 6.7 per
+// cycle and SM.  63 005 x 1 142 long-tail, tau 1 024 (3.4e9 pairs): 2.83 ms,
+// 4.72 before, when each member went through the run cursor by itself and one
+// 1 024-thread CTA per SM took every row; 0.6 ms of it is the 4 GB block.
 
 #include <climits>
 
@@ -37,6 +44,12 @@ constexpr int RD_WORDS = 32768;          // u32 counter words in shared memory (
 inline int counter_words(size_t width) { return (int)std::min<size_t>(RD_WORDS, width / 2); }
 template <int T>
 inline int rd_smem(int cwords) { return cwords * 4 + (2 * T + 1) * 4 + 2 * T * 4 + 64 * 4; }
+// Runs of a row staged at a time by the row-run kernels.
+template <int T>
+constexpr int kCap = T >= 256 ? 2 * T : 512;
+constexpr int kMinCap = 512;
+template <int T>
+constexpr int runs_smem(int cwords, int cap = kCap<T>) { return cwords * 4 + (2 * cap + 2 + 64) * 4; }
 constexpr unsigned FULL = 0xFFFFFFFFu;
 
 __device__ __forceinline__ uint64_t lower_bound_m(const uint32_t* __restrict__ m, uint64_t lo, uint64_t hi,
@@ -237,32 +250,175 @@ __device__ __forceinline__ void count_runs(uint32_t* cnt, uint32_t* pre, uint32_
     walk_part(cnt, pre, run, (int)tot[1], e_begin, e_end, members, wb, lane);
 }
 
-// Row i's partners from its precomputed runs (RareGroups::roff ..), counted
-// at column j - wb: up to 2T runs at a time are copied into pre / run
-// (coalesced), their items cut into one equal part per warp and walked.  The
-// row's partners must all lie in this pass's columns.  Called by all threads
-// of the CTA after the counters are zeroed (it synchronises them).
-template <int T>
-__device__ __forceinline__ void count_row_runs(uint32_t* cnt, uint32_t* pre, uint32_t* run, const RareGroups& g, int i,
-                                               int wb) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    constexpr int NWARPS = T / 32;
-    const uint64_t q0 = g.roff[i];
-    const uint32_t nrun = (uint32_t)(g.roff[i + 1] - q0);
-    for (uint32_t c0 = 0; c0 < nrun; c0 += 2 * T) {
-        const uint32_t cn = min(2u * T, nrun - c0);
-        __syncthreads();  // the zeroing, or the previous group of runs' readers
-        for (uint32_t t = tid; t < cn; t += T) {
-            pre[t] = __ldg(g.rpre + q0 + c0 + t);
-            run[t] = __ldg(g.rlo + q0 + c0 + t);
+// ---- precomputed row runs (RareGroups::roff ..), 16 bytes of members per lane
+//
+// A row's partners are runs of consecutive members; a run covers whole 16-byte
+// pieces of the member array but for its first and last one (8 members of two
+// bytes when every row index fits them, else 4 of four).  The pieces of a row's
+// runs, laid end to end, are cut into one equal part per warp, and a lane takes
+// a whole piece: finding its run, the load and the two end masks cost about 30
+// instructions per piece, and each member five and its shared atomic.  Walking
+// the members one by one, every one with its own look at the run cursor, took
+// 26 instructions per atomic.
+
+template <class M>
+constexpr int kPiece = 16 / (int)sizeof(M);  // members per piece
+
+// Shared add under a predicate (as an `if` each one became a branch: 19
+// instructions per atomic).
+__device__ __forceinline__ void red_add_if(uint32_t cond, uint32_t addr, uint32_t v) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %0, 0;\n\t@p red.shared.add.u32 [%1], %2;\n\t}\n" ::"r"(cond),
+                 "r"(addr), "r"(v)
+                 : "memory");
+}
+
+// Where column j's u16 counter lies: half (j - odd) & 1 of the word at base + 4
+// ((j - odd) >> 1), odd = 1 when the counters start at an odd column.
+struct Counters {
+    uint32_t base;
+    uint32_t odd;
+};
+__device__ __forceinline__ Counters counters_at(const void* cnt, int first_col) {
+    Counters c;
+    c.odd = (uint32_t)first_col & 1u;
+    c.base = (uint32_t)__cvta_generic_to_shared(cnt) - 2u * ((uint32_t)first_col - c.odd);
+    return c;
+}
+
+// The members of a piece that `mask` names, counted.
+__device__ __forceinline__ void count_piece(const Counters& c, const uint4& v, uint32_t mask, uint16_t) {
+    uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    const uint32_t base = c.base;
+    if (c.odd) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) w[q] = __vsub2(w[q], 0x00010001u);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        red_add_if(mask & (1u << (2 * q)), base + ((w[q] << 1) & 0x1FFFCu), (w[q] & 1u) * 0xFFFFu + 1u);
+        red_add_if(mask & (2u << (2 * q)), base + ((w[q] >> 15) & 0x1FFFCu), max(w[q] & 0x10000u, 1u));
+    }
+}
+__device__ __forceinline__ void count_piece(const Counters& c, const uint4& v, uint32_t mask, uint32_t) {
+    const uint32_t w[4] = {v.x - c.odd, v.y - c.odd, v.z - c.odd, v.w - c.odd};
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+        red_add_if(mask & (1u << q), c.base + ((w[q] << 1) & ~3u), (w[q] & 1u) * 0xFFFFu + 1u);
+}
+
+// Pieces [e_begin, e_end) of nr staged runs, by one warp.  run[q].x = (first piece
+// of run q among the row's) << 3 | place of its last member in its last piece,
+// run[nr].x >> 3 bounds the last run; run[q].y = its first member.
+template <class M>
+__device__ __forceinline__ void walk_pieces(const Counters& c, const uint2* run, int nr, uint32_t e_begin,
+                                            uint32_t e_end, const M* __restrict__ members,
+                                            int lane) {
+    constexpr int G = kPiece<M>;
+    if (e_begin >= e_end) return;
+    int p = 0;  // the run holding e_begin
+    for (int hi = nr; hi - p > 1;) {
+        const int m = (p + hi) >> 1;
+        if ((run[m].x >> 3) <= e_begin) p = m; else hi = m;
+    }
+    uint2 cur = run[p], next = run[p + 1];  // this lane's current run and the one after it
+    for (uint32_t e0 = e_begin; e0 < e_end; e0 += 64) {
+        uint4 v[2];
+        uint32_t mask[2];
+#pragma unroll
+        for (int u = 0; u < 2; u++) {  // both loads before the first atomic
+            const uint32_t e = e0 + (uint32_t)(32 * u + lane);
+            mask[u] = 0;
+            v[u] = make_uint4(0, 0, 0, 0);
+            if (e < e_end) {
+                while (e >= next.x >> 3) {  // next run (run[nr].x >> 3 = the end of all > e bounds it)
+                    cur = next;
+                    next = run[++p + 1];
+                }
+                const uint32_t k = e - (cur.x >> 3);
+                mask[u] = (1u << G) - 1u;
+                if (k == 0) mask[u] &= ~0u << (cur.y % G);
+                if (e + 1 == next.x >> 3) mask[u] &= (2u << (cur.x & 7u)) - 1u;
+                v[u] = __ldg(reinterpret_cast<const uint4*>(members) + (cur.y / G + k));
+            }
         }
-        if (tid == 0) pre[cn] = c0 + cn < nrun ? __ldg(g.rpre + q0 + c0 + cn) : __ldg(g.rtot + i);
-        __syncthreads();
-        const uint32_t base = pre[0], total = pre[cn] - base;
+        count_piece(c, v[0], mask[0], M());
+        if (e0 + 32 < e_end) count_piece(c, v[1], mask[1], M());
+    }
+}
+
+// Copies runs [c0, c0 + cn) of the row whose runs are [q0, q1) into `run`, and
+// the piece after the last of them into run[cn].x.
+template <int T>
+__device__ __forceinline__ void stage_runs(const RareGroups& g, int i, uint64_t q0, uint64_t q1, uint32_t c0,
+                                           uint32_t cap, uint2* run) {
+    const uint32_t nrun = (uint32_t)(q1 - q0), cn = min(cap, nrun - c0);
+    for (uint32_t t = threadIdx.x; t < cn; t += T) {
+        run[t] = make_uint2(__ldg(g.rpre + q0 + c0 + t), __ldg(g.rlo + q0 + c0 + t));
+    }
+    if (threadIdx.x == 0)
+        run[cn] = make_uint2(c0 + cn < nrun ? __ldg(g.rpre + q0 + c0 + cn) : __ldg(g.rtot + i), 0u);
+}
+
+// Counts every run of row i; the first `cap` of them are staged and visible to
+// all threads.  Called by all threads of the CTA.
+template <int T, class M>
+__device__ __forceinline__ void count_staged_row(const Counters& c, uint2* run, const RareGroups& g, const M* members, int i, uint64_t q0, uint64_t q1, uint32_t cap) {
+    constexpr int NWARPS = T / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t nrun = (uint32_t)(q1 - q0);
+    for (uint32_t c0 = 0; c0 < nrun; c0 += cap) {
+        if (c0) {
+            __syncthreads();  // the previous runs' readers
+            stage_runs<T>(g, i, q0, q1, c0, cap, run);
+            __syncthreads();
+        }
+        const uint32_t cn = min(cap, nrun - c0);
+        const uint32_t first = run[0].x >> 3, total = (run[cn].x >> 3) - first;
         const uint32_t part = (total + NWARPS - 1) / NWARPS;
-        const uint32_t e_begin = base + min(total, (uint32_t)warp * part);
-        const uint32_t e_end = base + min(total, (uint32_t)warp * part + part);
-        walk_part(cnt, pre, run, (int)cn, e_begin, e_end, g.members, wb, lane);
+        const uint32_t e_begin = first + min(total, (uint32_t)warp * part);
+        const uint32_t e_end = first + min(total, (uint32_t)warp * part + part);
+        walk_pieces<M>(c, run, (int)cn, e_begin, e_end, members, lane);
+    }
+}
+
+// Rows [row_begin, row_end) of a stripe whose rows have precomputed runs, each in
+// one pass of the counters: `cwords` of them hold row_begin's width, the widest.
+// Persistent over the rows: the finished row is written out and its counters
+// cleared in one sweep, which also stages the next row's runs.
+template <int T, class M>
+__global__ void __launch_bounds__(T, T >= 1024 ? 1 : 1536 / T)
+    rare_runs_kernel(const RareGroups g, int r0, int row_begin, int row_end, uint16_t* __restrict__ R, size_t ldr,
+                     int cend, int cwords, int cap) {
+    extern __shared__ uint4 smem_rd[];
+    uint32_t* cnt = reinterpret_cast<uint32_t*>(smem_rd);
+    uint2* run = reinterpret_cast<uint2*>(cnt + cwords);  // cap + 1
+    const M* members = sizeof(M) == 2 ? reinterpret_cast<const M*>(g.members16) : reinterpret_cast<const M*>(g.members);
+    const int tid = threadIdx.x;
+    int r = row_begin + (int)blockIdx.x;
+    if (r >= row_end) return;
+    for (int w = tid; w < cwords / 4; w += T) smem_rd[w] = make_uint4(0, 0, 0, 0);
+    uint64_t q0 = g.roff[r0 + r], q1 = g.roff[r0 + r + 1];
+    if (q1 > q0) stage_runs<T>(g, r0 + r, q0, q1, 0, cap, run);
+    for (;;) {
+        const int next = r + (int)gridDim.x;
+        uint64_t n0 = 0, n1 = 0;
+        if (next < row_end) n0 = g.roff[r0 + next], n1 = g.roff[r0 + next + 1];
+        __syncthreads();  // counters zero, runs staged
+        const int cbeg = r0 + (r & ~(kRareDenseAlign - 1));  // first column of the row's diagonal tile
+        count_staged_row<T, M>(counters_at(cnt, cbeg), run, g, members, r0 + r, q0, q1, (uint32_t)cap);
+        __syncthreads();  // row counted
+        if (n1 > n0) stage_runs<T>(g, r0 + next, n0, n1, 0, cap, run);
+        uint4* dst = reinterpret_cast<uint4*>(R + (size_t)r * ldr + (size_t)(cbeg - r0));
+        const int nq = (cend - cbeg) >> 3;
+        const bool more = next < row_end;
+        for (int w = tid; w < nq; w += T) {
+            dst[w] = smem_rd[w];
+            if (more) smem_rd[w] = make_uint4(0, 0, 0, 0);
+        }
+        if (!more) break;
+        r = next;
+        q0 = n0;
+        q1 = n1;
     }
 }
 
@@ -284,9 +440,10 @@ __global__ void __launch_bounds__(T, 1024 / T)
                       int cwords) {
     extern __shared__ uint4 smem_rd[];
     uint32_t* cnt = reinterpret_cast<uint32_t*>(smem_rd);
-    uint32_t* pre = cnt + cwords;
-    uint32_t* run = pre + (2 * T) + 1;
-    uint32_t* wsum = run + (2 * T);
+    uint32_t* wsum = cnt + cwords;          // 64: per-warp totals of the scans
+    uint2* runs = reinterpret_cast<uint2*>(wsum + 64);   // kCap<T> + 1 staged row runs, or
+    uint32_t* run = wsum + 64;              // kCap<T>: first member of each run found per locus
+    uint32_t* pre = run + kCap<T>;          // kCap<T> + 1: exclusive prefix of the run lengths
     const int tid = threadIdx.x;
     for (int gr = blockIdx.x; gr < total_rows; gr += gridDim.x) {
         const RareJob& jb = jobs[__ldg(row_job + gr)];
@@ -297,8 +454,11 @@ __global__ void __launch_bounds__(T, 1024 / T)
         const int nq = (jb.cend - cbeg) >> 3;
         for (int w = tid; w < nq; w += T) smem_rd[w] = make_uint4(0, 0, 0, 0);
         const uint32_t jlo = (uint32_t)(i + 1), jhi = (uint32_t)n;
-        if (g.roff) {  // the row's precomputed runs
-            count_row_runs<T>(cnt, pre, run, g, i, cbeg);
+        if (g.members16) {  // the row's precomputed runs
+            const uint64_t q0 = g.roff[i], q1 = g.roff[i + 1];
+            if (q1 > q0) stage_runs<T>(g, i, q0, q1, 0, kCap<T>, runs);
+            __syncthreads();
+            count_staged_row<T, uint16_t>(counters_at(cnt, cbeg), runs, g, g.members16, i, q0, q1, kCap<T>);
         } else {
             for (int kc = 0; jlo < jhi && kc < L; kc += (2 * T)) {
                 const int k0 = kc + 2 * tid;
@@ -330,10 +490,7 @@ __global__ void __launch_bounds__(T, 1024 / T)
     // with every locus in one scan (L <= 2T) a thread keeps the same two
     // loci for all rows: their count offsets stay in registers and the next
     // row's ranks and positions are fetched while this row is counted
-    // the rows' precomputed runs, when there are any and every row's partners
-    // fit one counter pass; otherwise the runs are found per locus
-    const bool row_runs = g.roff != nullptr && cend - r0 <= 2 * cwords;
-    const bool one_chunk = !row_runs && L <= (2 * T);
+    const bool one_chunk = L <= (2 * T);
     uint64_t co0 = 0, co1 = 0;
     if (one_chunk) {
         if (2 * tid < L) co0 = g.cnt_off[2 * tid];
@@ -352,8 +509,7 @@ __global__ void __launch_bounds__(T, 1024 / T)
             const int nq = (we - wb) >> 3;  // uint4 of counters (8 columns each); we - wb is a multiple of 256
             for (int w = tid; w < nq; w += T) smem_rd[w] = make_uint4(0, 0, 0, 0);
             const uint32_t jlo = (uint32_t)max(wb, i + 1), jhi = (uint32_t)min(we, n);
-            if (row_runs) count_row_runs<T>(cnt, pre, run, g, i, wb);
-            for (int kc = 0; !row_runs && jlo < jhi && kc < L; kc += (2 * T)) {
+            for (int kc = 0; jlo < jhi && kc < L; kc += (2 * T)) {
                 // this thread's two loci, then a block-wide exclusive scan of the run lengths
                 const int k0 = kc + 2 * tid;
                 uint32_t lo0 = 0, lo1 = 0, l0 = 0, l1 = 0;
@@ -519,7 +675,7 @@ cudaError_t rare_batch_prepare(const std::vector<RareBatchItem>& items, RareBatc
     bool& attr = attrs[current_device()];
     if (!attr) {
         e = cudaFuncSetAttribute(rare_batch_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 rd_smem<NT>(RD_WORDS));
+                                 runs_smem<NT>(RD_WORDS));
         if (e != cudaSuccess) return e;
         attr = true;
     }
@@ -532,7 +688,7 @@ cudaError_t launch_rare_batch(const RareBatchPlan& plan, int sms, cudaStream_t s
     // (the sets' widths and taus), and the block scheduler balances them
     (void)sms;
     const int grid = std::max(1, plan.total_rows);
-    rare_batch_kernel<NT><<<grid, NT, rd_smem<NT>(plan.cwords), st>>>(
+    rare_batch_kernel<NT><<<grid, NT, runs_smem<NT>(plan.cwords), st>>>(
         static_cast<const RareJob*>(plan.d_jobs), static_cast<const int*>(plan.d_row_job), plan.total_rows,
         plan.cwords);
     return cudaGetLastError();
@@ -545,43 +701,89 @@ void rare_batch_release(RareBatchPlan* plan) {
     plan->njobs = plan->total_rows = 0;
 }
 
+// Shared memory of one CTA when an SM holds `per_sm` of them (1 KB of it is the
+// system's).
+constexpr int runs_room(int per_sm) { return (227 * 1024) / per_sm - 1024; }
+
+// One launch of rare_runs_kernel over rows [ra, rb) of the stripe: `per_sm` CTAs
+// of T threads on an SM, as many of them as hold the widest row's counters; the
+// runs staged at a time take what is left, up to a row's most.
+template <int T, class M>
+static cudaError_t launch_runs(const RareGroups& g, int r0, int ra, int rb, uint16_t* R, size_t ldr, int cend,
+                               int per_sm, bool persistent, int sms, cudaStream_t st) {
+    const int cwords = (cend - r0 - (ra & ~(kRareDenseAlign - 1))) / 2;
+    while (per_sm > 1 && runs_smem<T>(cwords, kMinCap) > runs_room(per_sm)) per_sm--;
+    const int left = (runs_room(per_sm) - runs_smem<T>(cwords, 0)) / 8;
+    const int cap = std::max(std::min(left, (int)up((size_t)g.L, 32)), kMinCap);
+    const int grid = persistent ? std::min(per_sm * sms, rb - ra) : rb - ra;
+    rare_runs_kernel<T, M><<<grid, T, runs_smem<T>(cwords, cap), st>>>(g, r0, ra, rb, R, ldr, cend, cwords, cap);
+    return cudaGetLastError();
+}
+
+// The stripe's rows in bands of like width, each with as many CTAs per SM as
+// its counters leave room for: rows of 63 005 columns take the whole SM, those of
+// half the width share it in twos and threes.
+template <class M>
+static cudaError_t launch_rare_runs(const RareGroups& g, int r0, int rows, uint16_t* R, size_t ldr, int sms,
+                                    cudaStream_t st) {
+    const int width = (int)up((size_t)(g.n - r0), kRareDenseAlign), cend = r0 + width;
+    // widest row that leaves room for two CTAs on an SM
+    constexpr int kWide = (runs_room(2) - runs_smem<512>(0, kMinCap)) / 2 / kRareDenseAlign * kRareDenseAlign;
+    // narrow rows: a CTA of NT (128) threads each, so that many rows' chains of
+    // dependent steps overlap (5 000 profiles, tau 64: 0.039 ms, with 512 threads
+    // 0.060; from 8 192 columns on the two are alike)
+    constexpr int kNarrow = 8192;
+    cudaError_t e = cudaSuccess;
+    static bool attrs[kMaxDevices] = {};  // once per device (also keeps it out of graph captures)
+    bool& attr = attrs[current_device()];
+    if (!attr) {
+        const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
+        e = cudaFuncSetAttribute(rare_runs_kernel<1024, M>, at, runs_room(1));
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(rare_runs_kernel<512, M>, at, runs_room(1));
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(rare_runs_kernel<NT, M>, at, runs_room(1));
+        if (e != cudaSuccess) return e;
+        attr = true;
+    }
+    for (int ra = 0; ra < rows && e == cudaSuccess;) {
+        const int w = width - (ra & ~(kRareDenseAlign - 1));
+        // the end of the rows from ra on that are wider than `limit` columns
+        auto wider = [&](int limit) { return w <= limit ? ra : std::min(rows, width - limit); };
+        int rb;
+        if ((rb = wider(kWide)) > ra) {
+            e = launch_runs<1024, M>(g, r0, ra, rb, R, ldr, cend, 1, true, sms, st);
+        } else if ((rb = wider(28672)) > ra) {
+            e = launch_runs<512, M>(g, r0, ra, rb, R, ldr, cend, 2, true, sms, st);
+        } else if ((rb = wider(kNarrow)) > ra) {
+            e = launch_runs<512, M>(g, r0, ra, rb, R, ldr, cend, 3, true, sms, st);
+        } else {
+            rb = rows;
+            e = launch_runs<NT, M>(g, r0, ra, rb, R, ldr, cend, 8, false, sms, st);
+        }
+        ra = rb;
+    }
+    return e;
+}
+
 cudaError_t launch_rare_dense(const RareGroups& g, int r0, int rows, uint16_t* R, size_t ldr, int sms,
                               cudaStream_t st) {
     if (rows <= 0) return cudaSuccess;
     const size_t width = up((size_t)(g.n - r0), kRareDenseAlign);
     if (ldr < width || (ldr & 7) || ((uintptr_t)R & 15)) return cudaErrorInvalidValue;
+    // every row's precomputed runs, where the widest row fits one counter pass
+    if (g.roff && width <= (size_t)2 * RD_WORDS)
+        return g.members16 ? launch_rare_runs<uint16_t>(g, r0, rows, R, ldr, sms, st)
+                           : launch_rare_runs<uint32_t>(g, r0, rows, R, ldr, sms, st);
     static bool attrs[kMaxDevices] = {};  // once per device (also keeps it out of graph captures)
     bool& attr = attrs[current_device()];
     if (!attr) {
-        cudaError_t e = cudaFuncSetAttribute(rare_dense_kernel<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             rd_smem<1024>(RD_WORDS));
-
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(rare_dense_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     rd_smem<NT>(RD_WORDS));
+        const cudaError_t e = cudaFuncSetAttribute(rare_dense_kernel<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   rd_smem<1024>(RD_WORDS));
         if (e != cudaSuccess) return e;
         attr = true;
     }
     const int cwords = counter_words(width);
-    // a narrow stripe takes CTAs of NT (128) threads, one row each: eight fit on
-    // an SM, so eight rows' chains of dependent steps overlap, and solves that
-    // run side by side share the SMs.  Narrow rows carry little counting work,
-    // so their time is those chains: the 512-set batch (50-5 000 profiles each)
-    // took 17.4 ms with 128 threads per row and 18.5 ms with 256.
-    // TCH_RARE_SMALL_ROWS sets a row limit for it.
-    static int small_rows = -1;
-    if (small_rows < 0) {
-        const char* v = getenv("TCH_RARE_SMALL_ROWS");
-        small_rows = v ? std::max(0, atoi(v)) : INT_MAX;
-    }
-    if (rows < small_rows && width <= 8192) {
-        rare_dense_kernel<NT><<<std::max(1, rows), NT, rd_smem<NT>(cwords), st>>>(g, r0, rows, R, ldr,
-                                                                                   r0 + (int)width, cwords);
-    } else {
-        const int grid = std::max(1, std::min(rows, sms));
-        rare_dense_kernel<1024><<<grid, 1024, rd_smem<1024>(cwords), st>>>(g, r0, rows, R, ldr, r0 + (int)width,
-                                                                            cwords);
-    }
+    rare_dense_kernel<1024><<<std::max(1, std::min(rows, sms)), 1024, rd_smem<1024>(cwords), st>>>(
+        g, r0, rows, R, ldr, r0 + (int)width, cwords);
     return cudaGetLastError();
 }
 

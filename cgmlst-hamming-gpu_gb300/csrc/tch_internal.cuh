@@ -205,13 +205,18 @@ void tc_batch_release(TcBatchPlan* plan);
 // ---- k_encode.cu ------------------------------------------------------------------
 // Rates of the analytic tau model on this GPU.
 struct TauModel {
-    // pair x column MACs per second of the fp4 tile pass (63 005 x 1 142
-    // long-tail profiles: 3.0e15 at tau 1 024, 2.85e15 at 2 048)
-    double gemm_rate = 2.9e15;
+    // pair x column MACs per second of the fp4 tile pass, at the margin (63 005 x
+    // 1 142 long-tail profiles: 5.3e15 from tau 2 048 to 1 024, 4.7e15 on to 512)
+    double gemm_rate = 4.8e15;
     double rare_rate = 1.0e12;  // rare pairs per second of the pair-list counts (pair lists)
     // rare pairs per second of the dense rare-count build, at the margin (its
-    // fixed part, the u16 block written per stripe, does not depend on tau)
-    double dense_rate = 1.5e12;
+    // fixed part, the u16 block written per stripe, does not depend on tau):
+    // 2.0e12 on the same profiles, 1.5e12 on founder alleles' shorter runs
+    double dense_rate = 1.9e12;
+    // The rates behind the estimate that the learned model reads as a feature:
+    // those in force when its training sets were timed, unless they are set.
+    double feature_gemm_rate = 2.9e15;
+    double feature_dense_rate = 1.5e12;
 };
 
 // The rare alleles as groups of rows, kept on the device: the dense rare
@@ -221,12 +226,15 @@ struct RareGroups {
     const uint64_t* cnt_off = nullptr;  // L + 1: slot of (locus k, rank a) is cnt_off[k] + a
     const uint64_t* goff = nullptr;     // slots + 1: a rare group's rows are members[goff[q] .. goff[q+1])
     const uint32_t* members = nullptr;  // rows of every rare group (count >= 2), ascending per group
+    const uint16_t* members16 = nullptr;  // the same in two bytes (sets with row runs and n <= 65 536; members null)
     const uint32_t* mpos = nullptr;     // n x L: index in members of row i's own entry, kNoGroup outside groups
     int n = 0, L = 0;
     // Row runs (optional; null: found per locus from the arrays above): row i's
-    // partners are runs roff[i] .. roff[i + 1] - 1, in locus order; run q is
-    // members[rlo[q] ..) and its items start at rpre[q] within the row (an
-    // exclusive prefix), the row's last run ending at rtot[i].
+    // partners are runs roff[i] .. roff[i + 1] - 1, in locus order; run q starts
+    // at member rlo[q] and covers pieces of 16 bytes of the member array (8
+    // members of members16, or 4 of members); rpre[q] = (its first piece among
+    // the row's) << 3 | the place of its last member in its last piece, and
+    // rtot[i] = (the row's pieces) << 3.
     const uint64_t* roff = nullptr;
     const uint32_t* rlo = nullptr;
     const uint32_t* rpre = nullptr;
@@ -290,6 +298,7 @@ struct DeviceEncoding {
     uint64_t* cnt_off = nullptr;
     uint64_t* goff = nullptr;
     uint32_t* members = nullptr;
+    uint16_t* members16 = nullptr;  // in place of members (RareGroups)
     uint32_t* mpos = nullptr;
     // every row's partner runs (RareGroups::roff ..), built for triangle solves
     uint64_t* roff = nullptr;

@@ -149,6 +149,7 @@ struct tch_solver {
     uint64_t* gcnt_off = nullptr;
     uint64_t* ggoff = nullptr;
     uint32_t* gmembers = nullptr;
+    uint16_t* gmembers16 = nullptr;
     uint32_t* gmpos = nullptr;
     uint64_t* groff = nullptr;       // every row's partner runs
     uint32_t* grlo = nullptr;
@@ -185,6 +186,7 @@ void solver_free(tch_solver* s) {
     cudaFree(s->gcnt_off);
     cudaFree(s->ggoff);
     cudaFree(s->gmembers);
+    cudaFree(s->gmembers16);
     cudaFree(s->gmpos);
     cudaFree(s->groff);
     cudaFree(s->grlo);
@@ -392,6 +394,7 @@ static int solver_from_input(int device, int n, int L, const uint64_t* calls, co
         s->gcnt_off = enc.cnt_off;
         s->ggoff = enc.goff;
         s->gmembers = enc.members;
+        s->gmembers16 = enc.members16;
         s->gmpos = enc.mpos;
         s->groff = enc.roff;
         s->grlo = enc.rlo;
@@ -445,6 +448,7 @@ static RareGroups rare_groups(const tch_solver* s) {
     g.cnt_off = s->gcnt_off;
     g.goff = s->ggoff;
     g.members = s->gmembers;
+    g.members16 = s->gmembers16;
     g.mpos = s->gmpos;
     g.roff = s->groff;
     g.rlo = s->grlo;
@@ -1016,7 +1020,7 @@ int tch_set_max_chunk_bytes(size_t bytes) {
 
 int tch_set_dense_rare_rate(double rate) {
     if (!(rate > 0)) return 1;
-    g_tau_model.dense_rate = rate;
+    g_tau_model.dense_rate = g_tau_model.feature_dense_rate = rate;
     return 0;
 }
 
@@ -1027,7 +1031,7 @@ int tch_set_rare_term(int dense) {
 
 int tch_set_tau_model(double gemm_rate, double rare_rate) {
     if (!(gemm_rate > 0) || !(rare_rate > 0)) return 1;
-    g_tau_model.gemm_rate = gemm_rate;
+    g_tau_model.gemm_rate = g_tau_model.feature_gemm_rate = gemm_rate;
     g_tau_model.rare_rate = rare_rate;
     return 0;
 }

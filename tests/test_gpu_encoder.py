@@ -141,3 +141,33 @@ def test_wide_stripe_blocks(tch):
             ref = oracle.hamming_block(x, r0, r0 + rows, r0, n)
             for r in range(rows):
                 np.testing.assert_array_equal(got[r, r + 1: n - r0], ref[r, r + 1:])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [2, 7, 8, 9, 33, 255, 257, 600])
+@pytest.mark.parametrize("groups", ["pairs", "eights", "whole", "mixed"])
+def test_row_runs_piece_edges(pkg, n, groups):
+    """Rare groups of two rows, of about eight (one 16-byte piece of members),
+    of every row, and of all sizes, so that runs start, end and lie anywhere in
+    their pieces; more loci than runs are staged at a time; stripes whose
+    counters start at even and odd columns."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(n)
+    L = 1300
+    high = {"pairs": max(2, n // 2), "eights": max(2, n // 8), "whole": 2, "mixed": 0}[groups]
+    if high:
+        A = rng.integers(1, high, size=(n, L))
+    else:
+        A = rng.integers(1, rng.integers(2, n + 2, size=L) + 1, size=(n, L))
+    A[rng.random((n, L)) < 0.05] = 0
+    A = A.astype(np.uint64)
+    want = oracle.hamming(pkg.dense_ranks(A)[0])
+    with pkg.Solver.from_calls(A, tau=65536) as s:  # every allele rare
+        for r0 in (0, 1, n // 2):
+            rows, ldo = n - r0, (n - r0 + 7) // 8 * 8
+            d = torch.zeros((max(rows, 1), ldo), dtype=torch.int16, device="cuda:0")
+            s.stripe(r0, rows, d.data_ptr(), ldo, torch.cuda.current_stream().cuda_stream)
+            s.check()
+            got = d.cpu().numpy().view(np.uint16)
+            for r in range(rows):
+                np.testing.assert_array_equal(got[r, r + 1:rows], want[r0 + r, r0 + r + 1:])
