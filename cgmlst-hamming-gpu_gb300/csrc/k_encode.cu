@@ -296,6 +296,34 @@ __global__ void row_runs_kernel(const uint16_t* __restrict__ x, int n, int L, co
     }
 }
 
+// Where slot q's group (members [goff[q], goff[q + 1]), ascending) enters each
+// window of rows; one entry past the last slot closes the last window.
+__global__ void window_kernel(const uint64_t* __restrict__ goff, const uint32_t* __restrict__ members, uint64_t slots,
+                              int windows, uint32_t* wpos) {
+    const uint64_t total = slots * windows;
+    for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t <= total;
+         t += (uint64_t)gridDim.x * blockDim.x) {
+        if (t == total) {
+            wpos[t] = (uint32_t)goff[slots];
+            break;
+        }
+        const uint64_t q = t / windows;
+        const uint32_t key = (uint32_t)(t % windows) * kQueryWindow;
+        uint64_t lo = goff[q], hi = goff[q + 1];
+        while (lo < hi) {
+            const uint64_t mid = lo + (hi - lo) / 2;
+            if (members[mid] < key) lo = mid + 1; else hi = mid;
+        }
+        wpos[t] = (uint32_t)lo;
+    }
+}
+
+// members modulo 65 536 in two bytes.
+__global__ void narrow_members_kernel(const uint32_t* __restrict__ members, size_t count, uint16_t* out) {
+    for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < count; t += (size_t)gridDim.x * blockDim.x)
+        out[t] = (uint16_t)members[t];
+}
+
 __device__ __forceinline__ uint64_t lower_bound_rows(const uint32_t* __restrict__ a, uint64_t lo, uint64_t hi,
                                                      uint32_t key) {
     while (lo < hi) {
@@ -604,7 +632,7 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
     const int nk_max = (int)std::max<size_t>(1, std::min<size_t>((size_t)L, ((size_t)2 << 30) / per_locus));
     unsigned long long* keys = nullptr;
     uint32_t *cnts = nullptr, *nd = nullptr, *list_slots = nullptr, *cnt_flat = nullptr, *gfill = nullptr;
-    uint32_t *members = nullptr, *sorted = nullptr, *row_count = nullptr, *base_d = nullptr, *mpos = nullptr;
+    uint32_t *members = nullptr, *sorted = nullptr, *wpos = nullptr, *row_count = nullptr, *base_d = nullptr, *mpos = nullptr;
     uint16_t *rank_slot = nullptr, *sorted16 = nullptr;
     unsigned long long* list_keys = nullptr;
     uint64_t *cnt_off_d = nullptr, *goff_d = nullptr, *groups_d = nullptr, *start64 = nullptr;
@@ -803,6 +831,16 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
             }
         }
 
+        if (query_maps) {  // groups as the new profiles' rare counts read them
+            const int windows = query_windows(n);
+            const size_t entries = off_h[L] * (size_t)windows + 1;
+            TCH_CK(e, dalloc(&wpos, entries, &out->bytes));
+            window_kernel<<<grid_for(entries, sms), 256>>>(goff_d, sorted, off_h[L], windows, wpos);
+            TCH_CK(e, cudaGetLastError());
+            TCH_CK(e, dalloc(&sorted16, n_members + 8, &tmp_bytes));  // the last piece is loaded whole
+            narrow_members_kernel<<<grid_for(std::max<size_t>(n_members, 1), sms), 256>>>(sorted, n_members, sorted16);
+            TCH_CK(e, cudaGetLastError());
+        }
         mark("rare groups");
         if (runs) {  // the partner runs of every row, for triangle solves
             TCH_CK(e, dalloc(&row_count, (size_t)n, &tmp_bytes));
@@ -832,14 +870,16 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
             out->n_rare = (size_t)n_rare_pairs;
             out->cnt_off = cnt_off_d;
             out->goff = goff_d;
-            out->members = sorted;
+            out->members = query_maps ? nullptr : sorted;  // freed with the rest
             out->members16 = sorted16;
             out->mpos = mpos;
-            out->bytes += ((size_t)L + 1) * 8 + (off_h[L] + 1) * 8 + n_members * (narrow ? 2 : 4) + (size_t)n * L * 4;
+            out->bytes += ((size_t)L + 1) * 8 + (off_h[L] + 1) * 8 + n_members * (sorted16 ? 2 : 4) + (size_t)n * L * 4;
             if (query_maps) {  // what new profiles need to be encoded like these
                 out->slot_ids = reinterpret_cast<uint64_t*>(slot_ids);
                 out->col = col_d;
                 out->base = base_d;
+                out->wpos = wpos;
+                wpos = nullptr;
                 out->bytes += off_h[L] * 12 + ((size_t)L + 1) * 4;
                 slot_ids = nullptr;
                 col_d = nullptr;
@@ -847,7 +887,7 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
             }
             cnt_off_d = nullptr;
             goff_d = nullptr;
-            sorted = nullptr;
+            if (out->members) sorted = nullptr;
             sorted16 = nullptr;
             mpos = nullptr;
             goto done;
@@ -893,12 +933,12 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
     }
 done:
     cudaFree(err_d); cudaFree(nd); cudaFree(cnt_off_d); cudaFree(cnt_flat); cudaFree(col_d); cudaFree(base_d);
-    cudaFree(goff_d); cudaFree(members); cudaFree(sorted); cudaFree(sorted16); cudaFree(gfill); cudaFree(groups_d); cudaFree(row_count);
+    cudaFree(goff_d); cudaFree(members); cudaFree(sorted); cudaFree(sorted16); cudaFree(wpos); cudaFree(gfill); cudaFree(groups_d); cudaFree(row_count);
     cudaFree(start64); cudaFree(mpos); cudaFree(slot_ids);
     return 0;
 fail:
     cudaFree(err_d); cudaFree(nd); cudaFree(cnt_off_d); cudaFree(cnt_flat); cudaFree(col_d); cudaFree(base_d);
-    cudaFree(goff_d); cudaFree(members); cudaFree(sorted); cudaFree(sorted16); cudaFree(gfill); cudaFree(groups_d); cudaFree(row_count);
+    cudaFree(goff_d); cudaFree(members); cudaFree(sorted); cudaFree(sorted16); cudaFree(wpos); cudaFree(gfill); cudaFree(groups_d); cudaFree(row_count);
     cudaFree(start64); cudaFree(keys); cudaFree(cnts); cudaFree(rank_slot); cudaFree(list_keys); cudaFree(list_slots);
     cudaFree(mpos); cudaFree(slot_ids);
     free_device_encoding(out);
@@ -914,6 +954,7 @@ void free_device_encoding(DeviceEncoding* d) {
     cudaFree(d->goff);
     cudaFree(d->members);
     cudaFree(d->members16);
+    cudaFree(d->wpos);
     cudaFree(d->mpos);
     cudaFree(d->roff);
     cudaFree(d->rlo);
@@ -933,6 +974,7 @@ void free_device_encoding(DeviceEncoding* d) {
     d->cnt_off = d->goff = nullptr;
     d->members = d->mpos = nullptr;
     d->members16 = nullptr;
+    d->wpos = nullptr;
 }
 
 }  // namespace tch

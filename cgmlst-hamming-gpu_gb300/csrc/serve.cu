@@ -190,15 +190,14 @@ int db_query(tch_db* db, int m, const uint64_t* qcalls, uint16_t* h_qdb, uint16_
             ce = cudaGetLastError();
             if (ce != cudaSuccess) goto done;
             RareGroups g;
-            g.x = enc.x;
             g.cnt_off = enc.cnt_off;
-            g.goff = enc.goff;
-            g.members = enc.members;
-            g.mpos = enc.mpos;
+            g.members16 = enc.members16;
+            g.wpos = enc.wpos;
+            g.windows = query_windows(n);
             g.n = n;
             g.L = L;
             mark();
-            ce = launch_rare_query(g, xq, m, R, ldr, db->sms, st);
+            ce = launch_rare_query(g, xq, m, R, ldr, st);
             mark();
             if (ce != cudaSuccess) goto done;
             StripeArgs a;

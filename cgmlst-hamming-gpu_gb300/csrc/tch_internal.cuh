@@ -239,7 +239,17 @@ struct RareGroups {
     const uint32_t* rlo = nullptr;
     const uint32_t* rpre = nullptr;
     const uint32_t* rtot = nullptr;
+    // For new profiles (databases; members16 modulo 65 536): wpos[q * windows + w] =
+    // the first member of slot q's group at or after row w * kQueryWindow, and the
+    // next entry where the window's members end (slot q + 1's first for the last).
+    const uint32_t* wpos = nullptr;
+    int windows = 0;
 };
+// Columns that one CTA of the new profiles' rare counts covers (32 KB of
+// counters): narrower windows put more CTAs on a single profile (25 of 8 192 for
+// 200 000 rows) but pay the 32-locus scans once more each.  Divides 65 536.
+constexpr int kQueryWindow = 16384;
+inline int query_windows(int n) { return std::max(1, (n + kQueryWindow - 1) / kQueryWindow); }
 
 // R[(i - r0) * ldr + (j - r0)] = number of loci where rows i and j share a
 // rare allele, for r0 <= i < r0 + rows and i < j < n; written as 0 for the
@@ -254,7 +264,7 @@ constexpr uint32_t kNoGroup = 0xFFFFFFFFu;
 // R[r * ldr + j] = loci where new profile r (ranks xq, m x L u32 in the set's
 // numbering) and row j of the set share an allele that is rare in the set
 // (groups must include single-row groups), for j < n; 0 up to up(n, 256).
-cudaError_t launch_rare_query(const RareGroups& g, const uint32_t* xq, int m, uint16_t* R, size_t ldr, int sms,
+cudaError_t launch_rare_query(const RareGroups& g, const uint32_t* xq, int m, uint16_t* R, size_t ldr,
                               cudaStream_t st);
 cudaError_t launch_rare_dense(const RareGroups& g, int r0, int rows, uint16_t* R, size_t ldr, int sms,
                               cudaStream_t st);
@@ -310,6 +320,7 @@ struct DeviceEncoding {
     uint64_t* slot_ids = nullptr;
     int32_t* col = nullptr;
     uint32_t* base = nullptr;
+    uint32_t* wpos = nullptr;   // where each group enters each window of rows (RareGroups)
     size_t bytes = 0;
 };
 

@@ -137,3 +137,27 @@ def test_query_against_k_chunked_database(tch):
         tch.set_max_chunk_bytes(0)
     exp_qdb, exp_qq = expected(A[:500], A[500:])
     check(qdb, qq, exp_qdb, exp_qq)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 9, 16383, 16384, 16385, 65537, 70001])
+@pytest.mark.parametrize("tau", [0, 100000])
+def test_query_window_edges(pkg, n, tau):
+    """Database sizes around the windows of the rare counts (16 384 rows) and
+    past two-byte row numbers; alleles of single rows, of a few and of most
+    rows; ids the database never saw; automatic tau and every allele rare."""
+    rng = np.random.default_rng(n)
+    L, m = 37, 5
+    top = np.maximum(2, (n * rng.random(L) ** 4).astype(np.int64))
+    A = rng.integers(0, top[None, :] + 1, size=(n, L)).astype(np.uint64)
+    Q = A[rng.integers(0, n, m)].copy()
+    fresh = rng.random((m, L)) < 0.2
+    Q[fresh] = rng.integers(2**40, 2**41, size=int(fresh.sum()), dtype=np.uint64)
+    Q[rng.random((m, L)) < 0.05] = 0
+    want = np.stack([((A != q) & (A != 0) & (q != 0)).sum(1) for q in Q])
+    with pkg.Database(A, tau=tau) as db:
+        got, qq = db.query(Q)
+        np.testing.assert_array_equal(got, want)
+        np.testing.assert_array_equal(db.query(Q[:1], want_qq=False)[0], want[:1])
+    both = np.stack([((Q != q) & (Q != 0) & (q != 0)).sum(1) for q in Q])
+    np.testing.assert_array_equal(np.triu(qq, 1), np.triu(both, 1))
