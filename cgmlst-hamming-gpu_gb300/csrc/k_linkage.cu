@@ -4,28 +4,29 @@
 // (outbreak clustering, minimum spanning trees, nearest-neighbour searches;
 // docs/index.html, "The problem").  The reference stops at the matrix.
 //
-// Both kernels read the full n x n u16 matrix in HBM row by row: a row is one
-// contiguous run of n values that a CTA reads with 16-byte loads, so each
-// pass over the matrix is bound by HBM bandwidth (2 n^2 bytes per pass).
+// Both read the full n x n u16 matrix in HBM row by row, a warp per row with
+// 16-byte loads: a pass over the matrix is bound by HBM bandwidth (2 n^2 bytes).
 //
 // Minimum spanning tree (Borůvka).  Edges are ordered by (distance, smaller
 // index, larger index), a strict order, so the tree is unique and equals
-// Kruskal's under the same order.  Each round:
-//   scan    every row's lightest edge to another component.  Within a row the
-//           order above is (distance, column), so a thread keeps the first
-//           column of its smallest distance while it walks its columns in
-//           ascending order; the CTA reduces the row and one atomicMin folds it
-//           into the best key of the row's component.  A CTA takes kScanRows
-//           rows at once, so the component labels of the columns are loaded
-//           once for all of them.
-//   hook    every component root across its best edge to the component on
-//           the other side, recording the edge (of two components that chose
-//           the same edge, only the larger root hooks, which breaks the only
-//           cycles such a choice can make);
-//   relabel pointer doubling over the roots, ceil(log2 n) + 1 steps, then
-//           every profile takes its root's new root.
-// Each round at least halves the number of components, so at most
-// ceil(log2 n) rounds.  No step waits on another thread.
+// Kruskal's under the same order.  One pass gives every row its 16 nearest
+// columns; a round then needs only these lists, most of the time:
+//   lists   a row's lightest edge out of its component is its first listed
+//           column outside; one atomicMin folds it into the component's best
+//           key.  A row whose listed columns all lie inside is exhausted: all
+//           its other edges are at least as heavy as `beyond`, what its last
+//           pass left out.
+//   rescan  an exhausted row whose component's best so far is not below
+//           `beyond` is read again, and its list becomes its nearest columns
+//           outside, up to the component's best.  The largest component is left
+//           out: all others hooking still halves their number, and a component
+//           that takes no part this round loses nothing.
+//   hook    every other component root across its best edge, recording it (of
+//           two components that chose the same edge, only the larger root hooks,
+//           which breaks the only cycles such a choice can make);
+//   relabel pointers to the new roots, then every profile its new root.
+// Each round at least halves the number of the other components, so at most
+// ceil(log2 n) + 1 rounds.  No step waits on another thread.
 //
 // Nearest neighbours.  A warp per row reads the row once and keeps its k
 // smallest (distance, column) keys in its lanes' registers.
@@ -42,8 +43,6 @@ namespace tch {
 namespace {
 
 constexpr unsigned FULL = 0xFFFFFFFFu;
-constexpr int kScanThreads = 256;
-constexpr int kScanRows = 4;  // rows of one scan CTA, sharing the column-label loads
 constexpr int kNbrThreads = 256;
 constexpr int kMaxNeighbors = 32;
 constexpr int kIndexBits = 21;  // a profile index in an edge key
@@ -52,7 +51,7 @@ constexpr unsigned long long kNoEdge = ~0ull;
 constexpr uint32_t kNoDistance = 0x10000u;  // above every u16 distance
 
 enum LinkErr : int {
-    LINKERR_EDGE = 1,     // a component's best edge does not leave it
+    LINKERR_EDGE = 1,     // a component's best edge does not leave it, or the edges leave profiles apart
     LINKERR_COUNT = 2,    // more than n - 1 tree edges
     LINKERR_SELECT = 4,   // the neighbour selection lost count
 };
@@ -67,114 +66,6 @@ __device__ __forceinline__ unsigned long long edge_key(uint32_t w, uint32_t i, u
 __device__ __forceinline__ uint32_t lane16(const uint4& h, int e) {
     const uint32_t x = e < 2 ? h.x : e < 4 ? h.y : e < 6 ? h.z : h.w;
     return (e & 1) ? x >> 16 : x & 0xFFFFu;
-}
-
-__device__ __forceinline__ unsigned long long warp_min64(unsigned long long v) {
-    for (int o = 16; o; o >>= 1) {
-        const unsigned long long t = __shfl_xor_sync(FULL, v, o);
-        v = t < v ? t : v;
-    }
-    return v;
-}
-
-// comp[x] = x for x < n; the padding up to up(n, 8) is never used as a label.
-__global__ void mst_init_kernel(uint32_t* comp, int n, int n8) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    if (x < n8) comp[x] = x < n ? (uint32_t)x : 0xFFFFFFFFu;
-}
-
-// best[comp[i]] = min over rows i of the component and columns j of other
-// components of edge_key(H[i][j], i, j).  comp holds up(n, 8) entries.
-__global__ void __launch_bounds__(kScanThreads) mst_scan_kernel(const uint16_t* __restrict__ H, size_t ld, int n,
-                                                                const uint32_t* __restrict__ comp,
-                                                                unsigned long long* best) {
-    __shared__ unsigned long long part[kScanThreads / 32][kScanRows];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int nq = (n + 7) >> 3;  // 8-column chunks of a row
-    const uint4* comp4 = reinterpret_cast<const uint4*>(comp);
-    for (int i0 = blockIdx.x * kScanRows; i0 < n; i0 += gridDim.x * kScanRows) {  // uniform over the CTA
-        uint32_t ci[kScanRows], bw[kScanRows], bj[kScanRows];
-        const uint4* row[kScanRows];
-#pragma unroll
-        for (int r = 0; r < kScanRows; r++) {
-            const int i = i0 + r < n ? i0 + r : n - 1;
-            ci[r] = i0 + r < n ? __ldg(comp + i) : 0xFFFFFFFFu;
-            row[r] = reinterpret_cast<const uint4*>(H + (size_t)i * ld);
-            bw[r] = kNoDistance;
-            bj[r] = 0xFFFFFFFFu;
-        }
-        for (int q = threadIdx.x; q < nq; q += kScanThreads) {
-            const uint4 c0 = __ldg(comp4 + 2 * q), c1 = __ldg(comp4 + 2 * q + 1);
-            const uint32_t cj[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-#pragma unroll
-            for (int r = 0; r < kScanRows; r++) {
-                if (i0 + r >= n) break;
-                const uint4 h = __ldcs(row[r] + q);  // read once per round: do not keep it in L1
-#pragma unroll
-                for (int e = 0; e < 8; e++) {
-                    const uint32_t w = lane16(h, e);
-                    const int j = 8 * q + e;
-                    if (j < n && cj[e] != ci[r] && w < bw[r]) {
-                        bw[r] = w;
-                        bj[r] = (uint32_t)j;
-                    }
-                }
-            }
-        }
-#pragma unroll
-        for (int r = 0; r < kScanRows; r++) {
-            const unsigned long long m = warp_min64(((unsigned long long)bw[r] << 32) | bj[r]);
-            if (lane == 0) part[warp][r] = m;
-        }
-        __syncthreads();
-        if (threadIdx.x < kScanRows && i0 + (int)threadIdx.x < n) {
-            const int r = threadIdx.x;
-            unsigned long long m = part[0][r];
-            for (int w = 1; w < kScanThreads / 32; w++) m = part[w][r] < m ? part[w][r] : m;
-            const uint32_t w = (uint32_t)(m >> 32), j = (uint32_t)m;
-            if (w < kNoDistance) atomicMin(best + ci[r], edge_key(w, (uint32_t)(i0 + r), j));
-        }
-        __syncthreads();
-    }
-}
-
-// parent[c] = the root that c hooks to this round (c itself when it does not).
-__global__ void mst_hook_kernel(int n, const uint32_t* __restrict__ comp, const unsigned long long* __restrict__ best,
-                                uint32_t* parent, unsigned long long* edges, unsigned int* nedges, int* err) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= n) return;
-    uint32_t p = (uint32_t)c;
-    const unsigned long long key = best[c];
-    if (comp[c] == (uint32_t)c && key != kNoEdge) {
-        const uint32_t u = (uint32_t)(key >> kIndexBits) & kIndexMask, v = (uint32_t)key & kIndexMask;
-        if (u >= (uint32_t)n || v >= (uint32_t)n) {
-            atomicOr(err, LINKERR_EDGE);
-        } else {
-            const uint32_t cu = comp[u], cv = comp[v];
-            const uint32_t d = cu == (uint32_t)c ? cv : cu;
-            if ((cu != (uint32_t)c && cv != (uint32_t)c) || d == (uint32_t)c || d >= (uint32_t)n) {
-                atomicOr(err, LINKERR_EDGE);
-            } else if (!(best[d] == key && (uint32_t)c < d)) {
-                p = d;
-                const unsigned int slot = atomicAdd(nedges, 1u);
-                if (slot < (unsigned int)(n - 1))
-                    edges[slot] = key;
-                else
-                    atomicOr(err, LINKERR_COUNT);
-            }
-        }
-    }
-    parent[c] = p;
-}
-
-__global__ void mst_jump_kernel(int n, const uint32_t* __restrict__ pa, uint32_t* __restrict__ pb) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    if (x < n) pb[x] = pa[pa[x]];
-}
-
-__global__ void mst_relabel_kernel(int n, uint32_t* comp, const uint32_t* __restrict__ root) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    if (x < n) comp[x] = root[comp[x]];
 }
 
 // ---- nearest neighbours: one warp per row, one pass over the row
@@ -224,19 +115,16 @@ __device__ __forceinline__ uint32_t key_distance(unsigned long long key) {
     return key == kNoEdge ? kNoDistance : (uint32_t)(key >> 32);
 }
 
-// Row i's k nearest columns (j != i) by (distance, column).
-__global__ void __launch_bounds__(kNbrThreads) neighbors_kernel(const uint16_t* __restrict__ H, size_t ld, int n,
-                                                                int k, uint32_t* idx, uint16_t* dist, int* err) {
-    __shared__ unsigned long long buffers[kNbrWarps][64];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int i = blockIdx.x * kNbrWarps + warp;
-    if (i >= n) return;  // uniform over the warp; no block-wide step follows
-    unsigned long long* buf = buffers[warp];
-    const uint4* row = reinterpret_cast<const uint4*>(H + (size_t)i * ld);
+// The 32 nearest columns j != i of a row by (distance, column), in the lanes'
+// order, as far as k of them (those of distance `thr` and above may be missing
+// even so); with OUT only columns whose component is not `own`.
+template <bool OUT>
+__device__ __forceinline__ unsigned long long nearest_keys(const uint4* __restrict__ row, int n, int i, int k,
+                                                           const uint32_t* __restrict__ comp, uint32_t own,
+                                                           uint32_t thr, unsigned long long* buf, int lane) {
     const int nq = (n + 7) >> 3;
     unsigned long long list = kNoEdge;
-    uint32_t held = 0;           // keys in the buffer
-    uint32_t thr = kNoDistance;  // a value at or above it is not among the k nearest
+    uint32_t held = 0;  // keys in the buffer
     for (int q0 = 0; q0 < nq; q0 += 128) {
         uint4 h[4];
 #pragma unroll
@@ -253,10 +141,10 @@ __global__ void __launch_bounds__(kNbrThreads) neighbors_kernel(const uint16_t* 
                 for (int e = 0; e < 8; e++) {
                     const int j = 8 * (32 * u + lane) + e;
                     const uint32_t w = lane16(h[u], e);
-                    if (j < n && j != i && w < m) m = w;
+                    if (w < m && j < n && j != i && (!OUT || __ldg(comp + j) != own)) m = w;
                 }
             const unsigned long long s = sort_descending((unsigned long long)m, lane);
-            thr = (uint32_t)__shfl_sync(FULL, s, 32 - k) + 1u;  // at least k valid values lie below it
+            thr = min(thr, (uint32_t)__shfl_sync(FULL, s, 32 - k) + 1u);  // at least k valid values lie below it
         }
         // every key in the list or the buffer comes from smaller columns, except
         // those of this block: a later value at the k-th distance is no hit
@@ -269,7 +157,8 @@ __global__ void __launch_bounds__(kNbrThreads) neighbors_kernel(const uint16_t* 
             uint32_t hits = 0;
 #pragma unroll
             for (int e = 0; e < 8; e++)
-                hits |= (lane16(h[u], e) < thr && j0 + e < n && j0 + e != i ? 1u : 0u) << e;
+                if (lane16(h[u], e) < thr && j0 + e < n && j0 + e != i && (!OUT || __ldg(comp + j0 + e) != own))
+                    hits |= 1u << e;
             for (;;) {  // the lanes' first remaining hits, until none is left
                 const unsigned who = __ballot_sync(FULL, hits != 0);
                 if (!who) break;
@@ -299,10 +188,247 @@ __global__ void __launch_bounds__(kNbrThreads) neighbors_kernel(const uint16_t* 
         __syncwarp();
         list = merge_keys(list, lane < (int)held ? buf[lane] : kNoEdge, lane);
     }
+    return list;
+}
+
+// Row i's k nearest columns (j != i) by (distance, column).
+__global__ void __launch_bounds__(kNbrThreads) neighbors_kernel(const uint16_t* __restrict__ H, size_t ld, int n,
+                                                                int k, uint32_t* idx, uint16_t* dist, int* err) {
+    __shared__ unsigned long long buffers[kNbrWarps][64];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int i = blockIdx.x * kNbrWarps + warp;
+    if (i >= n) return;  // uniform over the warp; no block-wide step follows
+    const unsigned long long list = nearest_keys<false>(reinterpret_cast<const uint4*>(H + (size_t)i * ld), n, i, k,
+                                                        nullptr, 0, kNoDistance, buffers[warp], lane);
     if (lane < k) {
         if (list == kNoEdge) atomicOr(err, LINKERR_SELECT);
         idx[(size_t)i * k + lane] = (uint32_t)list;
         dist[(size_t)i * k + lane] = (uint16_t)(list >> 32);
+    }
+}
+
+// ---- minimum spanning tree ---------------------------------------------------
+
+// Columns listed per row.  8, 16 and 32 of them: 1.49, 1.52 and 1.64 ms for the
+// tree of 30 011 profiles in clusters of about 40, 0.99, 1.03 and 1.10 ms for
+// long-tail profiles, 0.57, 0.53 and 0.54 for 5 003 small ones.
+constexpr int kListed = 16;
+
+// Scalars of a run, and what the host reads after a round.
+struct MstState {
+    unsigned long long largest;  // size << 32 | ~root of the largest component (the first of equal ones)
+    unsigned long long total;    // sum of the edges' distances
+    unsigned int nedges;
+    int err;
+};
+
+// Every profile its own component, and every row its list.
+__global__ void __launch_bounds__(kNbrThreads)
+    mst_lists_kernel(const uint16_t* __restrict__ H, size_t ld, int n, unsigned long long* lists, uint32_t* beyond,
+                     uint32_t* comp, uint32_t* size) {
+    __shared__ unsigned long long buffers[kNbrWarps][64];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int i = blockIdx.x * kNbrWarps + warp;
+    if (i >= n) return;
+    const int k = min(kListed, n - 1);
+    const unsigned long long list = nearest_keys<false>(reinterpret_cast<const uint4*>(H + (size_t)i * ld), n, i, k,
+                                                        nullptr, 0, kNoDistance, buffers[warp], lane);
+    if (lane < kListed) lists[(size_t)i * kListed + lane] = lane < k ? list : kNoEdge;
+    const uint32_t last = key_distance(__shfl_sync(FULL, list, kListed - 1));
+    if (lane == 0) {
+        beyond[i] = n - 1 <= kListed ? kNoDistance : last;
+        comp[i] = (uint32_t)i;
+        size[i] = 1;
+    }
+}
+
+// best[c] = the lightest listed edge out of component c; exhausted[i] = 1 for
+// a row with none; the largest component's root.
+__global__ void __launch_bounds__(256)
+    mst_best_kernel(int n, const unsigned long long* __restrict__ lists, const uint32_t* __restrict__ comp,
+                    const uint32_t* __restrict__ size, unsigned long long* best, uint8_t* exhausted,
+                    MstState* state) {
+    const int lane = threadIdx.x & 31;
+    const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (i >= n) return;
+    const uint32_t own = comp[i];
+    const unsigned long long key = lane < kListed ? lists[(size_t)i * kListed + lane] : kNoEdge;
+    const bool out = key != kNoEdge && comp[(uint32_t)key] != own;
+    const unsigned who = __ballot_sync(FULL, out);
+    if (who && lane == __ffs(who) - 1)
+        atomicMin(best + own, edge_key((uint32_t)(key >> 32), (uint32_t)i, (uint32_t)key));
+    if (lane == 0) {
+        exhausted[i] = who ? 0 : 1;
+        if (own == (uint32_t)i) {
+            const unsigned long long mine = (unsigned long long)size[i] << 32 | ~(uint32_t)i;
+            if (mine > *(volatile unsigned long long*)&state->largest) atomicMax(&state->largest, mine);
+        }
+    }
+}
+
+// Exhausted rows that their component's best does not rule out are read again.
+__global__ void __launch_bounds__(kNbrThreads)
+    mst_rescan_kernel(const uint16_t* __restrict__ H, size_t ld, int n, unsigned long long* lists, uint32_t* beyond,
+                      const uint32_t* __restrict__ comp, const uint8_t* __restrict__ exhausted,
+                      unsigned long long* best, const MstState* state) {
+    __shared__ unsigned long long buffers[kNbrWarps][64];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int i = blockIdx.x * kNbrWarps + warp;
+    if (i >= n || !exhausted[i]) return;
+    const uint32_t own = comp[i], floor = beyond[i];
+    if (own == ~(uint32_t)state->largest || floor >= kNoDistance) return;
+    // the best only falls while rows of the component are read: any value of it
+    // rules out what is heavier
+    const unsigned long long b = __shfl_sync(FULL, *(volatile unsigned long long*)(best + own), 0);
+    const uint32_t limit = b == kNoEdge ? kNoDistance : (uint32_t)(b >> (2 * kIndexBits)) + 1u;
+    if (floor >= limit) return;  // every edge that is not listed is heavier than the best
+    const unsigned long long list = nearest_keys<true>(reinterpret_cast<const uint4*>(H + (size_t)i * ld), n, i,
+                                                       kListed, comp, own, limit, buffers[warp], lane);
+    if (lane < kListed) lists[(size_t)i * kListed + lane] = list;
+    const uint32_t last = key_distance(__shfl_sync(FULL, list, kListed - 1));
+    if (lane == 0) {
+        beyond[i] = min(limit, last);
+        if (list != kNoEdge) atomicMin(best + own, edge_key((uint32_t)(list >> 32), (uint32_t)i, (uint32_t)list));
+    }
+}
+
+// parent[c] = the root that c hooks to this round (c itself when it does not).
+__global__ void mst_hook_kernel(int n, const uint32_t* __restrict__ comp, const unsigned long long* __restrict__ best,
+                                uint32_t* parent, uint32_t* size, unsigned long long* edges, MstState* state) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31;
+    uint32_t p = (uint32_t)c;
+    const uint32_t largest = ~(uint32_t)state->largest;
+    const unsigned long long key = c < n ? best[c] : kNoEdge;
+    bool hooks = false;
+    if (c < n && comp[c] == (uint32_t)c && key != kNoEdge && (uint32_t)c != largest) {
+        const uint32_t u = (uint32_t)(key >> kIndexBits) & kIndexMask, v = (uint32_t)key & kIndexMask;
+        if (u >= (uint32_t)n || v >= (uint32_t)n) {
+            atomicOr(&state->err, LINKERR_EDGE);
+        } else {
+            const uint32_t cu = comp[u], cv = comp[v];
+            const uint32_t d = cu == (uint32_t)c ? cv : cu;
+            if ((cu != (uint32_t)c && cv != (uint32_t)c) || d == (uint32_t)c || d >= (uint32_t)n) {
+                atomicOr(&state->err, LINKERR_EDGE);
+            } else if (!(best[d] == key && d != largest && (uint32_t)c < d)) {
+                p = d;
+                hooks = true;
+            }
+        }
+    }
+    const unsigned who = __ballot_sync(FULL, hooks);
+    if (who) {  // one atomic per warp
+        const uint32_t sum = __reduce_add_sync(FULL, hooks ? (uint32_t)(key >> (2 * kIndexBits)) : 0u);
+        unsigned int slot = 0;
+        if (lane == 0) {
+            slot = atomicAdd(&state->nedges, (unsigned int)__popc(who));
+            atomicAdd(&state->total, (unsigned long long)sum);
+        }
+        slot = __shfl_sync(FULL, slot, 0) + (unsigned int)__popc(who & ((1u << lane) - 1u));
+        if (hooks) {
+            if (slot < (unsigned int)(n - 1)) edges[slot] = key;
+            else atomicOr(&state->err, LINKERR_COUNT);
+        }
+    }
+    if (c >= n) return;
+    size[c] = 0;  // counted anew by the relabelling
+    parent[c] = p;
+}
+
+// Every pointer straight to its root: all threads shorten their chains at once,
+// each step taking whatever the others have made of its parent so far, so a
+// chain of length l takes about log2 l steps; pointers only ever move rootwards.
+__global__ void mst_jump_kernel(int n, volatile uint32_t* parent) {
+    const int x = blockIdx.x * blockDim.x + threadIdx.x;
+    if (x >= n) return;
+    for (uint32_t p = parent[x];;) {
+        const uint32_t g = parent[p];
+        if (g == p) break;
+        parent[x] = p = g;
+    }
+}
+
+__global__ void mst_relabel_kernel(int n, uint32_t* comp, const uint32_t* __restrict__ parent, uint32_t* size) {
+    const int x = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t c = x < n ? parent[comp[x]] : FULL;
+    if (x < n) comp[x] = c;
+    const unsigned peers = __match_any_sync(FULL, c);
+    if (x < n && (threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(size + c, (uint32_t)__popc(peers));
+}
+
+// The edges in order: counted by distance, gathered there, and placed among the
+// edges of the same distance by counting the smaller keys, a warp per edge.
+// (Counting against every edge took 0.13 ms for 30 010 of them, this 0.045; the
+// host's sort 1.2 with its checks.)
+constexpr int kDistances = 65536;
+
+__global__ void mst_count_kernel(int m, const unsigned long long* __restrict__ edges, uint32_t* count) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e < m) atomicAdd(count + (edges[e] >> (2 * kIndexBits)), 1u);
+}
+
+// count -> exclusive sums (kDistances + 1 of them) and a copy to fill from; one
+// CTA, each warp 2 048 counts, 128 at a time.
+__global__ void __launch_bounds__(1024) mst_sum_kernel(uint32_t* count, uint32_t* fill) {
+    __shared__ uint32_t warp_sum[32];
+    constexpr int kSteps = kDistances / 32 / 128;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint4* c4 = reinterpret_cast<uint4*>(count) + warp * (kDistances / 32 / 4) + lane;
+    uint4* f4 = reinterpret_cast<uint4*>(fill) + warp * (kDistances / 32 / 4) + lane;
+    uint4 v[kSteps];
+    uint32_t sum = 0;
+#pragma unroll
+    for (int q = 0; q < kSteps; q++) v[q] = c4[32 * q];
+#pragma unroll
+    for (int q = 0; q < kSteps; q++) sum += v[q].x + v[q].y + v[q].z + v[q].w;
+    sum = __reduce_add_sync(FULL, sum);
+    if (lane == 0) warp_sum[warp] = sum;
+    __syncthreads();
+    uint32_t before = __reduce_add_sync(FULL, lane < warp ? warp_sum[lane] : 0u);
+#pragma unroll
+    for (int q = 0; q < kSteps; q++) {
+        const uint32_t mine = v[q].x + v[q].y + v[q].z + v[q].w;
+        uint32_t inc = mine;
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t t = __shfl_up_sync(FULL, inc, d);
+            if (lane >= d) inc += t;
+        }
+        uint4 s;
+        s.x = before + inc - mine;
+        s.y = s.x + v[q].x;
+        s.z = s.y + v[q].y;
+        s.w = s.z + v[q].z;
+        c4[32 * q] = s;
+        f4[32 * q] = s;
+        before += __shfl_sync(FULL, inc, 31);
+    }
+    if (threadIdx.x == 1023) count[kDistances] = before;
+}
+
+__global__ void mst_gather_kernel(int m, const unsigned long long* __restrict__ edges, uint32_t* fill,
+                                  unsigned long long* out) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e < m) out[atomicAdd(fill + (edges[e] >> (2 * kIndexBits)), 1u)] = edges[e];
+}
+
+// The edges decoded at their places.  Also checks that the relabelling left one
+// component (with n - 1 edges, a tree).
+__global__ void __launch_bounds__(256)
+    mst_decode_kernel(int n, const unsigned long long* __restrict__ keys, const uint32_t* __restrict__ first,
+                      const uint32_t* __restrict__ comp, uint32_t* u, uint32_t* v, uint16_t* w, MstState* state) {
+    const int lane = threadIdx.x & 31, e = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (e >= n) return;
+    if (lane == 0 && comp[e] != comp[0]) atomicOr(&state->err, LINKERR_EDGE);
+    if (e == n - 1) return;
+    const unsigned long long key = keys[e];
+    const uint32_t d = (uint32_t)(key >> (2 * kIndexBits)), begin = first[d], end = first[d + 1];
+    uint32_t smaller = 0;
+    for (uint32_t t = begin + lane; t < end; t += 32) smaller += keys[t] < key;
+    const uint32_t at = begin + __reduce_add_sync(FULL, smaller);
+    if (lane == 0) {
+        u[at] = (uint32_t)(key >> kIndexBits) & kIndexMask;
+        v[at] = (uint32_t)key & kIndexMask;
+        w[at] = (uint16_t)d;
     }
 }
 
@@ -315,96 +441,96 @@ int check_matrix(const uint16_t* d_H, size_t ld, int n, Err& e) {
     return 0;
 }
 
-int mst_on_device(const uint16_t* d_H, size_t ld, int n, cudaStream_t st, std::vector<unsigned long long>& keys,
-                  Err& e) {
-    keys.clear();
+int mst_on_device(const uint16_t* d_H, size_t ld, int n, cudaStream_t st, uint32_t* u, uint32_t* v, uint16_t* w,
+                  uint64_t* total, Err& e) {
+    if (total) *total = 0;
     if (check_matrix(d_H, ld, n, e)) return 1;
     if (n < 2) return 0;
-    const size_t n8 = up((size_t)n, 8);
+    const size_t m = (size_t)n - 1;
     char* ws = nullptr;
-    uint32_t *comp, *pa, *pb;
-    unsigned long long *best, *edges;
-    unsigned int* nedges;
-    int* derr;
-    int dev = 0, sms = 0, rc = 1;
-    unsigned int got = 0, prev = 0;
-    int herr = 0;
+    unsigned long long *lists, *best, *edges;
+    uint32_t *comp, *parent, *size, *beyond, *d_u, *d_v, *count;
+    uint16_t* d_w;
+    uint8_t* exhausted;
+    MstState* state;
+    MstState got = {};
+    int rc = 1;
+    unsigned int prev = 0;
     const int steps = 32 - __builtin_clz((unsigned)(n - 1)) + 1;  // ceil(log2 n) + 1
-    const size_t bytes = n8 * 4 * 3 + (size_t)n * 8 * 2 + 64;
-    TCH_CK(e, cudaGetDevice(&dev));
-    TCH_CK(e, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const unsigned rows_grid = (unsigned)((n + kNbrWarps - 1) / kNbrWarps), vgrid = (unsigned)((n + 255) / 256);
+    const size_t n8 = up((size_t)n, 8);
+    // the lists' room (128 bytes a profile) serves the gathered edges afterwards
+    const size_t bytes = sizeof(MstState) + n8 * (8 * kListed + 8 + 8 + 4 * 4 + 4 + 4 + 2 + 1) + 16 +
+                         ((size_t)2 * kDistances + 4) * 4;
     TCH_CK(e, cudaMallocAsync(&ws, bytes, st));
-    comp = reinterpret_cast<uint32_t*>(ws);
-    pa = comp + n8;
-    pb = pa + n8;
-    best = reinterpret_cast<unsigned long long*>(pb + n8);
-    edges = best + n;
-    nedges = reinterpret_cast<unsigned int*>(edges + n);
-    derr = reinterpret_cast<int*>(nedges + 4);
-    TCH_CK(e, cudaMemsetAsync(nedges, 0, 32, st));
-    mst_init_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, st>>>(comp, n, (int)n8);
+    lists = reinterpret_cast<unsigned long long*>(ws);
+    best = lists + n8 * kListed;
+    edges = best + n8;
+    state = reinterpret_cast<MstState*>(edges + n8);
+    comp = reinterpret_cast<uint32_t*>(state + 1);
+    parent = comp + n8;
+    size = parent + n8;
+    beyond = size + n8;
+    d_u = beyond + n8;
+    d_v = d_u + n8;
+    d_w = reinterpret_cast<uint16_t*>(d_v + n8);
+    exhausted = reinterpret_cast<uint8_t*>(d_w + n8);
+    count = reinterpret_cast<uint32_t*>(ws + up((size_t)(reinterpret_cast<char*>(exhausted + n8) - ws), 16));
+    TCH_CK(e, cudaMemsetAsync(state, 0, sizeof(MstState), st));
+    mst_lists_kernel<<<rows_grid, kNbrThreads, 0, st>>>(d_H, ld, n, lists, beyond, comp, size);
     TCH_CK(e, cudaGetLastError());
+    // each round at least halves the other components: ceil(log2 n) + 1 rounds at most
+    for (int round = 0; got.nedges < m; round++) {
+        if (round > steps) {
+            e.set("minimum spanning tree: %u of %zu edges after %d rounds", got.nedges, m, round);
+            goto fail;
+        }
+        TCH_CK(e, cudaMemsetAsync(best, 0xFF, (size_t)n * 8, st));
+        TCH_CK(e, cudaMemsetAsync(&state->largest, 0, 8, st));
+        mst_best_kernel<<<(unsigned)((n + 7) / 8), 256, 0, st>>>(n, lists, comp, size, best, exhausted, state);
+        mst_rescan_kernel<<<rows_grid, kNbrThreads, 0, st>>>(d_H, ld, n, lists, beyond, comp, exhausted, best, state);
+        mst_hook_kernel<<<vgrid, 256, 0, st>>>(n, comp, best, parent, size, edges, state);
+        mst_jump_kernel<<<vgrid, 256, 0, st>>>(n, parent);
+        mst_relabel_kernel<<<vgrid, 256, 0, st>>>(n, comp, parent, size);
+        TCH_CK(e, cudaGetLastError());
+        TCH_CK(e, cudaMemcpyAsync(&got, state, sizeof(got), cudaMemcpyDeviceToHost, st));
+        TCH_CK(e, cudaStreamSynchronize(st));
+        if (got.err) {
+            e.set("minimum spanning tree: device check failed (code %d)", got.err);
+            goto fail;
+        }
+        if (got.nedges == prev) {
+            e.set("minimum spanning tree: no edge added in round %d", round);
+            goto fail;
+        }
+        prev = got.nedges;
+    }
     {
-        const int rows_grid = (n + kScanRows - 1) / kScanRows;
-        const int grid = std::max(1, std::min(rows_grid, sms * (2048 / kScanThreads)));
-        const unsigned vgrid = (unsigned)((n + 255) / 256);
-        // each round at least halves the components: ceil(log2 n) rounds at most
-        for (int round = 0; got < (unsigned)(n - 1); round++) {
-            if (round > steps) {
-                e.set("minimum spanning tree: %u of %d edges after %d rounds", got, n - 1, round);
-                goto fail;
-            }
-            TCH_CK(e, cudaMemsetAsync(best, 0xFF, (size_t)n * 8, st));
-            mst_scan_kernel<<<grid, kScanThreads, 0, st>>>(d_H, ld, n, comp, best);
-            mst_hook_kernel<<<vgrid, 256, 0, st>>>(n, comp, best, pa, edges, nedges, derr);
-            uint32_t *from = pa, *to = pb;
-            for (int s = 0; s < steps; s++) {
-                mst_jump_kernel<<<vgrid, 256, 0, st>>>(n, from, to);
-                std::swap(from, to);
-            }
-            mst_relabel_kernel<<<vgrid, 256, 0, st>>>(n, comp, from);
-            TCH_CK(e, cudaGetLastError());
-            TCH_CK(e, cudaMemcpyAsync(&got, nedges, 4, cudaMemcpyDeviceToHost, st));
-            TCH_CK(e, cudaMemcpyAsync(&herr, derr, 4, cudaMemcpyDeviceToHost, st));
-            TCH_CK(e, cudaStreamSynchronize(st));
-            if (herr) {
-                e.set("minimum spanning tree: device check failed (code %d)", herr);
-                goto fail;
-            }
-            if (got == prev) {
-                e.set("minimum spanning tree: no edge added in round %d", round);
-                goto fail;
-            }
-            prev = got;
-        }
+        uint32_t* fill = count + kDistances + 4;
+        unsigned long long* keys = lists;
+        TCH_CK(e, cudaMemsetAsync(count, 0, (size_t)kDistances * 4, st));
+        mst_count_kernel<<<vgrid, 256, 0, st>>>((int)m, edges, count);
+        mst_sum_kernel<<<1, 1024, 0, st>>>(count, fill);
+        mst_gather_kernel<<<vgrid, 256, 0, st>>>((int)m, edges, fill, keys);
+        mst_decode_kernel<<<(unsigned)((n + 7) / 8), 256, 0, st>>>(n, keys, count, comp, d_u, d_v, d_w, state);
+        TCH_CK(e, cudaGetLastError());
     }
-    keys.resize((size_t)n - 1);
-    TCH_CK(e, cudaMemcpyAsync(keys.data(), edges, keys.size() * 8, cudaMemcpyDeviceToHost, st));
+    if (u) TCH_CK(e, cudaMemcpyAsync(u, d_u, m * 4, cudaMemcpyDeviceToHost, st));
+    if (v) TCH_CK(e, cudaMemcpyAsync(v, d_v, m * 4, cudaMemcpyDeviceToHost, st));
+    if (w) TCH_CK(e, cudaMemcpyAsync(w, d_w, m * 2, cudaMemcpyDeviceToHost, st));
+    TCH_CK(e, cudaMemcpyAsync(&got, state, sizeof(got), cudaMemcpyDeviceToHost, st));
     TCH_CK(e, cudaStreamSynchronize(st));
-    std::sort(keys.begin(), keys.end());
-    {  // the edges must join every profile: n - 1 unions
-        std::vector<uint32_t> p((size_t)n);
-        std::iota(p.begin(), p.end(), 0u);
-        auto find = [&](uint32_t x) {
-            while (p[x] != x) x = p[x] = p[p[x]];
-            return x;
-        };
-        for (unsigned long long k : keys) {
-            const uint32_t a = find((uint32_t)(k >> kIndexBits) & kIndexMask), b = find((uint32_t)k & kIndexMask);
-            if (a == b) {
-                e.set("minimum spanning tree: the edges contain a cycle");
-                goto fail;
-            }
-            p[std::max(a, b)] = std::min(a, b);
-        }
+    if (got.err) {
+        e.set("minimum spanning tree: device check failed (code %d)", got.err);
+        goto fail;
     }
+    if (total) *total = got.total;
     rc = 0;
 fail:
     if (ws) {
         cudaFreeAsync(ws, st);
         cudaStreamSynchronize(st);
     }
-    if (rc) keys.clear();
     return rc;
 }
 
@@ -472,20 +598,6 @@ fail:
     return 1;
 }
 
-void decode_edges(const std::vector<unsigned long long>& keys, uint32_t* u, uint32_t* v, uint16_t* w,
-                  uint64_t* total) {
-    uint64_t t = 0;
-    for (size_t q = 0; q < keys.size(); q++) {
-        const unsigned long long k = keys[q];
-        const uint32_t dw = (uint32_t)(k >> (2 * kIndexBits));
-        if (u) u[q] = (uint32_t)(k >> kIndexBits) & kIndexMask;
-        if (v) v[q] = (uint32_t)k & kIndexMask;
-        if (w) w[q] = (uint16_t)dw;
-        t += dw;
-    }
-    if (total) *total = t;
-}
-
 struct StreamGuard {
     cudaStream_t st = nullptr;
     bool own = false;
@@ -512,10 +624,7 @@ extern "C" int tch_mst_device(const uint16_t* d_H, size_t ld, int n, void* strea
     Err e{err, errlen};
     StreamGuard g;
     if (g.make(stream)) return e.set("could not create a stream");
-    std::vector<unsigned long long> keys;
-    if (mst_on_device(d_H, ld, n, g.st, keys, e)) return 1;
-    decode_edges(keys, u, v, w, total);
-    return 0;
+    return mst_on_device(d_H, ld, n, g.st, u, v, w, total, e);
 }
 
 extern "C" int tch_neighbors_device(const uint16_t* d_H, size_t ld, int n, int k, void* stream, uint32_t* idx,
@@ -533,13 +642,14 @@ extern "C" int tch_solver_mst(tch_solver* s, uint32_t* u, uint32_t* v, uint16_t*
     uint16_t* H = nullptr;
     size_t ld = 0;
     int n = 0, rc = 1;
-    std::vector<unsigned long long> keys;
     if (g.make(nullptr)) return e.set("could not create a stream");
     if (full_matrix(s, &n, &H, &ld, g.st, err, errlen)) return 1;
-    if (n >= 2 && mst_on_device(H, ld, n, g.st, keys, e)) goto done;
-    decode_edges(keys, u, v, w, total);
-    rc = 0;
-done:
+    if (n < 2) {
+        if (total) *total = 0;
+        rc = 0;
+    } else {
+        rc = mst_on_device(H, ld, n, g.st, u, v, w, total, e);
+    }
     cudaFree(H);
     return rc;
 }

@@ -265,3 +265,28 @@ def test_gpu_neighbors_block_edges(pkg, n, order):
         idx, dist = pkg.neighbors_device(d.data_ptr(), ld, n, k)
         wi, wd = oracle.neighbors(H, k)
         assert (idx == wi).all() and (dist == wd).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [2, 32, 33, 34, 40, 700, 1301])
+@pytest.mark.parametrize("nested", ["clusters", "levels", "line", "equal"])
+def test_gpu_mst_exhausted_lists(pkg, n, nested):
+    """Matrices whose rows have far more than 32 columns at hand inside their
+    component: tight clusters, clusters of clusters, points on a line with
+    widening gaps (one long chain of hooks) and one distance everywhere."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(n)
+    if nested == "equal":
+        H = np.full((n, n), 7)
+    elif nested == "line":
+        x = np.cumsum(np.arange(n))
+        H = np.minimum(np.abs(x[:, None] - x[None, :]), 65535)
+    else:
+        H = rng.integers(0, 4, size=(n, n))
+        for size in ((50,) if nested == "clusters" else (40, 130, 410)):
+            part = rng.permutation(n) // size
+            H = H + np.where(part[:, None] == part[None, :], 0, 40 * size + rng.integers(0, 3, size=(n, n)))
+    H = np.triu(np.minimum(H, 65535), 1)
+    H = (H + H.T).astype(np.uint16)
+    d, ld = device_matrix(torch, H)
+    same_tree(pkg.mst_device(d.data_ptr(), ld, n), H)
