@@ -111,3 +111,25 @@ def test_solver_from_parsed_table(pkg, golden):
     n = len(tab.ids)
     iu = np.triu_indices(n, 1)
     np.testing.assert_array_equal(H[iu], ref[iu])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("pad", [0, 1, 7, 14, 15, 16, 17, 495, 510, 511, 512, 513])
+def test_cells_across_load_boundaries(pkg, pad):
+    """Rows that start anywhere in 16 bytes and cells that straddle the 16- and
+    512-byte steps of the parse: runs of empty cells, one cell longer than a
+    step, values of 1 to 20 digits, prefixes, the missing token, more and fewer
+    cells than loci, and a row that ends without a separator."""
+    rng = np.random.default_rng(pad)
+    L = 90
+    pick = ["", "7", "-", "INF-12", " 42 ", "1234567890123456789", "18446744073709551615", "x9", "00012", " 5"]
+    rows = ["FILE" + "".join(f"\tl{k}" for k in range(L))]
+    for r in range(24):
+        cells = [pick[int(c)] for c in rng.integers(0, len(pick), size=int(rng.integers(0, 2 * L)))]
+        if r == 3:
+            cells = [""] * 700
+        if r == 4:
+            cells = ["9" * 600 + "x", "5"]
+        rows.append("s" * ((pad + 3 * r) % 530) + "".join("\t" + c for c in cells))
+    same(pkg, "\n".join(rows) + "\n")
+    same(pkg, "\r\n".join(rows))
