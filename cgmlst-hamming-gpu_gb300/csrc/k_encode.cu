@@ -318,6 +318,38 @@ __global__ void window_kernel(const uint64_t* __restrict__ goff, const uint32_t*
     }
 }
 
+// Bit columns of the rows (DeviceEncoding::bits): a warp takes 32 loci (lane =
+// locus) and one word of 32 rows, whose ranks it reads with its lanes on
+// consecutive loci; the eight warps of a CTA take neighbouring words, so that a
+// column's 32 bytes are written together.
+__global__ void __launch_bounds__(256)
+    bit_columns_kernel(const uint16_t* __restrict__ x, int n, int L, const uint64_t* __restrict__ cnt_off,
+                       const int32_t* __restrict__ col_flat, const uint32_t* __restrict__ base, size_t words,
+                       uint32_t* bits) {
+    const int lane = threadIdx.x & 31;
+    const int k = blockIdx.y * 32 + lane;
+    const size_t w = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (w >= words || k >= L) return;
+    const uint64_t off = cnt_off[k];
+    int c[32];
+    uint32_t called = 0;
+#pragma unroll
+    for (int r = 0; r < 32; r++) {
+        const size_t i = w * 32 + r;
+        const int a = i < (size_t)n ? x[i * L + k] : 0;
+        c[r] = a ? col_flat[off + a] : -1;
+        called |= a ? 1u << r : 0u;
+    }
+    const int columns = (int)(base[k + 1] - base[k]);
+    for (int q = 0; q < columns; q++) {
+        uint32_t same = 0;
+#pragma unroll
+        for (int r = 0; r < 32; r++) same |= c[r] == q ? 1u << r : 0u;
+        bits[(base[k] + q) * words + w] = called & ~same;
+    }
+    bits[((size_t)base[L] + k) * words + w] = called;
+}
+
 // members modulo 65 536 in two bytes.
 __global__ void narrow_members_kernel(const uint32_t* __restrict__ members, size_t count, uint16_t* out) {
     for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < count; t += (size_t)gridDim.x * blockDim.x)
@@ -840,6 +872,16 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
             TCH_CK(e, dalloc(&sorted16, n_members + 8, &tmp_bytes));  // the last piece is loaded whole
             narrow_members_kernel<<<grid_for(std::max<size_t>(n_members, 1), sms), 256>>>(sorted, n_members, sorted16);
             TCH_CK(e, cudaGetLastError());
+            // bit columns for the smallest batches, when they leave most of the memory free
+            const size_t words = up((size_t)n, 1024) / 32, columns = (size_t)D + L;
+            TCH_CK(e, cudaMemGetInfo(&freeb, &totb));
+            if (columns * words * 4 <= freeb / 4) {
+                TCH_CK(e, dalloc(&out->bits, columns * words, &out->bytes));
+                out->bit_words = words;
+                bit_columns_kernel<<<dim3((unsigned)((words + 7) / 8), (unsigned)((L + 31) / 32)), 256>>>(
+                    out->x, n, L, cnt_off_d, col_d, base_d, words, out->bits);
+                TCH_CK(e, cudaGetLastError());
+            }
         }
         mark("rare groups");
         if (runs) {  // the partner runs of every row, for triangle solves
@@ -955,6 +997,7 @@ void free_device_encoding(DeviceEncoding* d) {
     cudaFree(d->members);
     cudaFree(d->members16);
     cudaFree(d->wpos);
+    cudaFree(d->bits);
     cudaFree(d->mpos);
     cudaFree(d->roff);
     cudaFree(d->rlo);
@@ -975,6 +1018,7 @@ void free_device_encoding(DeviceEncoding* d) {
     d->members = d->mpos = nullptr;
     d->members16 = nullptr;
     d->wpos = nullptr;
+    d->bits = nullptr;
 }
 
 }  // namespace tch

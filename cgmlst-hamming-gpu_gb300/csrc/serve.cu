@@ -13,7 +13,9 @@
 //              present but matches nothing); the database keeps only its
 //              B-side copy (one-hot columns negated)
 //   rare       u16 counts of rare equal alleles against every database row
-//   tile pass  the tcgen05 kernel over the m x n rectangle, subtracting them
+//   distances  the tcgen05 tile pass over the m x n rectangle, subtracting them;
+//              for a few profiles the database's bit columns instead, added up
+//              row by row (query_bits_kernel)
 //   q x q      the batch's own upper triangle by a direct count on the calls
 //              (ids compared as given; 0 = missing)
 // Every distance is exact; the database's tau only decides which alleles go
@@ -41,8 +43,11 @@
 namespace tch {
 namespace {
 
+// xq = the ids' ranks; sel (optional) = the bit column of every cell's allele
+// (DeviceEncoding::bits, `D` frequent ones first), ~0 for a missing call.
 __global__ void query_rank_kernel(const uint64_t* __restrict__ q, int m, int L, const uint64_t* __restrict__ cnt_off,
-                                  const uint64_t* __restrict__ slot_ids, uint32_t* xq) {
+                                  const uint64_t* __restrict__ slot_ids, uint32_t* xq, uint32_t* sel,
+                                  const int32_t* __restrict__ col, const uint32_t* __restrict__ base, uint32_t D) {
     const size_t total = (size_t)m * L;
     for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
         const int k = (int)(t % L);
@@ -58,6 +63,78 @@ __global__ void query_rank_kernel(const uint64_t* __restrict__ q, int m, int L, 
             r = (lo < cnt_off[k + 1] && slot_ids[lo] == v) ? (uint32_t)(lo - cnt_off[k]) : kNovelRank;
         }
         xq[t] = r;
+        if (sel) {
+            const int32_t c = r && r != kNovelRank ? col[cnt_off[k] + r] : -1;
+            sel[t] = !r ? ~0u : c >= 0 ? base[k] + (uint32_t)c : D + (uint32_t)k;
+        }
+    }
+}
+
+// Distances of one new profile (blockIdx.y) to 1 024 rows of the database from
+// its bit columns: a row differs at the loci whose column (the one that sel
+// names) has its bit, less those where the two share a rare allele (R).  Each
+// warp adds up a share of the loci, lane = 32 rows, bit by bit: eight columns go
+// through carry-save adders into binary counters held as planes of bits, which
+// are spread into row counts once at the end.
+//
+// Bound by the columns' read, n / 8 bytes per locus (28 MB for 200 000 x 1 142,
+// mostly from L2 when queries carry common alleles), where the tile pass reads
+// every row's whole operand (1.07 GB): a query of one profile takes 92 us, with
+// the tile pass 253.
+constexpr int QB_T = 512, QB_PLANES = 13;  // 16 warps: at most 4 096 loci each
+__device__ __forceinline__ uint32_t carry_add(uint32_t& a, uint32_t b, uint32_t c) {
+    const uint32_t carry = (a & b) | (a & c) | (b & c);
+    a = a ^ b ^ c;
+    return carry;
+}
+__global__ void __launch_bounds__(QB_T)
+    query_bits_kernel(const uint32_t* __restrict__ bits, size_t words, const uint32_t* __restrict__ sel, int n, int L,
+                      const uint16_t* __restrict__ R, size_t ldr, uint16_t* __restrict__ out, size_t ldo) {
+    __shared__ uint32_t count[32 * 33];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, r = blockIdx.y;
+    for (int t = tid; t < 32 * 33; t += QB_T) count[t] = 0;
+    __syncthreads();
+    const uint32_t* mine = bits + (size_t)blockIdx.x * 32 + lane;
+    const int per = (L + QB_T / 32 - 1) / (QB_T / 32);
+    const int k0 = min(L, warp * per), k1 = min(L, k0 + per);
+    uint32_t p[QB_PLANES];
+#pragma unroll
+    for (int b = 0; b < QB_PLANES; b++) p[b] = 0;
+    for (int k = k0; k < k1; k += 32) {
+        const uint32_t s = k + lane < k1 ? __ldg(sel + (size_t)r * L + k + lane) : ~0u;
+#pragma unroll
+        for (int g = 0; g < 32; g += 8) {
+            uint32_t x[8];
+#pragma unroll
+            for (int e = 0; e < 8; e++) {
+                const uint32_t c = __shfl_sync(0xFFFFFFFFu, s, g + e);
+                x[e] = c != ~0u ? __ldg(mine + (size_t)c * words) : 0u;
+            }
+            const uint32_t a0 = carry_add(p[0], x[0], x[1]), a1 = carry_add(p[0], x[2], x[3]);
+            const uint32_t b0 = carry_add(p[1], a0, a1);
+            const uint32_t a2 = carry_add(p[0], x[4], x[5]), a3 = carry_add(p[0], x[6], x[7]);
+            const uint32_t b1 = carry_add(p[1], a2, a3);
+            uint32_t c = carry_add(p[2], b0, b1);
+#pragma unroll
+            for (int b = 3; b < QB_PLANES; b++) {
+                const uint32_t t = p[b] & c;
+                p[b] ^= c;
+                c = t;
+            }
+        }
+    }
+#pragma unroll 4
+    for (int i = 0; i < 32; i++) {
+        uint32_t v = 0;
+#pragma unroll
+        for (int b = 0; b < QB_PLANES; b++) v |= ((p[b] >> i) & 1u) << b;
+        if (v) atomicAdd(count + i * 33 + lane, v);
+    }
+    __syncthreads();
+    for (int t = tid; t < 1024; t += QB_T) {
+        const int j = blockIdx.x * 1024 + t;
+        if (j < n)
+            out[(size_t)r * ldo + j] = (uint16_t)(count[(t & 31) * 33 + (t >> 5)] - R[(size_t)r * ldr + j]);
     }
 }
 
@@ -128,6 +205,13 @@ struct tch_db {
 namespace tch {
 namespace {
 
+// Batches of at most this many profiles go by the bit columns, whose read grows
+// with them, larger ones by the tile pass, whose does not up to 256: 1 / 8 / 16
+// profiles take 92 / 213 / 332 us by columns and 253 / 284 / 304 by tiles against
+// 200 000 x 1 142, 103 / 166 / 212 and 236 / 247 / 254 against 50 000 x 3 016.
+constexpr int kBitProfiles = 8;
+bool by_bits(const tch_db* db, int m) { return m <= kBitProfiles && db->enc.bits; }
+
 size_t query_bytes(const tch_db* db, int m) {
     const size_t mr = up((size_t)std::max(m, 1), 256);
     return (size_t)m * db->L * 12 + mr * (size_t)db->enc.kb + (size_t)m * up((size_t)db->n, kRareDenseAlign) * 2 +
@@ -140,7 +224,7 @@ int db_query(tch_db* db, int m, const uint64_t* qcalls, uint16_t* h_qdb, uint16_
     const size_t mr = up((size_t)std::max(m, 1), 256);
     const size_t ldr = up((size_t)n, kRareDenseAlign), ldo = up((size_t)n, 8), ldq = up((size_t)m, 8);
     uint64_t* dq = nullptr;
-    uint32_t* xq = nullptr;
+    uint32_t *xq = nullptr, *sel = nullptr;
     uint16_t *R = nullptr, *out = nullptr, *qq = nullptr;
     int* derr = nullptr;
     Fp4Operands QX;  // the batch's A-side rows: the database's K layout, m rows
@@ -149,6 +233,7 @@ int db_query(tch_db* db, int m, const uint64_t* qcalls, uint16_t* h_qdb, uint16_
     QX.n_rows = mr;
     QX.kb = enc.kb;
     KChunks& X = QX.pos;
+    const bool bits = by_bits(db, m);
     cudaError_t ce = cudaSuccess;
     // TCH_VERBOSE=1: device time of each phase on stderr
     const char* vb = getenv("TCH_VERBOSE");
@@ -167,7 +252,9 @@ int db_query(tch_db* db, int m, const uint64_t* qcalls, uint16_t* h_qdb, uint16_
     alloc((void**)&dq, (size_t)m * L * 8);
     alloc((void**)&xq, (size_t)m * L * 4);
     alloc((void**)&derr, 4);
-    for (int c = 0; c < X.n; c++) alloc((void**)&X.p[c], mr * (size_t)X.width_of(c));
+    if (h_qdb && bits) alloc((void**)&sel, (size_t)m * L * 4);
+    if (h_qdb && !bits)
+        for (int c = 0; c < X.n; c++) alloc((void**)&X.p[c], mr * (size_t)X.width_of(c));
     if (h_qdb) {
         alloc((void**)&R, (size_t)m * ldr * 2);
         alloc((void**)&out, (size_t)m * ldo * 2);
@@ -181,12 +268,13 @@ int db_query(tch_db* db, int m, const uint64_t* qcalls, uint16_t* h_qdb, uint16_
     {
         const int grid = (int)std::min<size_t>(((size_t)m * L + 255) / 256, (size_t)db->sms * 16);
         if (h_qdb) {
-            for (int c = 0; c < X.n && ce == cudaSuccess; c++)
+            for (int c = 0; c < X.n && ce == cudaSuccess && !bits; c++)
                 ce = cudaMemsetAsync(X.p[c], 0, mr * (size_t)X.width_of(c), st);
             if (ce != cudaSuccess) goto done;
             mark();
-            query_rank_kernel<<<grid, 256, 0, st>>>(dq, m, L, enc.cnt_off, enc.slot_ids, xq);
-            query_pack_kernel<<<grid, 256, 0, st>>>(xq, m, L, enc.cnt_off, enc.col, enc.base, X);
+            query_rank_kernel<<<grid, 256, 0, st>>>(dq, m, L, enc.cnt_off, enc.slot_ids, xq, sel, enc.col, enc.base,
+                                                    (uint32_t)enc.D);
+            if (!bits) query_pack_kernel<<<grid, 256, 0, st>>>(xq, m, L, enc.cnt_off, enc.col, enc.base, X);
             ce = cudaGetLastError();
             if (ce != cudaSuccess) goto done;
             RareGroups g;
@@ -208,7 +296,13 @@ int db_query(tch_db* db, int m, const uint64_t* qcalls, uint16_t* h_qdb, uint16_
             a.ldo = ldo;
             a.err = derr;
             a.rect = true;
-            ce = launch_tc_stripe(QX, &enc.X, R, ldr, a, db->sms, st);
+            if (bits) {
+                query_bits_kernel<<<dim3((unsigned)(enc.bit_words / 32), m), QB_T, 0, st>>>(
+                    enc.bits, enc.bit_words, sel, n, L, R, ldr, out, ldo);
+                ce = cudaGetLastError();
+            } else {
+                ce = launch_tc_stripe(QX, &enc.X, R, ldr, a, db->sms, st);
+            }
             if (ce != cudaSuccess) goto done;
             mark();
             // one linear copy when the rows are packed (ldo == n), a pitched one otherwise
@@ -233,7 +327,7 @@ done:
     {
         int herr = 0;
         if (derr && ce == cudaSuccess) ce = cudaMemcpyAsync(&herr, derr, 4, cudaMemcpyDeviceToHost, st);
-        for (void* p : {(void*)dq, (void*)xq, (void*)R, (void*)out, (void*)qq, (void*)derr})
+        for (void* p : {(void*)dq, (void*)xq, (void*)sel, (void*)R, (void*)out, (void*)qq, (void*)derr})
             if (p) cudaFreeAsync(p, st);
         for (int c = 0; c < X.n; c++)
             if (X.p[c]) cudaFreeAsync(X.p[c], st);

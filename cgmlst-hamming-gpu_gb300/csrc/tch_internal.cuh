@@ -321,6 +321,12 @@ struct DeviceEncoding {
     int32_t* col = nullptr;
     uint32_t* base = nullptr;
     uint32_t* wpos = nullptr;   // where each group enters each window of rows (RareGroups)
+    // A query's differences as bit columns over the rows (null when they do not
+    // fit beside the operand), bit_words words each: column c < D has the rows
+    // called at the locus of frequent column c with another allele, column D + k
+    // those called at locus k.
+    uint32_t* bits = nullptr;
+    size_t bit_words = 0;
     size_t bytes = 0;
 };
 

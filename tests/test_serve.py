@@ -161,3 +161,19 @@ def test_query_window_edges(pkg, n, tau):
         np.testing.assert_array_equal(db.query(Q[:1], want_qq=False)[0], want[:1])
     both = np.stack([((Q != q) & (Q != 0) & (q != 0)).sum(1) for q in Q])
     np.testing.assert_array_equal(np.triu(qq, 1), np.triu(both, 1))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 31, 33, 1023, 1025, 2051])
+@pytest.mark.parametrize("L", [1, 15, 17, 511, 513, 1100])
+def test_few_profiles_by_bit_columns(pkg, n, L):
+    """One, eight (the most that go by the bit columns) and nine profiles (the
+    tile pass) give the same distances, at row counts around the columns' words
+    and CTAs and locus counts around the warps' shares."""
+    rng = np.random.default_rng(n * 7 + L)
+    A = rng.integers(0, rng.integers(2, 30, size=L)[None, :], size=(n, L)).astype(np.uint64)
+    Q = rng.integers(0, 30, size=(9, L)).astype(np.uint64)
+    want = np.stack([((A != q) & (A != 0) & (q != 0)).sum(1) for q in Q])
+    with pkg.Database(A, tau=max(2, n // 12)) as db:
+        for m in (1, 8, 9):
+            np.testing.assert_array_equal(db.query(Q[:m])[0], want[:m])
