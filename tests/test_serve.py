@@ -177,3 +177,44 @@ def test_few_profiles_by_bit_columns(pkg, n, L):
     with pkg.Database(A, tau=max(2, n // 12)) as db:
         for m in (1, 8, 9):
             np.testing.assert_array_equal(db.query(Q[:m])[0], want[:m])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [16500, 16504])
+@pytest.mark.parametrize("m", [255, 256, 257, 600])
+@pytest.mark.parametrize("pinned", [False, True])
+def test_results_copied_in_blocks(pkg, n, m, pinned):
+    """Results large enough to go back block by block (256 profiles each) beside
+    the kernels, rows packed and pitched, into page-locked and pageable buffers,
+    twice in a row on the same lane and from two threads."""
+    rng = np.random.default_rng(n + m)
+    L = 21
+    A = rng.integers(0, 12, size=(n, L)).astype(np.uint64)
+    Q = rng.integers(0, 13, size=(m, L)).astype(np.uint64)
+    want = np.zeros((m, n), np.uint16)
+    both = np.zeros((m, m), np.uint16)
+    for k in range(L):
+        want += (Q[:, k, None] != A[None, :, k]) & (Q[:, k, None] != 0) & (A[None, :, k] != 0)
+        both += (Q[:, k, None] != Q[None, :, k]) & (Q[:, k, None] != 0) & (Q[None, :, k] != 0)
+    with pkg.Database(A, tau=600) as db:
+        def one():
+            out = pkg.pinned_empty((m, n)) if pinned else np.empty((m, n), np.uint16)
+            for _ in range(2):
+                out[:] = 0xFFFF
+                qdb, qq = db.query(Q, out=out)
+                np.testing.assert_array_equal(qdb, want)
+                np.testing.assert_array_equal(np.triu(qq, 1), np.triu(both, 1))
+        errors = []
+
+        def guarded():
+            try:
+                one()
+            except BaseException as e:  # noqa: BLE001
+                errors.append(e)
+
+        threads = [threading.Thread(target=guarded) for _ in range(2)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        assert not errors, errors[0]
