@@ -403,10 +403,10 @@ __global__ void __launch_bounds__(T, T >= 1024 ? 1 : 1536 / T)
     extern __shared__ uint4 smem_rd[];
     uint32_t* cnt = reinterpret_cast<uint32_t*>(smem_rd);
     uint2* run = reinterpret_cast<uint2*>(cnt + cwords);  // cap + 1
+    grid_release();
     const M* members = sizeof(M) == 2 ? reinterpret_cast<const M*>(g.members16) : reinterpret_cast<const M*>(g.members);
     const int tid = threadIdx.x;
     int r = row_begin + (int)blockIdx.x;
-    if (r >= row_end) return;
     for (int w = tid; w < cwords / 4; w += T) smem_rd[w] = make_uint4(0, 0, 0, 0);
     uint64_t q0 = g.roff[r0 + r], q1 = g.roff[r0 + r + 1];
     if (q1 > q0) stage_runs<T>(g, r0 + r, q0, q1, 0, cap, run);
@@ -431,6 +431,7 @@ __global__ void __launch_bounds__(T, T >= 1024 ? 1 : 1536 / T)
         q0 = n0;
         q1 = n1;
     }
+    grid_wait();  // a band does not complete before the one launched ahead of it
 }
 
 // Many sets' whole triangles in one launch (batched solves): the rows of
@@ -456,6 +457,7 @@ __global__ void __launch_bounds__(T, 1024 / T)
     uint32_t* run = wsum + 64;              // kCap<T>: first member of each run found per locus
     uint32_t* pre = run + kCap<T>;          // kCap<T> + 1: exclusive prefix of the run lengths
     const int tid = threadIdx.x;
+    grid_release();
     for (int gr = blockIdx.x; gr < total_rows; gr += gridDim.x) {
         const RareJob& jb = jobs[__ldg(row_job + gr)];
         const RareGroups g = jb.g;
@@ -498,6 +500,7 @@ __global__ void __launch_bounds__(T, 1024 / T)
     uint32_t* wsum = run + (2 * T);        // 64: per-warp totals of the scans
     const int tid = threadIdx.x;
     const int n = g.n, L = g.L;
+    grid_release();
     // with every locus in one scan (L <= 2T) a thread keeps the same two
     // loci for all rows: their count offsets stay in registers and the next
     // row's ranks and positions are fetched while this row is counted
@@ -563,6 +566,7 @@ __global__ void __launch_bounds__(QT, 5)
     __shared__ uint4 counters[kQueryWindow / 8];
     __shared__ uint2 runs[QT / 32][33];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    grid_release();
     const int w = blockIdx.x, r = blockIdx.y;
     const int wb = w * kQueryWindow, nq = (min(cend, wb + kQueryWindow) - wb) >> 3;
     for (int q = tid; q < nq; q += QT) counters[q] = make_uint4(0, 0, 0, 0);
@@ -610,6 +614,7 @@ __global__ void __launch_bounds__(1024, 1)
     extern __shared__ uint4 smem_rd[];
     uint32_t* cnt = reinterpret_cast<uint32_t*>(smem_rd);
     const int tid = threadIdx.x;
+    grid_release();
     for (int r = blockIdx.x; r < rows; r += gridDim.x) {
         const int i = r0 + r;
         const uint32_t pa = __ldg(start + i), pb = __ldg(start + i + 1);
@@ -734,8 +739,9 @@ static cudaError_t launch_runs(const RareGroups& g, int r0, int ra, int rb, uint
     const int left = (runs_room(per_sm) - runs_smem<T>(cwords, 0)) / 8;
     const int cap = std::max(std::min(left, (int)up((size_t)g.L, 32)), kMinCap);
     const int grid = persistent ? std::min(per_sm * sms, rb - ra) : rb - ra;
-    rare_runs_kernel<T, M><<<grid, T, runs_smem<T>(cwords, cap), st>>>(g, r0, ra, rb, R, ldr, cend, cwords, cap);
-    return cudaGetLastError();
+    // a band after the first fills the SMs that the one before it leaves
+    return launch_after(ra > 0, rare_runs_kernel<T, M>, dim3((unsigned)grid), T, runs_smem<T>(cwords, cap), st, g, r0, ra,
+                        rb, R, ldr, cend, cwords, cap);
 }
 
 // The stripe's rows in bands of like width, each with as many CTAs per SM as

@@ -450,6 +450,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(peer_addr(scales, 0));
         }
+        // the operands do not depend on the launch before, so its tail overlaps the
+        // first tiles' MMAs; the rare counts do, and the output may still be read
+        grid_wait();
         int acc = 0;
         uint32_t aph = 0;
         bool bad = false;
@@ -661,8 +664,7 @@ cudaError_t launch_one(const Fp4Operands& A, const Fp4Operands& B, const uint16_
     p.tile_job = nullptr;
     if (p.num_tiles == 0) return cudaSuccess;
     const int grid = 2 * std::min(p.num_tiles, std::max(num_sms / 2, 1));
-    tc_stripe_kernel<false><<<grid, THREADS, SMEM_BYTES, st>>>(maps, p);
-    return cudaGetLastError();
+    return launch_after(a.after_counts, tc_stripe_kernel<false>, dim3((unsigned)grid), THREADS, SMEM_BYTES, st, maps, p);
 }
 
 }  // namespace
@@ -749,8 +751,8 @@ cudaError_t launch_tc_batch(const TcBatchPlan& plan, cudaStream_t st) {
     p.jobs = static_cast<const TcJob*>(plan.d_jobs);
     p.jmaps = static_cast<const CUtensorMap*>(plan.d_maps);
     p.tile_job = static_cast<const int*>(plan.d_tile_job);
-    tc_stripe_kernel<true><<<plan.grid, THREADS, SMEM_BYTES, st>>>(maps, p);
-    return cudaGetLastError();
+    // straight after the batch's rare counts
+    return launch_after(true, tc_stripe_kernel<true>, dim3((unsigned)plan.grid), THREADS, SMEM_BYTES, st, maps, p);
 }
 
 void tc_batch_release(TcBatchPlan* plan) {
@@ -777,6 +779,7 @@ cudaError_t launch_tc_stripe(const Fp4Operands& ops, const Fp4Operands* bops, co
         const size_t col = a.rect ? 0 : (size_t)done;  // a triangle's columns start at its first row
         s.out = a.out + (size_t)done * a.ldo + col;
         const uint16_t* Rs = R ? R + (size_t)done * ldr + col : nullptr;
+        if (done) s.after_counts = false;  // the launch before is another part's
         const cudaError_t e = launch_one(ops, b, Rs, ldr, s, num_sms, st);
         if (e != cudaSuccess) return e;
     }

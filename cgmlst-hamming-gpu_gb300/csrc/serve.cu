@@ -366,6 +366,7 @@ int db_query(tch_db* db, int m, const uint64_t* qcalls, uint16_t* h_qdb, uint16_
                     a.r0 = r0;
                     a.rows = rows;
                     a.out = out + (size_t)r0 * ldo;
+                    a.after_counts = true;
                     ce = launch_tc_stripe(QX, &enc.X, Rb, ldr, a, db->sms, st);
                 }
                 if (ce == cudaSuccess && lane) ce = cudaEventRecord(lane->ev[k], st);

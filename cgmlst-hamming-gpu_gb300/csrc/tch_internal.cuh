@@ -40,6 +40,33 @@ inline int current_device() {
     return d >= 0 && d < kMaxDevices ? d : 0;
 }
 
+// ---- launches that overlap the kernel before them ------------------------------
+// A kernel that calls grid_release() lets the next launch of its stream start
+// once all its own CTAs have started, when that launch asked for it
+// (launch_after); what the next kernel does before grid_wait() may not touch what
+// this one writes.
+#ifdef __CUDACC__
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Waits for the kernel launched before (if this launch may overlap it) to
+// complete with its writes visible.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class K, class... A>
+cudaError_t launch_after(bool overlap, K kernel, dim3 grid, int threads, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = overlap ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+#endif
+
 // Bits reported through the device error word.
 enum DevErr : int {
     DEVERR_RARE_PAIR = 1,  // a rare partner j outside (i, n)
@@ -140,6 +167,9 @@ struct StripeArgs {
     int* err = nullptr;
     bool rect = false;
     int group = 0;  // row blocks per raster group of the tile pass (0 = the library default)
+    // the launch before this one on the stream makes the rare counts and nothing
+    // else that the tile pass reads: the pass may start beside it
+    bool after_counts = false;
 };
 
 // ---- k_popc.cu --------------------------------------------------------------------

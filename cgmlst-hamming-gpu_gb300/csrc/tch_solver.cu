@@ -527,6 +527,7 @@ int solver_stripe(tch_solver* s, int r0, int rows, uint16_t* d_out, size_t ldo, 
         qa.out = d_out + (size_t)(q0 - r0) * ldo + (size_t)(q0 - r0);  // a triangle's columns start at its first row
         ce = s->dense ? launch_rare_dense(rare_groups(s), q0, qrows, R, ldr, s->num_sms, st)
                       : launch_rare_from_lists(s->dStart, s->dJs, s->n, q0, qrows, R, ldr, s->dErr, s->num_sms, st);
+        qa.after_counts = true;
         if (ce == cudaSuccess) ce = launch_dense_stripe(s, qa, R, ldr, st);
         const cudaError_t fe = cudaFreeAsync(R, st);
         if (ce == cudaSuccess) ce = fe;
@@ -869,6 +870,7 @@ int solver_stripe_counts(tch_solver* s, int r0, int rows, uint16_t* d_out, size_
     a.out = d_out;
     a.ldo = ldo;
     a.err = s->dErr;
+    a.after_counts = true;
     cudaError_t ce = launch_rare_dense(rare_groups(s), r0, rows, R, ldr, s->num_sms, st);
     if (ce == cudaSuccess) ce = launch_dense_stripe(s, a, R, ldr, st);
     if (ce != cudaSuccess) return e.set("stripe kernel: %s", cudaGetErrorString(ce));
