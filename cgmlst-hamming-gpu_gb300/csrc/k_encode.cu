@@ -40,14 +40,19 @@ namespace tch {
 namespace {
 
 constexpr uint32_t kMaxDistinct = 65535;
+constexpr int kSmallTable = 13;           // log2 of a locus's places in the first tables
+constexpr size_t kSmallProbes = 256;      // probes per id there
 constexpr int kJC = 65536;  // columns per counter chunk (u16 counters: 128 KB)
 
 __device__ __forceinline__ uint32_t hash_slot(uint64_t v, int logC) {
     return (uint32_t)((v * 0x9E3779B97F4A7C15ull) >> (64 - logC));
 }
 
+// Ids into their loci's tables; an id that finds no place within max_probe steps
+// is reported (the table is too small for its locus).
 __global__ void insert_kernel(const uint64_t* __restrict__ calls, int n, int L, int k0, int nk,
-                              unsigned long long* keys, uint32_t* cnts, int logC, uint32_t* nd, int* err) {
+                              unsigned long long* keys, uint32_t* cnts, int logC, size_t max_probe, uint32_t* nd,
+                              int* err) {
     const size_t C = (size_t)1 << logC, total = (size_t)n * nk;
     for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
         const size_t i = t / nk;
@@ -57,7 +62,7 @@ __global__ void insert_kernel(const uint64_t* __restrict__ calls, int n, int L, 
         unsigned long long* kt = keys + kk * C;
         uint32_t s = hash_slot(v, logC);
         bool placed = false;
-        for (size_t probe = 0; probe < C; probe++, s = (s + 1) & (uint32_t)(C - 1)) {
+        for (size_t probe = 0; probe < max_probe; probe++, s = (s + 1) & (uint32_t)(C - 1)) {
             unsigned long long cur = kt[s];
             if (cur == 0) cur = atomicCAS(kt + s, 0ull, v);
             if (cur == 0) {  // new distinct id
@@ -108,6 +113,19 @@ __global__ void rank_kernel(int k0, const unsigned long long* keys, const uint32
         return;
     }
     const uint64_t off = cnt_off[k0 + kk];
+    if (mm <= blockDim.x) {  // one id per thread (most loci): an eighth of the compares below
+        if (threadIdx.x < mm) tile[threadIdx.x] = lk[threadIdx.x];
+        __syncthreads();
+        if (threadIdx.x >= mm) return;
+        const unsigned long long mine = tile[threadIdx.x];
+        uint32_t r = 0;
+        for (uint32_t f = 0; f < mm; f++) r += tile[f] < mine;
+        const uint32_t slot = ls[threadIdx.x];
+        rank_slot[kk * C + slot] = (uint16_t)(r + 1);
+        cnt_flat[off + r + 1] = cnts[kk * C + slot];
+        if (slot_ids) slot_ids[off + r + 1] = mine;  // ids in rank order
+        return;
+    }
     // each thread ranks up to 8 ids per sweep of the id list through shared memory
     for (uint32_t e0 = 0; e0 < mm; e0 += 8 * blockDim.x) {
         unsigned long long mine[8];
@@ -206,12 +224,59 @@ __global__ void group_fill_kernel(const uint16_t* __restrict__ x, int n, int L, 
     }
 }
 
-// One CTA per rare group: rows are distinct, so a row's place is the number
-// of smaller rows in the group.  groups holds (first, end, locus) triples; the
-// rows go to sorted16 when given, else to sorted;
-// mpos (optional, n x L) receives every row's own index in `sorted`.
+// Rare groups in order: rows are distinct, so a row's place is the number of
+// smaller rows in the group.  groups holds (first, end, locus) triples; the rows
+// go to sorted16 when given, else to sorted; mpos (optional, n x L) receives every
+// row's own index there.
+struct SortedGroups {
+    uint32_t* sorted;
+    uint16_t* sorted16;
+    uint32_t* mpos;
+    int L;
+    __device__ __forceinline__ void put(uint64_t at, uint32_t row, int locus) const {
+        if (sorted16) sorted16[at] = (uint16_t)row;
+        else sorted[at] = row;
+        if (mpos) mpos[(size_t)row * L + locus] = (uint32_t)at;
+    }
+};
+
+// Groups of at most kWarpGroup rows, a warp each, four rows to a lane: most
+// groups have a handful of rows, for which a CTA is mostly idle threads (130 000
+// groups of 10 007 x 1 343 long-tail profiles: 0.53 ms, 0.20 so with the
+// larger ones).
+constexpr int kWarpGroup = 128;
+__global__ void __launch_bounds__(256)
+    group_sort_small_kernel(const uint64_t* __restrict__ groups, size_t ngroups, const uint32_t* __restrict__ members,
+                            SortedGroups out) {
+    __shared__ uint32_t tiles[8][kWarpGroup];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const size_t q = (size_t)blockIdx.x * 8 + warp;
+    if (q >= ngroups) return;
+    const uint64_t g0 = groups[3 * q];
+    const int count = (int)(groups[3 * q + 1] - g0), locus = (int)groups[3 * q + 2];
+    uint32_t* tile = tiles[warp];
+    uint32_t mine[4], rank[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        const int t = lane + 32 * u;
+        mine[u] = t < count ? members[g0 + t] : 0xFFFFFFFFu;
+        rank[u] = 0;
+        tile[t] = mine[u];
+    }
+    __syncwarp();
+    for (int t = 0; t < count; t++) {
+        const uint32_t w = tile[t];
+#pragma unroll
+        for (int u = 0; u < 4; u++) rank[u] += w < mine[u];
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+        if (lane + 32 * u < count) out.put(g0 + rank[u], mine[u], locus);
+}
+
+// Larger groups, a CTA each.
 __global__ void group_sort_kernel(const uint64_t* __restrict__ groups, const uint32_t* __restrict__ members,
-                                  uint32_t* sorted, uint16_t* sorted16, uint32_t* mpos, int L) {
+                                  SortedGroups out) {
     const uint64_t g0 = groups[3 * blockIdx.x], g1 = groups[3 * blockIdx.x + 1];
     const int locus = (int)groups[3 * blockIdx.x + 2];
     const uint32_t g = (uint32_t)(g1 - g0);
@@ -238,11 +303,7 @@ __global__ void group_sort_kernel(const uint64_t* __restrict__ groups, const uin
 #pragma unroll
         for (int q = 0; q < 4; q++) {
             const uint32_t e = e0 + q * blockDim.x + threadIdx.x;
-            if (e < g) {
-                if (sorted16) sorted16[g0 + r[q]] = (uint16_t)mine[q];
-                else sorted[g0 + r[q]] = mine[q];
-                if (mpos) mpos[(size_t)mine[q] * L + locus] = (uint32_t)(g0 + r[q]);
-            }
+            if (e < g) out.put(g0 + r[q], mine[q], locus);
         }
     }
 }
@@ -655,13 +716,17 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
     const bool query_maps = (flags & ENC_QUERY) != 0;
     int sms = 0, hflag = 0;
     size_t freeb = 0, totb = 0, tmp_bytes = 0;
-    int logC = 10;
-    while (((size_t)1 << logC) < 2 * (size_t)std::min<int>(std::max(n, 1), (int)kMaxDistinct)) logC++;
-    const size_t C = (size_t)1 << logC;
-    // loci per batch: hash tables + id lists within ~2 GB
-    const uint32_t lcap = (uint32_t)std::min<int>(std::max(n, 1), (int)kMaxDistinct);
-    const size_t per_locus = C * (8 + 4 + 2) + (size_t)lcap * 12;
-    const int nk_max = (int)std::max<size_t>(1, std::min<size_t>((size_t)L, ((size_t)2 << 30) / per_locus));
+    // Hash tables for kSmallTable ids per locus first: schemes have a few thousand
+    // alleles per locus at most, and clearing and scanning tables that hold as many
+    // ids as there are rows cost more than the inserts (10 007 x 1 343: 32 768 places
+    // per locus, 0.62 GB).  When a locus overfills its small table (or an id probes
+    // past kSmallProbes), the tables are built again with room for every row.
+    int full_log = 10;
+    while (((size_t)1 << full_log) < 2 * (size_t)std::min<int>(std::max(n, 1), (int)kMaxDistinct)) full_log++;
+    int logC = std::min(full_log, kSmallTable);
+    size_t C = 0;
+    uint32_t lcap = 0;
+    int nk_max = 0;
     unsigned long long* keys = nullptr;
     uint32_t *cnts = nullptr, *nd = nullptr, *list_slots = nullptr, *cnt_flat = nullptr, *gfill = nullptr;
     uint32_t *members = nullptr, *sorted = nullptr, *wpos = nullptr, *row_count = nullptr, *base_d = nullptr, *mpos = nullptr;
@@ -694,24 +759,36 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
     TCH_CK(e, dalloc(&nd, (size_t)L, nullptr));
     TCH_CK(e, cudaMemset(nd, 0, (size_t)L * 4));
     TCH_CK(e, dalloc(&out->x, (size_t)n * L, &out->bytes));
-    TCH_CK(e, dalloc(&keys, C * nk_max, &tmp_bytes));
-    TCH_CK(e, dalloc(&cnts, C * nk_max, &tmp_bytes));
-    TCH_CK(e, dalloc(&rank_slot, C * nk_max, &tmp_bytes));
-    TCH_CK(e, dalloc(&list_keys, (size_t)lcap * nk_max, &tmp_bytes));
-    TCH_CK(e, dalloc(&list_slots, (size_t)lcap * nk_max, &tmp_bytes));
     TCH_CK(e, dalloc(&cnt_off_d, (size_t)L + 1, nullptr));
 
     // ---- 1-3: ranks and counts, batch by batch
-    {
-        std::vector<uint32_t> cnt_parts;
-        for (int k0 = 0; k0 < L; k0 += nk_max) {
+    for (bool again = true; again;) {
+        again = false;
+        const bool small = logC < full_log;
+        const size_t max_probe = small ? kSmallProbes : (size_t)1 << logC;
+        C = (size_t)1 << logC;
+        lcap = (uint32_t)std::min<size_t>(std::min<int>(std::max(n, 1), (int)kMaxDistinct), C);
+        // loci per batch: hash tables + id lists within ~2 GB
+        nk_max = (int)std::max<size_t>(
+            1, std::min<size_t>((size_t)L, ((size_t)2 << 30) / (C * (8 + 4 + 2) + (size_t)lcap * 12)));
+        TCH_CK(e, dalloc(&keys, C * nk_max, &tmp_bytes));
+        TCH_CK(e, dalloc(&cnts, C * nk_max, &tmp_bytes));
+        TCH_CK(e, dalloc(&rank_slot, C * nk_max, &tmp_bytes));
+        TCH_CK(e, dalloc(&list_keys, (size_t)lcap * nk_max, &tmp_bytes));
+        TCH_CK(e, dalloc(&list_slots, (size_t)lcap * nk_max, &tmp_bytes));
+        for (int k0 = 0; k0 < L && !again; k0 += nk_max) {
             const int nk = std::min(nk_max, L - k0);
             TCH_CK(e, cudaMemset(keys, 0, C * nk * sizeof(unsigned long long)));
             TCH_CK(e, cudaMemset(cnts, 0, C * nk * sizeof(uint32_t)));
-            insert_kernel<<<grid_for((size_t)n * nk, sms), 256>>>(d_calls, n, L, k0, nk, keys, cnts, logC, nd, err_d);
+            insert_kernel<<<grid_for((size_t)n * nk, sms), 256>>>(d_calls, n, L, k0, nk, keys, cnts, logC, max_probe, nd,
+                                                                  err_d);
             TCH_CK(e, cudaGetLastError());
             TCH_CK(e, cudaMemcpy(nd_h.data() + k0, nd + k0, (size_t)nk * 4, cudaMemcpyDeviceToHost));
             TCH_CK(e, cudaMemcpy(&hflag, err_d, sizeof(int), cudaMemcpyDeviceToHost));
+            if (hflag && small) {
+                again = true;
+                break;
+            }
             if (hflag) { e.set("a locus has more than 65535 distinct alleles (limit 65535)"); goto fail; }
             for (int kk = 0; kk < nk; kk++) {
                 if (nd_h[k0 + kk] > kMaxDistinct) {
@@ -720,6 +797,17 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
                 }
                 off_h[k0 + kk + 1] = off_h[k0 + kk] + nd_h[k0 + kk] + 1;
             }
+        }
+        if (again) {
+            logC = full_log;
+            cudaFree(keys); keys = nullptr;
+            cudaFree(cnts); cnts = nullptr;
+            cudaFree(rank_slot); rank_slot = nullptr;
+            cudaFree(list_keys); list_keys = nullptr;
+            cudaFree(list_slots); list_slots = nullptr;
+            TCH_CK(e, cudaMemset(err_d, 0, sizeof(int)));
+            TCH_CK(e, cudaMemset(nd, 0, (size_t)L * 4));
+            continue;
         }
         // flat counts need every offset: a second sweep ranks the batches
         TCH_CK(e, cudaMemcpy(cnt_off_d, off_h.data(), ((size_t)L + 1) * 8, cudaMemcpyHostToDevice));
@@ -736,8 +824,8 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
             if (!one_batch) {
                 TCH_CK(e, cudaMemset(keys, 0, C * nk * sizeof(unsigned long long)));
                 TCH_CK(e, cudaMemset(cnts, 0, C * nk * sizeof(uint32_t)));
-                insert_kernel<<<grid_for((size_t)n * nk, sms), 256>>>(d_calls, n, L, k0, nk, keys, cnts, logC, nd,
-                                                                       err_d);
+                insert_kernel<<<grid_for((size_t)n * nk, sms), 256>>>(d_calls, n, L, k0, nk, keys, cnts, logC, max_probe,
+                                                                       nd, err_d);
                 TCH_CK(e, cudaGetLastError());
             }
             rank_kernel<<<nk, 512>>>(k0, keys, cnts, logC, nd, cnt_off_d, cnt_flat, rank_slot, list_keys, list_slots,
@@ -778,7 +866,7 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
         std::vector<int32_t> col(off_h[L], -1);
         std::vector<uint32_t> base((size_t)L + 1, 0);
         std::vector<uint64_t> goff(off_h[L] + 1, 0);
-        std::vector<uint64_t> groups;  // (first, end, locus) of every rare group
+        std::vector<uint64_t> groups, large;  // (first, end, locus) of the rare groups, by size
         double n_rare_pairs = 0;
         uint64_t D = 0;
         for (int k = 0; k < L; k++) {
@@ -794,9 +882,10 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
                 const bool rare = is_rank && !freq && c >= (query_maps ? 1u : 2u);
                 goff[q + 1] = goff[q] + (rare ? c : 0);
                 if (rare) {
-                    groups.push_back(goff[q]);
-                    groups.push_back(goff[q + 1]);
-                    groups.push_back((uint64_t)k);
+                    std::vector<uint64_t>& list = c <= (uint32_t)kWarpGroup ? groups : large;
+                    list.push_back(goff[q]);
+                    list.push_back(goff[q + 1]);
+                    list.push_back((uint64_t)k);
                     n_rare_pairs += (double)c * (double)(c - 1) / 2.0;
                 }
             }
@@ -836,7 +925,8 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
 
         mark("operand rows");
         // ---- 5: rare groups, sorted
-        const size_t ngroups = groups.size() / 3;
+        const size_t nsmall = groups.size() / 3, nlarge = large.size() / 3, ngroups = nsmall + nlarge;
+        groups.insert(groups.end(), large.begin(), large.end());
         TCH_CK(e, dalloc(&members, n_members, &tmp_bytes));
         // row runs where they are used (triangle solves) and their packed prefix
         // holds; two-byte members where every row index fits
@@ -856,11 +946,10 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
             TCH_CK(e, cudaMemcpy(groups_d, groups.data(), groups.size() * 8, cudaMemcpyHostToDevice));
             group_fill_kernel<<<grid_for((size_t)n * L, sms), 256>>>(out->x, n, L, cnt_off_d, goff_d, gfill, members);
             TCH_CK(e, cudaGetLastError());
-            for (size_t g0 = 0; g0 < ngroups; g0 += 65535) {
-                const unsigned gcount = (unsigned)std::min<size_t>(65535, ngroups - g0);
-                group_sort_kernel<<<gcount, 256>>>(groups_d + 3 * g0, members, sorted, sorted16, mpos, L);
-                TCH_CK(e, cudaGetLastError());
-            }
+            const SortedGroups sg{sorted, sorted16, mpos, L};
+            if (nsmall) group_sort_small_kernel<<<(unsigned)((nsmall + 7) / 8), 256>>>(groups_d, nsmall, members, sg);
+            if (nlarge) group_sort_kernel<<<(unsigned)nlarge, 256>>>(groups_d + 3 * nsmall, members, sg);
+            TCH_CK(e, cudaGetLastError());
         }
 
         if (query_maps) {  // groups as the new profiles' rare counts read them

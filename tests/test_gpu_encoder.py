@@ -171,3 +171,26 @@ def test_row_runs_piece_edges(pkg, n, groups):
             got = d.cpu().numpy().view(np.uint16)
             for r in range(rows):
                 np.testing.assert_array_equal(got[r, r + 1:rows], want[r0 + r, r0 + r + 1:])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("distinct", [(5, 511), (512, 513), (3000, 2049), (8000, 4), (8193, 40), (9100, 9100)])
+def test_distinct_counts_around_table_sizes(pkg, distinct):
+    """Loci with as many distinct ids as a small hash table holds, with more (the
+    tables are built again), and around the rank kernel's one id per thread."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(distinct[0])
+    n = 9100
+    cols = []
+    for d in distinct + (3,):
+        ids = rng.choice(2**62, size=d, replace=False).astype(np.uint64) + np.uint64(1)
+        cols.append(rng.permutation(np.concatenate([ids, ids[rng.integers(0, d, n - d)]])))
+    A = np.stack(cols, axis=1)
+    with pkg.Solver.from_calls(A, tau=4) as s:
+        ldo = (n + 7) // 8 * 8
+        d = torch.zeros((n, ldo), dtype=torch.int16, device="cuda:0")
+        s.stripe(0, n, d.data_ptr(), ldo, torch.cuda.current_stream().cuda_stream)
+        s.check()
+        t = torch.from_numpy(A.view(np.int64)).cuda()
+        want = sum((t[:, k, None] != t[None, :, k]).to(torch.int16) for k in range(A.shape[1]))
+        assert bool((torch.triu(d[:, :n], 1) == torch.triu(want, 1)).all())
