@@ -12,8 +12,9 @@
 //                         reference's sorted-unique rank, 1..k), and writes
 //                         the count of every rank
 //   3. cell_rank_kernel   every cell -> its rank (u16 matrix x, n x L)
-//      (host)             tau from the counts (analytic model), frequent
-//                         column map and per-locus offsets
+//      count_bins_kernel  the counts by size, from which the host picks tau
+//      locus_totals_kernel, locus_tables_kernel  frequent column map, rare groups
+//                         and per-locus offsets
 //   4. pack_x_kernel      x -> X rows [presence | one-hot] as packed e2m1
 //                         nibbles (+1.0), the pos copy; negate_onehot_kernel
 //                         derives the neg copy (one-hot part -1.0)
@@ -30,6 +31,7 @@
 // work (hashed ids included).
 
 #include <chrono>
+#include <mutex>
 #include <vector>
 
 #include <math.h>
@@ -513,6 +515,113 @@ rare_rows_kernel(const uint16_t* __restrict__ x, int n, int L, const uint64_t* _
     }
 }
 
+// ---- tables of the counts ------------------------------------------------------
+// The counts of all ranks stay on the device (a few hundred thousand of them):
+// the host sees their sums by size, from which it picks tau, and per-locus
+// totals, which it adds up.  Reading the counts on the host, building the tables
+// there and copying them back took 1.8 of 5.7 ms for 10 007 x 1 343 profiles.
+
+constexpr int kBins = 32;  // by floor(log2(count))
+struct CountBins {
+    unsigned long long n[kBins], sum[kBins], sq[kBins];  // how many, sum, sum of squares
+};
+
+__global__ void count_bins_kernel(const uint32_t* __restrict__ cnt, uint64_t slots, CountBins* bins) {
+    __shared__ CountBins mine;
+    for (int b = threadIdx.x; b < kBins; b += blockDim.x) mine.n[b] = mine.sum[b] = mine.sq[b] = 0;
+    __syncthreads();
+    for (uint64_t q = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; q < slots; q += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t c = cnt[q];
+        if (!c) continue;
+        const int b = 31 - __clz(c);
+        atomicAdd(&mine.n[b], 1ull);
+        atomicAdd(&mine.sum[b], (unsigned long long)c);
+        atomicAdd(&mine.sq[b], (unsigned long long)c * c);
+    }
+    __syncthreads();
+    for (int b = threadIdx.x; b < kBins; b += blockDim.x)
+        if (mine.n[b]) {
+            atomicAdd(&bins->n[b], mine.n[b]);
+            atomicAdd(&bins->sum[b], mine.sum[b]);
+            atomicAdd(&bins->sq[b], mine.sq[b]);
+        }
+}
+
+// One locus at a given tau: frequent columns, members and pairs of its rare
+// groups, and how many of these a warp and a CTA sort.
+struct LocusTotals {
+    unsigned long long columns, members, pairs, small, large;
+};
+
+// An allele seen c times: frequent (a one-hot column), or a rare group when it
+// has at least `least` rows.
+__device__ __forceinline__ bool rare_count(uint32_t c, uint32_t tau, uint32_t least) { return c < tau && c >= least; }
+
+__global__ void __launch_bounds__(256)
+    locus_totals_kernel(const uint32_t* __restrict__ cnt, const uint64_t* __restrict__ off, int L, uint32_t tau,
+                        uint32_t least, LocusTotals* out) {
+    const int lane = threadIdx.x & 31, k = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (k >= L) return;
+    unsigned long long t[5] = {};
+    for (uint64_t q = off[k] + 1 + lane; q < off[k + 1]; q += 32) {
+        const uint32_t c = cnt[q];
+        if (c >= tau) {
+            t[0]++;
+        } else if (rare_count(c, tau, least)) {
+            t[1] += c;
+            t[2] += (unsigned long long)c * (c - 1) / 2;
+            t[c <= (uint32_t)kWarpGroup ? 3 : 4]++;
+        }
+    }
+#pragma unroll
+    for (int v = 0; v < 5; v++)
+        for (int d = 16; d; d >>= 1) t[v] += __shfl_xor_sync(0xFFFFFFFFu, t[v], d);
+    if (lane == 0) out[k] = LocusTotals{t[0], t[1], t[2], t[3], t[4]};
+}
+
+// Where a locus's entries begin: `first` holds the totals of all loci before it.
+// col[q] = the slot's column within its locus or -1; goff[q] = where its group's
+// members begin; groups: (first, end, locus) triples, the small ones first.
+__global__ void __launch_bounds__(256)
+    locus_tables_kernel(const uint32_t* __restrict__ cnt, const uint64_t* __restrict__ off, int L, uint32_t tau,
+                        uint32_t least, const LocusTotals* __restrict__ first, unsigned long long nsmall, int32_t* col,
+                        uint64_t* goff, uint64_t* groups) {
+    const int lane = threadIdx.x & 31, k = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (k >= L) return;
+    const unsigned below = (1u << lane) - 1u;
+    unsigned long long columns = 0, at = first[k].members, small = first[k].small, large = nsmall + first[k].large;
+    const uint64_t end = off[k + 1];
+    for (uint64_t q0 = off[k]; q0 < end; q0 += 32) {  // the slot of rank 0 (missing) counts nothing
+        const uint64_t q = q0 + lane;
+        const uint32_t c = q < end && q > off[k] ? cnt[q] : 0;
+        const bool freq = c && c >= tau, rare = rare_count(c, tau, least), one = rare && c <= (uint32_t)kWarpGroup;
+        const unsigned mf = __ballot_sync(0xFFFFFFFFu, freq), ms = __ballot_sync(0xFFFFFFFFu, one),
+                       ml = __ballot_sync(0xFFFFFFFFu, rare && !one);
+        unsigned long long inc = rare ? c : 0;  // inclusive scan of the members
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const unsigned long long t = __shfl_up_sync(0xFFFFFFFFu, inc, d);
+            if (lane >= d) inc += t;
+        }
+        const unsigned long long begin = at + inc - (rare ? c : 0);
+        if (q < end) {
+            col[q] = freq ? (int32_t)(columns + __popc(mf & below)) : -1;
+            goff[q] = begin;
+        }
+        if (rare) {
+            uint64_t* g = groups + 3 * (one ? small + __popc(ms & below) : large + __popc(ml & below));
+            g[0] = begin;
+            g[1] = begin + c;
+            g[2] = (uint64_t)k;
+        }
+        columns += __popc(mf);
+        small += __popc(ms);
+        large += __popc(ml);
+        at += __shfl_sync(0xFFFFFFFFu, inc, 31);
+    }
+    if (k == L - 1 && lane == 0) goff[end] = at;
+}
+
 template <class T>
 cudaError_t dalloc(T** p, size_t count, size_t* bytes) {
     cudaError_t e = cudaMalloc((void**)p, std::max<size_t>(count, 1) * sizeof(T));
@@ -520,9 +629,61 @@ cudaError_t dalloc(T** p, size_t count, size_t* bytes) {
     return e;
 }
 
+// The encoder's working memory; what is still held goes back when the call ends.
+struct Working {
+    cudaMemPool_t pool = nullptr;
+    std::vector<void*> held;
+    template <class T>
+    cudaError_t get(T** p, size_t count) {
+        const cudaError_t e = cudaMallocFromPoolAsync((void**)p, std::max<size_t>(count, 1) * sizeof(T), pool, 0);
+        if (e == cudaSuccess) held.push_back(*p);
+        return e;
+    }
+    template <class T>
+    void drop(T** p) {
+        for (void*& h : held)
+            if (h == *p) {
+                cudaFreeAsync(h, 0);
+                h = held.back();
+                held.pop_back();
+                break;
+            }
+        *p = nullptr;
+    }
+    ~Working() {
+        for (void* h : held) cudaFreeAsync(h, 0);
+    }
+};
+
 int grid_for(size_t total, int sms) { return (int)std::min<size_t>((total + 255) / 256, (size_t)sms * 32); }
 
 }  // namespace
+
+// Working memory for building solvers, from a stream-ordered pool per device that
+// keeps up to 512 MB between calls (mapping it anew took a millisecond of a small
+// set's encoding); the driver hands back what is above that.
+cudaError_t working_pool(int device, cudaMemPool_t* out) {
+    constexpr uint64_t kKeptBytes = (uint64_t)512 << 20;
+    static std::mutex mu;
+    static cudaMemPool_t pools[kMaxDevices] = {};
+    if (device < 0 || device >= kMaxDevices) return cudaErrorInvalidDevice;
+    std::lock_guard<std::mutex> lk(mu);
+    if (!pools[device]) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        cudaMemPool_t pool;
+        cudaError_t e = cudaMemPoolCreate(&pool, &props);
+        if (e != cudaSuccess) return e;
+        uint64_t keep = kKeptBytes;
+        e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        if (e != cudaSuccess) return e;
+        pools[device] = pool;
+    }
+    *out = pools[device];
+    return cudaSuccess;
+}
 
 // One candidate tau: its encoding sizes, device memory and analytic time.
 struct TauRow {
@@ -538,27 +699,19 @@ struct TauRow {
 // Analytic cost of tau on GB300: tensor-core time for the one-hot columns plus
 // the rare term (fused pair-list walk, or the dense rare-count build), subject
 // to device memory.
-std::vector<TauRow> tau_rows(const std::vector<uint32_t>& cnt_flat, const std::vector<uint64_t>& off, int n, int L,
-                             size_t free_bytes, const TauModel& m, bool dense) {
+std::vector<TauRow> tau_rows(const CountBins& bins, int n, int L, size_t free_bytes, const TauModel& m, bool dense) {
     // the candidates are powers of two, so an allele is frequent at tau = 2^t
-    // exactly when floor(log2(count)) >= t: one pass bins the counts by that,
-    // and every candidate sums whole bins (the sums are integers far below 2^53,
-    // exact in double whatever their order)
-    constexpr int kBins = 33;
+    // exactly when floor(log2(count)) >= t: every candidate sums whole bins (the
+    // sums are integers far below 2^53, exact in double); a single row is no pair
     double bn[kBins] = {}, bsq[kBins] = {}, br[kBins] = {}, bcells[kBins] = {};
-    for (int k = 0; k < L; k++)
-        for (uint64_t q = off[k] + 1; q < off[k + 1]; q++) {
-            const uint32_t c = cnt_flat[q];
-            if (!c) continue;
-            const int b = 31 - __builtin_clz(c);
-            const double v = (double)c;
-            bn[b] += 1.0;
-            bsq[b] += v * v;
-            if (c >= 2) {
-                br[b] += v * (v - 1.0) / 2.0;
-                bcells[b] += v;
-            }
+    for (int b = 0; b < kBins; b++) {
+        bn[b] = (double)bins.n[b];
+        bsq[b] = (double)bins.sq[b];
+        if (b) {
+            br[b] = (double)((bins.sq[b] - bins.sum[b]) / 2);
+            bcells[b] = (double)bins.sum[b];
         }
+    }
     const double pairs = (double)n * (double)(n - 1) / 2.0;
     const size_t rows = up((size_t)std::max(n, 1), 256);
     const double nl = (double)n * (double)L;
@@ -606,14 +759,12 @@ int choose_tau_analytic(const std::vector<TauRow>& rows) {
 }
 
 // Feature rows of the candidates that fit (the layout tch.h documents).
-void tau_features(const std::vector<TauRow>& rows, const std::vector<uint32_t>& cnt_flat,
-                  const std::vector<uint64_t>& off, int n, int L, TauTable* t) {
+void tau_features(const std::vector<TauRow>& rows, const CountBins& bins, const std::vector<uint64_t>& off, int n, int L,
+                  TauTable* t) {
     std::vector<double> lnd((size_t)L);
     double present = 0;
-    for (int k = 0; k < L; k++) {
-        lnd[k] = log1p((double)(off[k + 1] - off[k] - 1));
-        for (uint64_t q = off[k] + 1; q < off[k + 1]; q++) present += cnt_flat[q];
-    }
+    for (int k = 0; k < L; k++) lnd[k] = log1p((double)(off[k + 1] - off[k] - 1));
+    for (int b = 0; b < kBins; b++) present += (double)bins.sum[b];
     std::sort(lnd.begin(), lnd.end());
     auto quant = [&](double f) { return L ? lnd[(size_t)std::min<double>(L - 1, f * (L - 1) + 0.5)] : 0.0; };
     const double nl = std::max(1.0, (double)n * (double)L);
@@ -676,16 +827,16 @@ int choose_tau_query(const std::vector<TauRow>& rows, int n, const TauModel& m, 
 // term in several and take the analytic pick (on 200 000 x 3 000 Zipf profiles
 // the learned pick ran 440 ms against the analytic 356 ms).
 constexpr int kLearnedMaxRows = 65536;
-int choose_tau_gb300(int device, const std::vector<uint32_t>& cnt_flat, const std::vector<uint64_t>& off, int n,
-                     int L, size_t free_bytes, const TauModel& m, bool dense, bool verbose, int* sub, int* group) {
-    const std::vector<TauRow> rows = tau_rows(cnt_flat, off, n, L, free_bytes, m, dense);
+int choose_tau_gb300(int device, const CountBins& bins, const std::vector<uint64_t>& off, int n, int L,
+                     size_t free_bytes, const TauModel& m, bool dense, bool verbose, int* sub, int* group) {
+    const std::vector<TauRow> rows = tau_rows(bins, n, L, free_bytes, m, dense);
     const int analytic = choose_tau_analytic(rows);
     int learned = 0, lsub = 0, lgroup = 0;
     std::vector<float> pred;
     TauTable t;
     float w[kMlpParams];
     if (n <= kLearnedMaxRows && tau_mlp_weights(w)) {
-        tau_features(rows, cnt_flat, off, n, L, &t);
+        tau_features(rows, bins, off, n, L, &t);
         pred.resize(t.taus.size());
         Err quiet{nullptr, 0};
         if (!t.taus.empty() && !mlp_run(device, w, t.feats.data(), nullptr, (int)t.taus.size(), pred.data(), nullptr,
@@ -736,7 +887,11 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
     int32_t* col_d = nullptr;
     unsigned long long* slot_ids = nullptr;
     int* err_d = nullptr;
-    std::vector<uint32_t> nd_h(L), cnt_h;
+    std::vector<uint32_t> nd_h(L);
+    CountBins bins_h;
+    CountBins* bins_d = nullptr;
+    LocusTotals* totals_d = nullptr;
+    Working work;
     std::vector<uint64_t> off_h((size_t)L + 1, 0);
     *out = DeviceEncoding();
     out->n = n;
@@ -754,9 +909,10 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
 
     TCH_CK(e, cudaSetDevice(device));
     TCH_CK(e, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    TCH_CK(e, dalloc(&err_d, 1, nullptr));
+    TCH_CK(e, working_pool(device, &work.pool));
+    TCH_CK(e, work.get(&err_d, 1));
     TCH_CK(e, cudaMemset(err_d, 0, sizeof(int)));
-    TCH_CK(e, dalloc(&nd, (size_t)L, nullptr));
+    TCH_CK(e, work.get(&nd, (size_t)L));
     TCH_CK(e, cudaMemset(nd, 0, (size_t)L * 4));
     TCH_CK(e, dalloc(&out->x, (size_t)n * L, &out->bytes));
     TCH_CK(e, dalloc(&cnt_off_d, (size_t)L + 1, nullptr));
@@ -771,11 +927,11 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
         // loci per batch: hash tables + id lists within ~2 GB
         nk_max = (int)std::max<size_t>(
             1, std::min<size_t>((size_t)L, ((size_t)2 << 30) / (C * (8 + 4 + 2) + (size_t)lcap * 12)));
-        TCH_CK(e, dalloc(&keys, C * nk_max, &tmp_bytes));
-        TCH_CK(e, dalloc(&cnts, C * nk_max, &tmp_bytes));
-        TCH_CK(e, dalloc(&rank_slot, C * nk_max, &tmp_bytes));
-        TCH_CK(e, dalloc(&list_keys, (size_t)lcap * nk_max, &tmp_bytes));
-        TCH_CK(e, dalloc(&list_slots, (size_t)lcap * nk_max, &tmp_bytes));
+        TCH_CK(e, work.get(&keys, C * nk_max));
+        TCH_CK(e, work.get(&cnts, C * nk_max));
+        TCH_CK(e, work.get(&rank_slot, C * nk_max));
+        TCH_CK(e, work.get(&list_keys, (size_t)lcap * nk_max));
+        TCH_CK(e, work.get(&list_slots, (size_t)lcap * nk_max));
         for (int k0 = 0; k0 < L && !again; k0 += nk_max) {
             const int nk = std::min(nk_max, L - k0);
             TCH_CK(e, cudaMemset(keys, 0, C * nk * sizeof(unsigned long long)));
@@ -800,18 +956,18 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
         }
         if (again) {
             logC = full_log;
-            cudaFree(keys); keys = nullptr;
-            cudaFree(cnts); cnts = nullptr;
-            cudaFree(rank_slot); rank_slot = nullptr;
-            cudaFree(list_keys); list_keys = nullptr;
-            cudaFree(list_slots); list_slots = nullptr;
+            work.drop(&keys);
+            work.drop(&cnts);
+            work.drop(&rank_slot);
+            work.drop(&list_keys);
+            work.drop(&list_slots);
             TCH_CK(e, cudaMemset(err_d, 0, sizeof(int)));
             TCH_CK(e, cudaMemset(nd, 0, (size_t)L * 4));
             continue;
         }
         // flat counts need every offset: a second sweep ranks the batches
         TCH_CK(e, cudaMemcpy(cnt_off_d, off_h.data(), ((size_t)L + 1) * 8, cudaMemcpyHostToDevice));
-        TCH_CK(e, dalloc(&cnt_flat, off_h[L], &tmp_bytes));
+        TCH_CK(e, work.get(&cnt_flat, off_h[L]));
         TCH_CK(e, cudaMemset(cnt_flat, 0, std::max<uint64_t>(off_h[L], 1) * 4));
         if (query_maps) {
             TCH_CK(e, dalloc(&slot_ids, off_h[L], nullptr));
@@ -835,68 +991,68 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
                                                                       out->x, err_d);
             TCH_CK(e, cudaGetLastError());
         }
+        TCH_CK(e, work.get(&bins_d, 1));
+        TCH_CK(e, cudaMemset(bins_d, 0, sizeof(CountBins)));
+        count_bins_kernel<<<grid_for(std::max<uint64_t>(off_h[L], 1), sms), 256>>>(cnt_flat, off_h[L], bins_d);
+        TCH_CK(e, cudaGetLastError());
+        TCH_CK(e, cudaMemcpy(&bins_h, bins_d, sizeof(bins_h), cudaMemcpyDeviceToHost));
         TCH_CK(e, cudaMemcpy(&hflag, err_d, sizeof(int), cudaMemcpyDeviceToHost));
         if (hflag) { e.set("device encoder: hash table error 0x%x", hflag); goto fail; }
-        cnt_h.resize(off_h[L]);
-        if (off_h[L]) TCH_CK(e, cudaMemcpy(cnt_h.data(), cnt_flat, off_h[L] * 4, cudaMemcpyDeviceToHost));
     }
-    cudaFree(keys); keys = nullptr;
-    cudaFree(cnts); cnts = nullptr;
-    cudaFree(rank_slot); rank_slot = nullptr;
-    cudaFree(list_keys); list_keys = nullptr;
-    cudaFree(list_slots); list_slots = nullptr;
+    work.drop(&keys);
+    work.drop(&cnts);
+    work.drop(&rank_slot);
+    work.drop(&list_keys);
+    work.drop(&list_slots);
 
     mark("ranks and counts");
     // ---- host: tau, frequent columns, rare groups
     {
         int tau = tau_req;
+        TCH_CK(e, cudaStreamSynchronize(0));  // the pool lets go of what it does not keep
         TCH_CK(e, cudaMemGetInfo(&freeb, &totb));
         if (table) {  // candidates and features only
-            tau_features(tau_rows(cnt_h, off_h, n, L, freeb, model, dense_rare), cnt_h, off_h, n, L, table);
+            tau_features(tau_rows(bins_h, n, L, freeb, model, dense_rare), bins_h, off_h, n, L, table);
             free_device_encoding(out);
             goto done;
         }
         if (tau <= 0) {
-            tau = query_maps ? choose_tau_query(tau_rows(cnt_h, off_h, n, L, freeb, model, true), n, model, verbose)
-                             : choose_tau_gb300(device, cnt_h, off_h, n, L, freeb, model, dense_rare, verbose,
+            tau = query_maps ? choose_tau_query(tau_rows(bins_h, n, L, freeb, model, true), n, model, verbose)
+                             : choose_tau_gb300(device, bins_h, off_h, n, L, freeb, model, dense_rare, verbose,
                                                 &out->sub_rows, &out->tile_group);
             if (!tau) { e.set("no tau fits in %.2f GB of free device memory", freeb / 1e9); goto fail; }
         }
         out->tau = tau;
-        std::vector<int32_t> col(off_h[L], -1);
+        // a query database also keeps single-row groups: a new profile with that
+        // allele equals its one row
+        const uint32_t least = query_maps ? 1 : 2;
+        std::vector<LocusTotals> totals((size_t)L);
+        TCH_CK(e, work.get(&totals_d, (size_t)L));
+        const unsigned lgrid = (unsigned)((L + 7) / 8);
+        locus_totals_kernel<<<lgrid, 256>>>(cnt_flat, cnt_off_d, L, (uint32_t)tau, least, totals_d);
+        TCH_CK(e, cudaGetLastError());
+        TCH_CK(e, cudaMemcpy(totals.data(), totals_d, (size_t)L * sizeof(LocusTotals), cudaMemcpyDeviceToHost));
         std::vector<uint32_t> base((size_t)L + 1, 0);
-        std::vector<uint64_t> goff(off_h[L] + 1, 0);
-        std::vector<uint64_t> groups, large;  // (first, end, locus) of the rare groups, by size
+        LocusTotals sum = {};
         double n_rare_pairs = 0;
         uint64_t D = 0;
         for (int k = 0; k < L; k++) {
+            const LocusTotals t = totals[k];
             base[k] = (uint32_t)D;
-            uint32_t d = 0;
-            for (uint64_t q = off_h[k]; q < off_h[k + 1]; q++) {
-                const bool is_rank = q > off_h[k];
-                const uint32_t c = cnt_h[q];
-                const bool freq = is_rank && c >= (uint32_t)tau;
-                if (freq) col[q] = (int32_t)d++;
-                // a query database also keeps single-row groups: a new profile with that
-                // allele equals its one row
-                const bool rare = is_rank && !freq && c >= (query_maps ? 1u : 2u);
-                goff[q + 1] = goff[q] + (rare ? c : 0);
-                if (rare) {
-                    std::vector<uint64_t>& list = c <= (uint32_t)kWarpGroup ? groups : large;
-                    list.push_back(goff[q]);
-                    list.push_back(goff[q + 1]);
-                    list.push_back((uint64_t)k);
-                    n_rare_pairs += (double)c * (double)(c - 1) / 2.0;
-                }
-            }
-            D += d;
+            totals[k] = sum;
+            D += t.columns;
+            sum.members += t.members;
+            sum.small += t.small;
+            sum.large += t.large;
+            n_rare_pairs += (double)t.pairs;
         }
         base[L] = (uint32_t)D;
         out->D = D;
         if (fp4_columns(L, D) / 2 > (size_t)INT32_MAX) { e.set("%llu one-hot columns: too many", (unsigned long long)D); goto fail; }
         out->kb = (int)(fp4_columns(L, D) / 2);
         out->x_rows = up((size_t)std::max(n, 1), 256);
-        const uint64_t n_members = goff[off_h[L]];
+        const uint64_t n_members = sum.members;
+        const size_t nsmall = sum.small, nlarge = sum.large, ngroups = nsmall + nlarge;
         if (dense_rare && n_members >= (1ull << 32)) {
             e.set("%llu rare cells: more than 2^32 (lower tau)", (unsigned long long)n_members);
             goto fail;
@@ -904,9 +1060,12 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
         TCH_CK(e, dalloc(&col_d, off_h[L], nullptr));
         TCH_CK(e, dalloc(&base_d, (size_t)L + 1, nullptr));
         TCH_CK(e, dalloc(&goff_d, off_h[L] + 1, nullptr));
-        if (off_h[L]) TCH_CK(e, cudaMemcpy(col_d, col.data(), off_h[L] * 4, cudaMemcpyHostToDevice));
+        TCH_CK(e, work.get(&groups_d, 3 * ngroups));
         TCH_CK(e, cudaMemcpy(base_d, base.data(), ((size_t)L + 1) * 4, cudaMemcpyHostToDevice));
-        TCH_CK(e, cudaMemcpy(goff_d, goff.data(), (off_h[L] + 1) * 8, cudaMemcpyHostToDevice));
+        TCH_CK(e, cudaMemcpy(totals_d, totals.data(), (size_t)L * sizeof(LocusTotals), cudaMemcpyHostToDevice));
+        locus_tables_kernel<<<lgrid, 256>>>(cnt_flat, cnt_off_d, L, (uint32_t)tau, least, totals_d, sum.small, col_d, goff_d,
+                                            groups_d);
+        TCH_CK(e, cudaGetLastError());
 
         mark("tau and column maps");
         // ---- 4: operand rows: pos by nibble, neg from pos
@@ -925,9 +1084,7 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
 
         mark("operand rows");
         // ---- 5: rare groups, sorted
-        const size_t nsmall = groups.size() / 3, nlarge = large.size() / 3, ngroups = nsmall + nlarge;
-        groups.insert(groups.end(), large.begin(), large.end());
-        TCH_CK(e, dalloc(&members, n_members, &tmp_bytes));
+        TCH_CK(e, work.get(&members, n_members));
         // row runs where they are used (triangle solves) and their packed prefix
         // holds; two-byte members where every row index fits
         const int piece = n <= 65536 ? 8 : 4;
@@ -935,15 +1092,13 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
         const bool narrow = runs && n <= 65536;
         if (narrow) TCH_CK(e, dalloc(&sorted16, n_members + 8, &tmp_bytes));  // the last piece is loaded whole
         else TCH_CK(e, dalloc(&sorted, n_members + 4, &tmp_bytes));
-        TCH_CK(e, dalloc(&gfill, off_h[L], &tmp_bytes));
+        TCH_CK(e, work.get(&gfill, off_h[L]));
         TCH_CK(e, cudaMemset(gfill, 0, std::max<uint64_t>(off_h[L], 1) * 4));
         if (dense_rare) {  // cells in no rare group keep the sentinel: the rare counts skip them
             TCH_CK(e, dalloc(&mpos, (size_t)n * L, &tmp_bytes));
             TCH_CK(e, cudaMemset(mpos, 0xFF, std::max<size_t>((size_t)n * L, 1) * 4));
         }
         if (ngroups) {
-            TCH_CK(e, dalloc(&groups_d, groups.size(), &tmp_bytes));
-            TCH_CK(e, cudaMemcpy(groups_d, groups.data(), groups.size() * 8, cudaMemcpyHostToDevice));
             group_fill_kernel<<<grid_for((size_t)n * L, sms), 256>>>(out->x, n, L, cnt_off_d, goff_d, gfill, members);
             TCH_CK(e, cudaGetLastError());
             const SortedGroups sg{sorted, sorted16, mpos, L};
@@ -974,7 +1129,7 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
         }
         mark("rare groups");
         if (runs) {  // the partner runs of every row, for triangle solves
-            TCH_CK(e, dalloc(&row_count, (size_t)n, &tmp_bytes));
+            TCH_CK(e, work.get(&row_count, (size_t)n));
             const int rgrid = (int)std::min<size_t>(((size_t)n + 7) / 8, (size_t)sms * 16);
             row_runs_kernel<<<rgrid, 256>>>(out->x, n, L, cnt_off_d, goff_d, mpos, piece, 0, row_count, nullptr, nullptr,
                                             nullptr, nullptr);
@@ -1024,8 +1179,8 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
             goto done;
         }
         // ---- 6: CSR of rare pairs, ascending per row
-        TCH_CK(e, dalloc(&row_count, (size_t)n, &tmp_bytes));
-        TCH_CK(e, dalloc(&start64, (size_t)n + 1, &tmp_bytes));
+        TCH_CK(e, work.get(&row_count, (size_t)n));
+        TCH_CK(e, work.get(&start64, (size_t)n + 1));
         const int rr_smem = kJC * 2;
         TCH_CK(e, cudaFuncSetAttribute(rare_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, rr_smem));
         const int rr_grid = std::max(1, std::min(n, sms * 1));
@@ -1063,15 +1218,12 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
         mark("rare CSR (2 passes)");
     }
 done:
-    cudaFree(err_d); cudaFree(nd); cudaFree(cnt_off_d); cudaFree(cnt_flat); cudaFree(col_d); cudaFree(base_d);
-    cudaFree(goff_d); cudaFree(members); cudaFree(sorted); cudaFree(sorted16); cudaFree(wpos); cudaFree(gfill); cudaFree(groups_d); cudaFree(row_count);
-    cudaFree(start64); cudaFree(mpos); cudaFree(slot_ids);
+    cudaFree(cnt_off_d); cudaFree(col_d); cudaFree(base_d); cudaFree(goff_d); cudaFree(sorted); cudaFree(sorted16);
+    cudaFree(wpos); cudaFree(mpos); cudaFree(slot_ids);
     return 0;
 fail:
-    cudaFree(err_d); cudaFree(nd); cudaFree(cnt_off_d); cudaFree(cnt_flat); cudaFree(col_d); cudaFree(base_d);
-    cudaFree(goff_d); cudaFree(members); cudaFree(sorted); cudaFree(sorted16); cudaFree(wpos); cudaFree(gfill); cudaFree(groups_d); cudaFree(row_count);
-    cudaFree(start64); cudaFree(keys); cudaFree(cnts); cudaFree(rank_slot); cudaFree(list_keys); cudaFree(list_slots);
-    cudaFree(mpos); cudaFree(slot_ids);
+    cudaFree(cnt_off_d); cudaFree(col_d); cudaFree(base_d); cudaFree(goff_d); cudaFree(sorted); cudaFree(sorted16);
+    cudaFree(wpos); cudaFree(mpos); cudaFree(slot_ids);
     free_device_encoding(out);
     return 1;
 }

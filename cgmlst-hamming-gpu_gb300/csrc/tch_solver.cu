@@ -343,6 +343,7 @@ static int solver_from_input(int device, int n, int L, const uint64_t* calls, co
     tch_solver* s = nullptr;
     uint64_t* d_calls = nullptr;
     uint16_t* d_ranks = nullptr;
+    cudaMemPool_t pool = nullptr;
     DeviceEncoding enc;
     *out = nullptr;
     if (n < 0 || L < 0) return e.set("negative size (n=%d, L=%d)", n, L);
@@ -363,19 +364,21 @@ static int solver_from_input(int device, int n, int L, const uint64_t* calls, co
     TCH_CK(e, cudaDeviceGetAttribute(&s->num_sms, cudaDevAttrMultiProcessorCount, device));
     TCH_CK(e, dmalloc(s, (void**)&s->dErr, sizeof(int)));
     TCH_CK(e, cudaMemset(s->dErr, 0, sizeof(int)));
-    if (!dev_calls) TCH_CK(e, cudaMalloc(&d_calls, std::max<size_t>((size_t)n * Le, 1) * 8));
+    TCH_CK(e, working_pool(device, &pool));
+    if (!dev_calls)
+        TCH_CK(e, cudaMallocFromPoolAsync((void**)&d_calls, std::max<size_t>((size_t)n * Le, 1) * 8, pool, 0));
     if (dev_calls) {
         // read in place
     } else if (L && ranks) {
         const size_t count = (size_t)n * L;
-        TCH_CK(e, cudaMalloc(&d_ranks, std::max<size_t>(count, 1) * 2));
+        TCH_CK(e, cudaMallocFromPoolAsync((void**)&d_ranks, std::max<size_t>(count, 1) * 2, pool, 0));
         if (count) {
             TCH_CK(e, cudaMemcpy(d_ranks, ranks, count * 2, cudaMemcpyHostToDevice));
             widen_ranks_kernel<<<(int)std::min<size_t>((count + 255) / 256, (size_t)s->num_sms * 32), 256>>>(
                 d_ranks, count, d_calls);
             TCH_CK(e, cudaGetLastError());
         }
-        cudaFree(d_ranks);
+        cudaFreeAsync(d_ranks, 0);
         d_ranks = nullptr;
     } else if (L) {
         if ((size_t)n * L) TCH_CK(e, cudaMemcpy(d_calls, calls, (size_t)n * L * 8, cudaMemcpyHostToDevice));
@@ -385,7 +388,7 @@ static int solver_from_input(int device, int n, int L, const uint64_t* calls, co
     if (encode_on_device(device, n, Le, dev_calls ? dev_calls : d_calls, tau, g_tau_model, verbose, max_chunk_bytes(),
                          rare_dense_default() ? ENC_DENSE : 0, &enc, e))
         goto fail;
-    cudaFree(d_calls);
+    if (d_calls) cudaFreeAsync(d_calls, 0);
     d_calls = nullptr;
     if (enc.dense) {  // the solver takes the rare groups
         s->dense = true;
@@ -426,8 +429,8 @@ static int solver_from_input(int device, int n, int L, const uint64_t* calls, co
     *out = s;
     return 0;
 fail:
-    if (d_calls) cudaFree(d_calls);
-    if (d_ranks) cudaFree(d_ranks);
+    if (d_calls) cudaFreeAsync(d_calls, 0);
+    if (d_ranks) cudaFreeAsync(d_ranks, 0);
     solver_free(s);
     return 1;
 }

@@ -194,3 +194,36 @@ def test_distinct_counts_around_table_sizes(pkg, distinct):
         t = torch.from_numpy(A.view(np.int64)).cuda()
         want = sum((t[:, k, None] != t[None, :, k]).to(torch.int16) for k in range(A.shape[1]))
         assert bool((torch.triu(d[:, :n], 1) == torch.triu(want, 1)).all())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tau", [1, 2, 32, 128, 129, 130, 1000])
+def test_tables_around_group_sizes(pkg, tau):
+    """Alleles seen 1, 2, 31-33, 127-129 and 300 times at loci of 1 to 70
+    alleles: the encoding's sizes against the host encoder's, the distances
+    against the count, with tau on either side of every size."""
+    rng = np.random.default_rng(tau)
+    n, sizes = 900, [1, 2, 31, 32, 33, 127, 128, 129, 300]
+    cols = []
+    for k in range(12):
+        col, left, a = [], n, 1
+        if k >= 8:
+            col = [1000 + i for i in range(60)]  # more alleles than lanes
+            left -= 60
+        for size in rng.permutation(sizes):
+            if size <= left:
+                col += [a] * int(size)
+                left -= int(size)
+                a += 1
+        cols.append(rng.permutation(np.array(col + [0] * left)))
+    A = np.stack(cols, axis=1).astype(np.uint64)
+    x, nd = pkg.dense_ranks(A)
+    want = oracle.hamming(x)
+    counts = [np.bincount(x[:, k])[1:] for k in range(x.shape[1])]
+    with pkg.Solver.from_calls(A, tau=tau) as s:
+        info = s.info()
+        assert info["d_onehot"] == sum(int((c >= tau).sum()) for c in counts)
+        assert info["n_rare"] == sum(int((c * (c - 1) // 2)[(c < tau) & (c >= 2)].sum()) for c in counts)
+        H, _ = s.run(200)
+    iu = np.triu_indices(n, 1)
+    np.testing.assert_array_equal(H[iu], want[iu])
