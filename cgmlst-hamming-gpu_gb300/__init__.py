@@ -490,8 +490,9 @@ class Tsv:
         self._text = bytes(text)
         self._h = ctypes.c_void_p()
         err = _errbuf()
-        buf = ctypes.create_string_buffer(self._text, len(self._text))
-        _check(lib().tch_tsv_parse(device, ctypes.cast(buf, ctypes.c_void_p), len(self._text),
+        # the bytes object's own buffer (a copy of 50 MB took 6 ms, the whole parse 1)
+        buf = ctypes.cast(ctypes.c_char_p(self._text), ctypes.c_void_p)
+        _check(lib().tch_tsv_parse(device, buf, len(self._text),
                                    sep.encode()[:1], 1 if skip_repl else 0, missing.encode(), ctypes.byref(self._h),
                                    err, len(err)), err)
 
