@@ -447,7 +447,7 @@ struct RareJob {
 };
 
 template <int T>
-__global__ void __launch_bounds__(T, 1024 / T)
+__global__ void __launch_bounds__(T, 1536 / T)
     rare_batch_kernel(const RareJob* __restrict__ jobs, const int* __restrict__ row_job, int total_rows,
                       int cwords) {
     extern __shared__ uint4 smem_rd[];
