@@ -22,7 +22,7 @@
 // A CTA pair (cluster of two, tcgen05 cta_group::2) per tile, 10 warps per
 // CTA, one CTA per SM, persistent over the stripe's tiles (upper triangle
 // only, or every tile of a rectangle):
-//   warp 0    TMA producer   7-stage ring of (A 128 x 128 B, B 120 x 128 B): each
+//   warp 0    TMA producer   ring of 6 or 7 stages (A 128 x 128 B, B 120 x 128 B): each
 //                            CTA its 128 rows of A and its half of the columns'
 //                            rows, completing on the first CTA's barrier
 //   warp 1    MMA issuer     (first CTA) 4 x tcgen05.mma (M 256, N 240, K = 64
@@ -37,13 +37,14 @@
 // Tiles are visited in raster groups of row blocks, column-major inside a
 // group, so that the pairs running at the same time share A and B tiles in L2.
 //
-// What bounds it: a stage's MMAs take 480 cycles (16 384 MACs per cycle and
-// SM, the probe's rate) and its operands 496 (31 KB per CTA at the 64 bytes a
-// cycle that an SM takes in from L2), so the pass runs at both limits inside a
-// tile (503 cycles per stage measured) plus about 1.9 us per tile, half of it
-// the tile's rare counts coming in.  One CTA per tile (128 x 224) takes 44 KB
-// for 448 cycles of MMAs and stops at 0.61 of the probe's rate: 8.46 ms for the
-// triangle of 63 005 long-tail profiles at tau 1 024, 6.24 ms in pairs (0.83).
+// What bounds it: the shared-memory data path.  A stage's 31 KB per CTA are
+// written by TMA and read by the MMAs at 128 bytes a cycle, 496 cycles in all (as
+// many as the 64 bytes a cycle that an SM takes in from L2 allow), while its MMAs
+// take 480 (16 384 MACs per cycle and SM, the probe's rate); 503 cycles per stage
+// measured, and the epilogue's accesses come on top, 1.9 us per tile with seven
+// stages.  One CTA per tile (128 x 224) takes 44 KB for 448 cycles of MMAs and
+// stops at 0.61 of the probe's rate: 8.46 ms for the triangle of 63 005 long-tail
+// profiles at tau 1 024, 5.95 ms in pairs (0.88).
 // Three more things were needed to get there, each measured on that triangle
 // (8.38 ms as a plain pair):
 //   - the next stage's barrier is looked at before a stage's MMAs are issued:
@@ -52,7 +53,8 @@
 //   - the epilogue touches whole 64-byte row pieces (8.18 -> 7.60, below);
 //   - producer and issuer run under elect.sync (7.60 -> 6.27): under
 //     `lane == 0` an MMA takes 86 cycles to issue, as its descriptors move
-//     through vector registers.
+//     through vector registers;
+// raster groups of 16 and the smaller shared-memory configuration did the rest.
 //
 // Every mbarrier wait is bounded (about 2 s of %globaltimer); on a timeout the
 // CTA records DEVERR_TIMEOUT, stops issuing work, drains what it issued,
@@ -73,7 +75,13 @@ constexpr int PM = 2 * BM;          // tile rows of a CTA pair (MMA M)
 constexpr int BN = 240;             // tile columns (MMA N)
 constexpr int BH = BN / 2;          // column rows staged by each CTA of the pair
 constexpr int BK = 128;             // bytes of K per stage: one 128-byte swizzle row, 256 elements
-constexpr int STAGES = 7;
+// Stages of the ring: seven fit, but with six the 196 KB configuration of shared
+// memory leaves the epilogue's loads 32 KB more of L1.  63 005 profiles, tau 1 024
+// (50 stages of K per tile): 6.19 ms with seven, 5.95 with six (6.42 with six in
+// the 228 KB configuration); 12 011 founders with 997 stages of K: 4.22 and 4.34;
+// alike with 81 stages, and for many sets in one launch.
+constexpr int FEW_STAGES = 6, ALL_STAGES = 7;
+constexpr int FEW_STAGES_K = 100;  // six up to this many stages of K per tile
 constexpr int A_BYTES = BM * BK;    // 16 KB
 constexpr int B_BYTES = BH * BK;    // 15 KB
 constexpr int STAGE_BYTES = A_BYTES + B_BYTES;  // of one CTA
@@ -89,8 +97,8 @@ constexpr int WARP_CHUNKS = (CHUNKS + 1) / 2;  // chunks of the first column hal
 // 1 024: 4 -> 6.82 ms, 8 -> 6.31, 16 -> 6.24, 32 -> 6.40
 constexpr int GROUP_M = 16;
 constexpr int BAR_BYTES = 256;
-constexpr int SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + BAR_BYTES;
-static_assert(SMEM_BYTES <= 232448, "shared memory per CTA");
+constexpr int smem_bytes(int stages) { return 1024 + stages * STAGE_BYTES + BAR_BYTES; }
+static_assert(smem_bytes(ALL_STAGES) <= 232448, "shared memory per CTA");
 static_assert(BN % 16 == 0 && BN <= 256 && ACC_STRIDE + BN <= SF_COL && SF_COL + 32 <= TMEM_COLS, "TMEM layout");
 static_assert(ACC_STRIDE + CHUNKS * CHUNK <= TMEM_COLS, "the last chunk's loads stay inside TMEM");
 static_assert(BH % 8 == 0, "whole 8-row swizzle atoms per CTA");
@@ -269,7 +277,7 @@ __device__ __forceinline__ uint32_t pack_u16(uint32_t v0, uint32_t v1, bool* bad
     return __byte_perm(__float_as_uint(x0), __float_as_uint(x1), 0x5410);
 }
 
-template <bool MULTI>
+template <bool MULTI, int STAGES>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
     tc_stripe_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -604,13 +612,25 @@ bool make_map(CUtensorMap* m, const uint8_t* X, size_t rows, int kb, int box_row
 
 bool same_chunking(const KChunks& x, const KChunks& y) { return x.n == y.n && x.width == y.width && x.kb == y.kb; }
 
+// Shared memory of one CTA, and the smallest configuration of it: left to itself
+// a launch beside the rare counts' tail stays in theirs (228 KB).
+template <bool MULTI, int STAGES>
+cudaError_t set_attributes() {
+    constexpr int bytes = smem_bytes(STAGES);
+    const auto kernel = tc_stripe_kernel<MULTI, STAGES>;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess) return e;
+    constexpr int kPercent = (100 * (bytes + 1024) + 228 * 1024 - 1) / (228 * 1024);
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, kPercent);
+}
+
 cudaError_t launch_one(const Fp4Operands& A, const Fp4Operands& B, const uint16_t* R, size_t ldr,
                        const StripeArgs& a, int num_sms, cudaStream_t st) {
     static bool attrs[kMaxDevices] = {};
     const int dev = current_device();
     if (!attrs[dev]) {
-        const cudaError_t e = cudaFuncSetAttribute(tc_stripe_kernel<false>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+        cudaError_t e = set_attributes<false, FEW_STAGES>();
+        if (e == cudaSuccess) e = set_attributes<false, ALL_STAGES>();
         if (e != cudaSuccess) return e;
         attrs[dev] = true;
     }
@@ -664,7 +684,10 @@ cudaError_t launch_one(const Fp4Operands& A, const Fp4Operands& B, const uint16_
     p.tile_job = nullptr;
     if (p.num_tiles == 0) return cudaSuccess;
     const int grid = 2 * std::min(p.num_tiles, std::max(num_sms / 2, 1));
-    return launch_after(a.after_counts, tc_stripe_kernel<false>, dim3((unsigned)grid), THREADS, SMEM_BYTES, st, maps, p);
+    const bool few = p.kblocks <= FEW_STAGES_K;
+    return launch_after(a.after_counts,
+                        few ? tc_stripe_kernel<false, FEW_STAGES> : tc_stripe_kernel<false, ALL_STAGES>,
+                        dim3((unsigned)grid), THREADS, smem_bytes(few ? FEW_STAGES : ALL_STAGES), st, maps, p);
 }
 
 }  // namespace
@@ -733,7 +756,7 @@ cudaError_t tc_batch_prepare(const std::vector<TcBatchItem>& items, int num_sms,
     static bool attrs[kMaxDevices] = {};
     const int dev = current_device();
     if (!attrs[dev]) {
-        e = cudaFuncSetAttribute(tc_stripe_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+        e = set_attributes<true, ALL_STAGES>();
         if (e != cudaSuccess) return e;
         attrs[dev] = true;
     }
@@ -752,7 +775,8 @@ cudaError_t launch_tc_batch(const TcBatchPlan& plan, cudaStream_t st) {
     p.jmaps = static_cast<const CUtensorMap*>(plan.d_maps);
     p.tile_job = static_cast<const int*>(plan.d_tile_job);
     // straight after the batch's rare counts
-    return launch_after(true, tc_stripe_kernel<true>, dim3((unsigned)plan.grid), THREADS, SMEM_BYTES, st, maps, p);
+    return launch_after(true, tc_stripe_kernel<true, ALL_STAGES>, dim3((unsigned)plan.grid), THREADS,
+                        smem_bytes(ALL_STAGES), st, maps, p);
 }
 
 void tc_batch_release(TcBatchPlan* plan) {
