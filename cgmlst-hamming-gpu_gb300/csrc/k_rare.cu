@@ -22,7 +22,7 @@
 // lanes of a warp on one bank, so an atomic takes 3.4 of the L1's data cycles,
 // and with the member loads and the run cursor those are 75-79 % busy (ncu,
 // 12 011 x 5 000 founders); at the margin it counts 2.0e12 pairs/s, of 6.7 per
-// cycle and SM.  63 005 x 1 142 long-tail, tau 1 024 (3.4e9 pairs): 2.83 ms,
+// cycle and SM.  63 005 x 1 142 long-tail, tau 1 024 (3.4e9 pairs): 2.69 ms,
 // 4.72 before, when each member went through the run cursor by itself and one
 // 1 024-thread CTA per SM took every row; 0.6 ms of it is the 4 GB block.
 
@@ -757,6 +757,13 @@ static cudaError_t launch_rare_runs(const RareGroups& g, int r0, int rows, uint1
     // dependent steps overlap (5 000 profiles, tau 64: 0.039 ms, with 512 threads
     // 0.060; from 8 192 columns on the two are alike)
     constexpr int kNarrow = 8192;
+    // sets with more than 32 768 rare pairs per row keep many warps per row busy:
+    // 256 threads a row, a CTA each, up to 20 480 columns (10 000 x 1 142, tau 1 024,
+    // 91 000 pairs per row: 0.552 ms, with 512 and 128 threads 0.658; 12 011
+    // founders: 4.04 and 4.60; wider rows run better on 512: 63 005 profiles 2.69
+    // ms, 2.89 when 256 threads take them up to 28 672)
+    const bool heavy = g.pairs > (size_t)32768 * g.n;
+    constexpr int kHeavyWidth = 20480;
     cudaError_t e = cudaSuccess;
     static bool attrs[kMaxDevices] = {};  // once per device (also keeps it out of graph captures)
     bool& attr = attrs[current_device()];
@@ -765,6 +772,7 @@ static cudaError_t launch_rare_runs(const RareGroups& g, int r0, int rows, uint1
         e = cudaFuncSetAttribute(rare_runs_kernel<1024, M>, at, runs_room(1));
         if (e == cudaSuccess) e = cudaFuncSetAttribute(rare_runs_kernel<512, M>, at, runs_room(1));
         if (e == cudaSuccess) e = cudaFuncSetAttribute(rare_runs_kernel<NT, M>, at, runs_room(1));
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(rare_runs_kernel<256, M>, at, runs_room(1));
         if (e != cudaSuccess) return e;
         attr = true;
     }
@@ -777,11 +785,12 @@ static cudaError_t launch_rare_runs(const RareGroups& g, int r0, int rows, uint1
             e = launch_runs<1024, M>(g, r0, ra, rb, R, ldr, cend, 1, true, sms, st);
         } else if ((rb = wider(28672)) > ra) {
             e = launch_runs<512, M>(g, r0, ra, rb, R, ldr, cend, 2, true, sms, st);
-        } else if ((rb = wider(kNarrow)) > ra) {
+        } else if ((rb = wider(heavy ? kHeavyWidth : kNarrow)) > ra) {
             e = launch_runs<512, M>(g, r0, ra, rb, R, ldr, cend, 3, true, sms, st);
         } else {
             rb = rows;
-            e = launch_runs<NT, M>(g, r0, ra, rb, R, ldr, cend, 8, false, sms, st);
+            e = heavy ? launch_runs<256, M>(g, r0, ra, rb, R, ldr, cend, 6, false, sms, st)
+                      : launch_runs<NT, M>(g, r0, ra, rb, R, ldr, cend, 8, false, sms, st);
         }
         ra = rb;
     }

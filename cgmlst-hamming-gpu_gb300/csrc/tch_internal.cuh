@@ -259,6 +259,7 @@ struct RareGroups {
     const uint16_t* members16 = nullptr;  // the same in two bytes (sets with row runs and n <= 65 536; members null)
     const uint32_t* mpos = nullptr;     // n x L: index in members of row i's own entry, kNoGroup outside groups
     int n = 0, L = 0;
+    size_t pairs = 0;                   // rare pairs of the whole set (for the launch shape; 0 = unknown)
     // Row runs (optional; null: found per locus from the arrays above): row i's
     // partners are runs roff[i] .. roff[i + 1] - 1, in locus order; run q starts
     // at member rlo[q] and covers pieces of 16 bytes of the member array (8

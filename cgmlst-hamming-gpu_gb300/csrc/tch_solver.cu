@@ -459,6 +459,7 @@ static RareGroups rare_groups(const tch_solver* s) {
     g.rtot = s->grtot;
     g.n = s->n;
     g.L = s->gL;
+    g.pairs = s->n_rare;
     return g;
 }
 

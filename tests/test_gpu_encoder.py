@@ -227,3 +227,24 @@ def test_tables_around_group_sizes(pkg, tau):
         H, _ = s.run(200)
     iu = np.triu_indices(n, 1)
     np.testing.assert_array_equal(H[iu], want[iu])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [9000, 21000])
+def test_rows_of_many_rare_pairs(pkg, n):
+    """Sets above and below the pairs per row at which the launch shape changes,
+    with rows on both sides of its widths: sampled rows against the count."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(n)
+    for L in (6, 40):
+        A = rng.integers(1, 7, size=(n, L)).astype(np.uint64)  # n / 6 rows per allele, all rare at tau 65536
+        with pkg.Solver.from_calls(A, tau=65536) as s:
+            assert (s.info()["n_rare"] > 32768 * n) == (n * L / 12 > 32768)
+            ldo = (n + 7) // 8 * 8
+            d = torch.zeros((n, ldo), dtype=torch.int16, device="cuda:0")
+            s.stripe(0, n, d.data_ptr(), ldo, torch.cuda.current_stream().cuda_stream)
+            s.check()
+            for i in (0, 1, 519, n - 20480 - 1, n - 20480, n - 8193, n - 8192, n - 300, n - 2):
+                if 0 <= i < n:
+                    want = (A[i + 1:] != A[i]).sum(1)
+                    np.testing.assert_array_equal(d[i, i + 1:n].cpu().numpy(), want)
