@@ -14,8 +14,8 @@
 //              B-side copy (one-hot columns negated)
 //   rare       u16 counts of rare equal alleles against every database row
 //   distances  the tcgen05 tile pass over the m x n rectangle, subtracting them;
-//              for a few profiles the database's bit columns instead, added up
-//              row by row (query_bits_kernel)
+//              for a few profiles ranks, rare counts and distances come out of
+//              one kernel, from the database's bit columns (query_few_kernel)
 //   q x q      the batch's own upper triangle by a direct count on the calls
 //              (ids compared as given; 0 = missing)
 // Every distance is exact; the database's tau only decides which alleles go
@@ -36,18 +36,22 @@
 #include <map>
 #include <mutex>
 #include <thread>
+#include <type_traits>
 #include <vector>
 
+#include <cooperative_groups.h>
+
+#include "rare_walk.cuh"
 #include "tch_internal.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace tch {
 namespace {
 
-// xq = the ids' ranks; sel (optional) = the bit column of every cell's allele
-// (DeviceEncoding::bits, `D` frequent ones first), ~0 for a missing call.
+// xq = the ids' ranks.
 __global__ void query_rank_kernel(const uint64_t* __restrict__ q, int m, int L, const uint64_t* __restrict__ cnt_off,
-                                  const uint64_t* __restrict__ slot_ids, uint32_t* xq, uint32_t* sel,
-                                  const int32_t* __restrict__ col, const uint32_t* __restrict__ base, uint32_t D) {
+                                  const uint64_t* __restrict__ slot_ids, uint32_t* xq) {
     const size_t total = (size_t)m * L;
     for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
         const int k = (int)(t % L);
@@ -63,63 +67,139 @@ __global__ void query_rank_kernel(const uint64_t* __restrict__ q, int m, int L, 
             r = (lo < cnt_off[k + 1] && slot_ids[lo] == v) ? (uint32_t)(lo - cnt_off[k]) : kNovelRank;
         }
         xq[t] = r;
-        if (sel) {
-            const int32_t c = r && r != kNovelRank ? col[cnt_off[k] + r] : -1;
-            sel[t] = !r ? ~0u : c >= 0 ? base[k] + (uint32_t)c : D + (uint32_t)k;
-        }
     }
 }
 
-// Distances of one new profile (blockIdx.y) to 1 024 rows of the database from
-// its bit columns: a row differs at the loci whose column (the one that sel
-// names) has its bit, less those where the two share a rare allele (R).  Each
-// warp adds up a share of the loci, lane = 32 rows, bit by bit: eight columns go
-// through carry-save adders into binary counters held as planes of bits, which
-// are spread into row counts once at the end.
+// Distances of one new profile (blockIdx.y) to every row of the database, straight
+// from its ids: a row differs at the loci whose bit column (that of the profile's
+// allele, DeviceEncoding::bits) has its bit, less those where the two share a rare
+// allele.  A cluster of eight CTAs takes one window of kQueryWindow rows:
+//   ranks    each CTA looks up an eighth of the ids, four lanes to an id, every
+//            step leaving a fifth of the locus's ids, and hands the columns to
+//            the other seven;
+//   rare     it counts the rare partners that its eighth of the loci has in the
+//            window, 16 bytes of members per lane;
+//   bits     it adds up all loci's columns for its own 2 048 rows: a warp takes
+//            1 024 of them (lane = 32 rows) and a sixteenth of the loci, eight
+//            columns at a time through carry-save adders into binary counters
+//            held as planes of bits, spread into row counts at the end;
+//   out      it adds the eight CTAs' rare counts of its rows and writes.
+// Loci go by in chunks of FEW_LOCI.
 //
-// Bound by the columns' read, n / 8 bytes per locus (28 MB for 200 000 x 1 142,
-// mostly from L2 when queries carry common alleles), where the tile pass reads
-// every row's whole operand (1.07 GB): a query of one profile takes 92 us, with
-// the tile pass 253.
-constexpr int QB_T = 512, QB_PLANES = 13;  // 16 warps: at most 4 096 loci each
+// Bound by chains of dependent loads at one profile (ids, window entries, members,
+// columns: each a trip to memory), at several by the columns' read, n / 8 bytes
+// per locus.  One profile against 200 000 x 1 142: 28 us with cold caches, the
+// whole call 44; three kernels (ranks; rare counts, a CTA per window; columns), one
+// after the other with their results in memory, took 60, the call 91.
+constexpr int FEW_T = 1024, FEW_CTAS = 8, FEW_ROWS = kQueryWindow / FEW_CTAS, FEW_LOCI = 2048;
+constexpr int FEW_PLANES = 13;                       // a warp counts at most 4 096 of 65 535 loci
+constexpr int FEW_RUNS = FEW_LOCI / FEW_CTAS / 32;   // loci a warp looks up in a chunk: 8
+static_assert(FEW_ROWS == 2 * 1024 && FEW_RUNS * 4 == 32, "two warps' rows and four lanes per locus");
+struct FewShared {
+    uint4 counters[kQueryWindow / 8];  // rare partners, u16 pairs
+    uint32_t count[2][32 * 33];        // row (i & 31) * 33 + (i >> 5) of each half
+    uint32_t sel[FEW_LOCI];            // bit column per locus, ~0 for a missing call
+    uint2 runs[FEW_T / 32][FEW_RUNS + 1];
+};
 __device__ __forceinline__ uint32_t carry_add(uint32_t& a, uint32_t b, uint32_t c) {
     const uint32_t carry = (a & b) | (a & c) | (b & c);
     a = a ^ b ^ c;
     return carry;
 }
-__global__ void __launch_bounds__(QB_T)
-    query_bits_kernel(const uint32_t* __restrict__ bits, size_t words, const uint32_t* __restrict__ sel, int n, int L,
-                      const uint16_t* __restrict__ R, size_t ldr, uint16_t* __restrict__ out, size_t ldo) {
-    __shared__ uint32_t count[32 * 33];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, r = blockIdx.y;
-    for (int t = tid; t < 32 * 33; t += QB_T) count[t] = 0;
-    __syncthreads();
-    const uint32_t* mine = bits + (size_t)blockIdx.x * 32 + lane;
-    const int per = (L + QB_T / 32 - 1) / (QB_T / 32);
-    const int k0 = min(L, warp * per), k1 = min(L, k0 + per);
-    uint32_t p[QB_PLANES];
+__global__ void __cluster_dims__(FEW_CTAS, 1, 1) __launch_bounds__(FEW_T)
+    query_few_kernel(const uint64_t* __restrict__ q, const RareGroups g, const uint64_t* __restrict__ slot_ids,
+                     const int32_t* __restrict__ col, const uint32_t* __restrict__ base, uint32_t D,
+                     const uint32_t* __restrict__ bits, size_t words, uint16_t* __restrict__ out, size_t ldo) {
+    extern __shared__ uint4 few_smem[];
+    FewShared& sm = *reinterpret_cast<FewShared*>(few_smem);
+    cg::cluster_group cluster = cg::this_cluster();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, L = g.L;
+    const int rank = (int)cluster.block_rank(), window = blockIdx.x / FEW_CTAS, r = blockIdx.y;
+    for (int t = tid; t < kQueryWindow / 8; t += FEW_T) sm.counters[t] = make_uint4(0, 0, 0, 0);
+    for (int t = tid; t < 2 * 32 * 33; t += FEW_T) (&sm.count[0][0])[t] = 0;
+    const Counters counters = window_counters(sm.counters);
+    const int half = warp >> 4, share = warp & 15;
+    const size_t word = (size_t)window * (kQueryWindow / 32) + rank * (FEW_ROWS / 32) + half * 32 + lane;
+    uint32_t p[FEW_PLANES];
 #pragma unroll
-    for (int b = 0; b < QB_PLANES; b++) p[b] = 0;
-    for (int k = k0; k < k1; k += 32) {
-        const uint32_t s = k + lane < k1 ? __ldg(sel + (size_t)r * L + k + lane) : ~0u;
-#pragma unroll
-        for (int g = 0; g < 32; g += 8) {
-            uint32_t x[8];
-#pragma unroll
-            for (int e = 0; e < 8; e++) {
-                const uint32_t c = __shfl_sync(0xFFFFFFFFu, s, g + e);
-                x[e] = c != ~0u ? __ldg(mine + (size_t)c * words) : 0u;
+    for (int b = 0; b < FEW_PLANES; b++) p[b] = 0;
+    for (int c0 = 0; c0 < L; c0 += FEW_LOCI) {
+        const int nl = min(FEW_LOCI, L - c0), per = (nl + FEW_CTAS - 1) / FEW_CTAS;
+        // the cluster's CTAs run and are done with the last chunk's columns
+        cluster.sync();
+        {
+            const int at = (tid >> 2) + rank * per, k = c0 + at, s = lane & 3;
+            const bool mine = (tid >> 2) < per && at < nl;
+            const uint64_t v = mine ? __ldg(q + (size_t)r * L + k) : 0;
+            uint64_t first = 0, lo = 0, hi = 0;
+            if (v) {  // ids of locus k ascend at slots cnt_off[k] + 1 .. cnt_off[k + 1] - 1
+                first = __ldg(g.cnt_off + k);
+                lo = first + 1;
+                hi = __ldg(g.cnt_off + k + 1);
             }
-            const uint32_t a0 = carry_add(p[0], x[0], x[1]), a1 = carry_add(p[0], x[2], x[3]);
-            const uint32_t b0 = carry_add(p[1], a0, a1);
-            const uint32_t a2 = carry_add(p[0], x[4], x[5]), a3 = carry_add(p[0], x[6], x[7]);
-            const uint32_t b1 = carry_add(p[1], a2, a3);
-            uint32_t c = carry_add(p[2], b0, b1);
+            const uint64_t end = hi;
+            while (__any_sync(0xFFFFFFFFu, lo < hi)) {
+                const uint64_t len = hi - lo;
+                const bool less = lo < hi && __ldg(slot_ids + lo + len * (s + 1) / 5) < v;
+                const int below = __popc(__ballot_sync(0xFFFFFFFFu, less) >> (lane & ~3) & 15u);
+                if (lo < hi) {
+                    if (below < 4) hi = lo + len * (below + 1) / 5;
+                    if (below) lo = lo + len * below / 5 + 1;
+                }
+            }
+            const bool known = v && lo < end && __ldg(slot_ids + lo) == v;
+            uint32_t e = 0;
+            if (known) {  // empty for an allele that is frequent in the set
+                if (s < 2) e = __ldg(g.wpos + lo * (uint64_t)g.windows + window + s);
+            }
+            if (mine) {
+                const int32_t c = known ? __ldg(col + lo) : -1;
+                const uint32_t m = !v ? ~0u : c >= 0 ? __ldg(base + k) + (uint32_t)c : D + (uint32_t)k;
+                cluster.map_shared_rank(sm.sel, 2 * s)[at] = m;
+                cluster.map_shared_rank(sm.sel, 2 * s + 1)[at] = m;
+            }
+            cluster.barrier_arrive();
+            // the warp's runs, end to end (lanes 4 q hold run q)
+            const uint32_t last = __shfl_sync(0xFFFFFFFFu, e, lane | 1);
+            const uint32_t pieces = s == 0 && last > e ? (last - 1) / 8 - e / 8 + 1 : 0;
+            uint32_t inc = pieces;
 #pragma unroll
-            for (int b = 3; b < QB_PLANES; b++) {
-                const uint32_t t = p[b] & c;
-                p[b] ^= c;
-                c = t;
+            for (int d = 4; d < 32; d <<= 1) {
+                const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, inc, d);
+                if (lane >= d) inc += t;
+            }
+            const uint32_t total = __shfl_sync(0xFFFFFFFFu, inc, 28);
+            const unsigned has = __ballot_sync(0xFFFFFFFFu, pieces > 0);
+            uint2* run = sm.runs[warp];
+            if (pieces) run[__popc(has & ((1u << lane) - 1u))] = make_uint2((inc - pieces) << 3 | ((last - 1) & 7u), e);
+            if (lane == 0) run[__popc(has)] = make_uint2(total << 3, 0);
+            __syncwarp();
+            walk_pieces<uint16_t>(counters, run, __popc(has), 0, total, g.members16, lane);
+            __syncwarp();
+            cluster.barrier_wait();
+        }
+        if (word < words) {
+            const uint32_t* mine = bits + word;
+            const int part = ((nl + 15) / 16 + 7) & ~7, k1 = min(nl, (share + 1) * part);
+#pragma unroll 2
+            for (int k = share * part; k < k1; k += 8) {
+                uint32_t x[8];
+#pragma unroll
+                for (int e = 0; e < 8; e++) {
+                    const uint32_t c = k + e < k1 ? sm.sel[k + e] : ~0u;
+                    x[e] = c != ~0u ? __ldg(mine + (size_t)c * words) : 0u;
+                }
+                const uint32_t a0 = carry_add(p[0], x[0], x[1]), a1 = carry_add(p[0], x[2], x[3]);
+                const uint32_t b0 = carry_add(p[1], a0, a1);
+                const uint32_t a2 = carry_add(p[0], x[4], x[5]), a3 = carry_add(p[0], x[6], x[7]);
+                const uint32_t b1 = carry_add(p[1], a2, a3);
+                uint32_t c = carry_add(p[2], b0, b1);
+#pragma unroll
+                for (int b = 3; b < FEW_PLANES; b++) {
+                    const uint32_t t = p[b] & c;
+                    p[b] ^= c;
+                    c = t;
+                }
             }
         }
     }
@@ -127,15 +207,21 @@ __global__ void __launch_bounds__(QB_T)
     for (int i = 0; i < 32; i++) {
         uint32_t v = 0;
 #pragma unroll
-        for (int b = 0; b < QB_PLANES; b++) v |= ((p[b] >> i) & 1u) << b;
-        if (v) atomicAdd(count + i * 33 + lane, v);
+        for (int b = 0; b < FEW_PLANES; b++) v |= ((p[b] >> i) & 1u) << b;
+        if (v) atomicAdd(&sm.count[half][i * 33 + lane], v);
     }
-    __syncthreads();
-    for (int t = tid; t < 1024; t += QB_T) {
-        const int j = blockIdx.x * 1024 + t;
-        if (j < n)
-            out[(size_t)r * ldo + j] = (uint16_t)(count[(t & 31) * 33 + (t >> 5)] - R[(size_t)r * ldr + j]);
+    cluster.sync();
+    {
+        uint32_t rare = 0;  // rows 2 tid and 2 tid + 1 of this CTA's; neither half reaches 65 536
+#pragma unroll
+        for (int c = 0; c < FEW_CTAS; c++)
+            rare += reinterpret_cast<const uint32_t*>(cluster.map_shared_rank(sm.counters, c))[rank * (FEW_ROWS / 2) + tid];
+        const int i = 2 * tid & 1023, j = window * kQueryWindow + rank * FEW_ROWS + 2 * tid;
+        const uint32_t* count = sm.count[tid >> 9] + (i >> 5);
+        const uint32_t d0 = count[(i & 31) * 33] - (rare & 0xFFFFu), d1 = count[((i & 31) + 1) * 33] - (rare >> 16);
+        if (j < g.n) *reinterpret_cast<uint32_t*>(out + (size_t)r * ldo + j) = (d0 & 0xFFFFu) | d1 << 16;
     }
+    cluster.sync();  // no CTA leaves while others read its counters
 }
 
 // +1.0 at column col of row `row` (zeroed before); two columns of one byte
@@ -160,31 +246,76 @@ __global__ void query_pack_kernel(const uint32_t* __restrict__ xq, int m, int L,
     }
 }
 
-// Direct count of the batch's own pairs: 16 x 16 pairs per block, the calls of
-// the two row groups staged in shared memory 64 loci at a time.
-constexpr int QQ_T = 16, QQ_K = 64;
-__global__ void qq_kernel(const uint64_t* __restrict__ q, int m, int L, uint16_t* out, size_t ldo) {
-    const int a0 = blockIdx.y * QQ_T, b0 = blockIdx.x * QQ_T;
-    if (b0 + QQ_T - 1 < a0) return;  // entirely below the diagonal
-    __shared__ uint64_t A[QQ_T][QQ_K + 1], B[QQ_T][QQ_K + 1];
-    const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * QQ_T + tx;
-    uint32_t d = 0;
-    for (int k0 = 0; k0 < L; k0 += QQ_K) {
-        const int kn = min(QQ_K, L - k0);
-        for (int e = tid; e < QQ_T * QQ_K; e += QQ_T * QQ_T) {
-            const int r = e / QQ_K, k = e % QQ_K;
-            A[r][k] = (a0 + r < m && k < kn) ? q[(size_t)(a0 + r) * L + k0 + k] : 0;
-            B[r][k] = (b0 + r < m && k < kn) ? q[(size_t)(b0 + r) * L + k0 + k] : 0;
+// Direct count of the batch's own pairs (ids compared as given): a cluster of
+// eight CTAs per 32 x 32 pairs, each with an eighth of the loci, 64 of them staged
+// in shared memory at a time, 2 x 2 pairs per thread.  Two profiles differ at the
+// loci where the presence of a call agrees less those where the ids (or the two
+// missing calls) are equal: the first by the rows' bit masks, taken as the ids are
+// staged, so a pair and locus costs one 64-bit compare.
+//
+// Bound by the compares for large batches and by the chain of load, barrier and
+// count for small ones, which the split of the loci shortens.  40 / 200 / 1 000
+// profiles of 1 142 loci: 15 / 23 / 179 us; 16 x 16 pairs per CTA, all loci in one
+// CTA and one pair per thread took 60 / 61 / 285.
+constexpr int QQ_T = 32, QQ_K = 64, QQ_CTAS = 8;
+__global__ void __cluster_dims__(QQ_CTAS, 1, 1) __launch_bounds__(256)
+    qq_kernel(const uint64_t* __restrict__ q, int m, int L, uint16_t* out, size_t ldo) {
+    const int a0 = blockIdx.y * QQ_T, b0 = blockIdx.x / QQ_CTAS * QQ_T;
+    if (b0 < a0) return;  // below the diagonal, the whole cluster
+    __shared__ uint64_t ids[2 * QQ_T][QQ_K + 1];  // rows of the two groups
+    __shared__ uint32_t present[2 * QQ_T][QQ_K / 32];
+    __shared__ uint32_t part[QQ_T * QQ_T];
+    cg::cluster_group cluster = cg::this_cluster();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tx = tid & 15, ty = tid >> 4;
+    const int rank = (int)cluster.block_rank(), per = (L + QQ_CTAS - 1) / QQ_CTAS;
+    const int k1 = min(L, (rank + 1) * per);
+    uint32_t d[2][2] = {};
+    for (int k0 = rank * per; k0 < k1; k0 += QQ_K) {
+#pragma unroll
+        for (int e = 0; e < 2 * QQ_T / 8; e++) {
+            const int t = warp + 8 * e, row = t < QQ_T ? a0 + t : b0 + t - QQ_T;
+#pragma unroll
+            for (int w = 0; w < QQ_K / 32; w++) {
+                const int k = k0 + 32 * w + lane;
+                const uint64_t v = row < m && k < k1 ? __ldg(q + (size_t)row * L + k) : 0;
+                ids[t][32 * w + lane] = v;
+                const uint32_t mask = __ballot_sync(0xFFFFFFFFu, v != 0);
+                if (lane == 0) present[t][w] = mask;
+            }
         }
         __syncthreads();
-        for (int k = 0; k < kn; k++) {
-            const uint64_t x = A[ty][k], y = B[tx][k];
-            d += (x != 0) & (y != 0) & (x != y);
+#pragma unroll
+        for (int u = 0; u < 2; u++)
+#pragma unroll
+            for (int v = 0; v < 2; v++)
+#pragma unroll
+                for (int w = 0; w < QQ_K / 32; w++)
+                    d[u][v] += __popc(~(present[ty + 16 * u][w] ^ present[QQ_T + tx + 16 * v][w]));
+#pragma unroll 8
+        for (int k = 0; k < QQ_K; k++) {
+            const uint64_t x0 = ids[ty][k], x1 = ids[ty + 16][k];
+            const uint64_t y0 = ids[QQ_T + tx][k], y1 = ids[QQ_T + tx + 16][k];
+            d[0][0] -= x0 == y0;
+            d[0][1] -= x0 == y1;
+            d[1][0] -= x1 == y0;
+            d[1][1] -= x1 == y1;
         }
         __syncthreads();
     }
-    const int a = a0 + ty, b = b0 + tx;
-    if (a < m && b < m && b > a) out[(size_t)a * ldo + b] = (uint16_t)d;
+#pragma unroll
+    for (int u = 0; u < 2; u++)
+#pragma unroll
+        for (int v = 0; v < 2; v++) part[(ty + 16 * u) * QQ_T + tx + 16 * v] = d[u][v];
+    cluster.sync();
+    constexpr int SHARE = QQ_T * QQ_T / QQ_CTAS;
+    if (tid < SHARE) {
+        const int t = rank * SHARE + tid, a = a0 + t / QQ_T, b = b0 + t % QQ_T;
+        uint32_t sum = 0;
+#pragma unroll
+        for (int c = 0; c < QQ_CTAS; c++) sum += cluster.map_shared_rank(part, c)[t];
+        if (a < m && b < m && b > a) out[(size_t)a * ldo + b] = (uint16_t)sum;
+    }
+    cluster.sync();  // no CTA leaves while others read its counts
 }
 
 double now_s() {
@@ -250,9 +381,11 @@ void give_lane(tch_db* db, CopyLane* l) {
 }
 
 // Batches of at most this many profiles go by the bit columns, whose read grows
-// with them, larger ones by the tile pass, whose does not up to 256: 1 / 8 / 16
-// profiles take 92 / 213 / 332 us by columns and 253 / 284 / 304 by tiles against
-// 200 000 x 1 142, 103 / 166 / 212 and 236 / 247 / 254 against 50 000 x 3 016.
+// with them, larger ones by the tile pass, whose does not up to 256.  1 / 8 / 12 /
+// 16 profiles, by columns: 44 / 215 / 322 / 404 us against 200 000 x 1 142, 67 /
+// 154 / 207 / 258 against 50 000 x 3 016, 42 / 77 / 77 / 103 against 20 000 x
+// 1 142; by tiles: 231 / 264 / 275 / 285, 188 / 203 / 219 / 222, 80 / 93 / 101 /
+// 102.
 constexpr int kBitProfiles = 8;
 bool by_bits(const tch_db* db, int m) { return m <= kBitProfiles && db->enc.bits; }
 
@@ -277,7 +410,7 @@ int db_query(tch_db* db, int m, const uint64_t* qcalls, uint16_t* h_qdb, uint16_
     const size_t mr = up((size_t)std::max(m, 1), 256);
     const size_t ldr = up((size_t)n, kRareDenseAlign), ldo = up((size_t)n, 8), ldq = up((size_t)m, 8);
     uint64_t* dq = nullptr;
-    uint32_t *xq = nullptr, *sel = nullptr;
+    uint32_t* xq = nullptr;
     uint16_t *R = nullptr, *out = nullptr, *qq = nullptr;
     int* derr = nullptr;
     Fp4Operands QX;  // the batch's A-side rows: the database's K layout, m rows
@@ -303,40 +436,46 @@ int db_query(tch_db* db, int m, const uint64_t* qcalls, uint16_t* h_qdb, uint16_
     auto mark = [&]() {
         if (verbose && nev < 8 && cudaEventCreate(&ev[nev]) == cudaSuccess) cudaEventRecord(ev[nev++], st);
     };
-    auto alloc = [&](void** p, size_t bytes) {
-        if (ce == cudaSuccess) ce = cudaMallocFromPoolAsync(p, std::max<size_t>(bytes, 16), db->pool, st);
-    };
     if (m <= 0) return e.set("empty query batch");
     if (!qcalls) return e.set("null query calls");
     if (cudaSetDevice(db->device) != cudaSuccess) return e.set("cudaSetDevice(%d) failed", db->device);
-    alloc((void**)&dq, (size_t)m * L * 8);
-    alloc((void**)&xq, (size_t)m * L * 4);
-    alloc((void**)&derr, 4);
-    if (h_qdb && bits) alloc((void**)&sel, (size_t)m * L * 4);
-    if (h_qdb && !bits)
-        for (int c = 0; c < X.n; c++) alloc((void**)&X.p[c], mr * (size_t)X.width_of(c));
-    if (h_qdb) {
-        alloc((void**)&R, (size_t)m * ldr * 2);
-        alloc((void**)&out, (size_t)m * ldo * 2);
+    // one allocation for all of it: each costs the call about 2 us
+    char* work = nullptr;
+    size_t bytes = 0, zero_at = 0, zero = 0;
+    auto place = [&](auto** p, size_t want) {  // two passes: sizes, then addresses
+        if (work) *p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>(work + bytes);
+        bytes += up(want, 256);
+    };
+    for (int pass = 0; pass < 2; pass++) {
+        bytes = 0;
+        place(&dq, (size_t)m * L * 8);
+        if (h_qdb) place(&out, (size_t)m * ldo * 2);
+        if (h_qq && m > 1) place(&qq, (size_t)m * ldq * 2);
+        if (h_qdb && !bits) {
+            place(&xq, (size_t)m * L * 4);
+            place(&R, (size_t)m * ldr * 2);
+            zero_at = bytes;  // zeroed: the operand rows and the error word
+            for (int c = 0; c < X.n; c++) place(&X.p[c], mr * (size_t)X.width_of(c));
+            place(&derr, 4);
+            zero = bytes - zero_at;
+        }
+        if (pass == 0) ce = cudaMallocFromPoolAsync((void**)&work, bytes, db->pool, st);
+        if (ce != cudaSuccess) goto done;
     }
-    if (h_qq && m > 1) alloc((void**)&qq, (size_t)m * ldq * 2);
-    if (ce != cudaSuccess) goto done;
     mark();
     ce = cudaMemcpyAsync(dq, qcalls, (size_t)m * L * 8, cudaMemcpyHostToDevice, st);
-    if (ce == cudaSuccess) ce = cudaMemsetAsync(derr, 0, 4, st);
+    if (ce == cudaSuccess && zero) ce = cudaMemsetAsync(work + zero_at, 0, zero, st);
     if (ce != cudaSuccess) goto done;
     {
         const int grid = (int)std::min<size_t>(((size_t)m * L + 255) / 256, (size_t)db->sms * 16);
         if (h_qdb) {
-            for (int c = 0; c < X.n && ce == cudaSuccess && !bits; c++)
-                ce = cudaMemsetAsync(X.p[c], 0, mr * (size_t)X.width_of(c), st);
-            if (ce != cudaSuccess) goto done;
             mark();
-            query_rank_kernel<<<grid, 256, 0, st>>>(dq, m, L, enc.cnt_off, enc.slot_ids, xq, sel, enc.col, enc.base,
-                                                    (uint32_t)enc.D);
-            if (!bits) query_pack_kernel<<<grid, 256, 0, st>>>(xq, m, L, enc.cnt_off, enc.col, enc.base, X);
-            ce = cudaGetLastError();
-            if (ce != cudaSuccess) goto done;
+            if (!bits) {
+                query_rank_kernel<<<grid, 256, 0, st>>>(dq, m, L, enc.cnt_off, enc.slot_ids, xq);
+                query_pack_kernel<<<grid, 256, 0, st>>>(xq, m, L, enc.cnt_off, enc.col, enc.base, X);
+                ce = cudaGetLastError();
+                if (ce != cudaSuccess) goto done;
+            }
             RareGroups g;
             g.cnt_off = enc.cnt_off;
             g.members16 = enc.members16;
@@ -355,14 +494,15 @@ int db_query(tch_db* db, int m, const uint64_t* qcalls, uint16_t* h_qdb, uint16_
             const int step = lane ? block : m;
             for (int r0 = 0, k = 0; r0 < m; r0 += step, k++) {
                 const int rows = std::min(step, m - r0);
-                uint16_t* Rb = R + (size_t)r0 * ldr;
-                ce = launch_rare_query(g, xq + (size_t)r0 * L, rows, Rb, ldr, st);
-                if (ce != cudaSuccess) goto done;
                 if (bits) {
-                    query_bits_kernel<<<dim3((unsigned)(enc.bit_words / 32), rows), QB_T, 0, st>>>(
-                        enc.bits, enc.bit_words, sel + (size_t)r0 * L, n, L, Rb, ldr, out + (size_t)r0 * ldo, ldo);
+                    query_few_kernel<<<dim3((unsigned)(g.windows * FEW_CTAS), rows), FEW_T, sizeof(FewShared), st>>>(
+                        dq + (size_t)r0 * L, g, enc.slot_ids, enc.col, enc.base, (uint32_t)enc.D, enc.bits,
+                        enc.bit_words, out + (size_t)r0 * ldo, ldo);
                     ce = cudaGetLastError();
                 } else {
+                    uint16_t* Rb = R + (size_t)r0 * ldr;
+                    ce = launch_rare_query(g, xq + (size_t)r0 * L, rows, Rb, ldr, st);
+                    if (ce != cudaSuccess) goto done;
                     a.r0 = r0;
                     a.rows = rows;
                     a.out = out + (size_t)r0 * ldo;
@@ -375,8 +515,8 @@ int db_query(tch_db* db, int m, const uint64_t* qcalls, uint16_t* h_qdb, uint16_
         }
         if (qq) {
             mark();
-            const dim3 blk(QQ_T, QQ_T), grd((m + QQ_T - 1) / QQ_T, (m + QQ_T - 1) / QQ_T);
-            qq_kernel<<<grd, blk, 0, st>>>(dq, m, L, qq, ldq);
+            const unsigned tiles = (unsigned)((m + QQ_T - 1) / QQ_T);
+            qq_kernel<<<dim3(tiles * QQ_CTAS, tiles), 256, 0, st>>>(dq, m, L, qq, ldq);
             ce = cudaGetLastError();
             if (ce == cudaSuccess && lane) ce = cudaEventRecord(lane->ev[kCopyBlocks], st);
             if (ce != cudaSuccess) goto done;
@@ -411,10 +551,7 @@ done:
             if (ce == cudaSuccess) ce = le;
         }
         if (derr && ce == cudaSuccess) ce = cudaMemcpyAsync(&herr, derr, 4, cudaMemcpyDeviceToHost, st);
-        for (void* p : {(void*)dq, (void*)xq, (void*)sel, (void*)R, (void*)out, (void*)qq, (void*)derr})
-            if (p) cudaFreeAsync(p, st);
-        for (int c = 0; c < X.n; c++)
-            if (X.p[c]) cudaFreeAsync(X.p[c], st);
+        if (work) cudaFreeAsync(work, st);
         mark();
         const cudaError_t se = cudaStreamSynchronize(st);
         if (ce == cudaSuccess) ce = se;
@@ -532,6 +669,8 @@ int tch_db_create(int device, int n, int L, const uint64_t* calls, int tau, tch_
         TCH_CK(e, cudaDeviceGetAttribute(&db->sms, cudaDevAttrMultiProcessorCount, device));
         TCH_CK(e, cudaMemPoolCreate(&db->pool, &props));
         TCH_CK(e, cudaMemPoolSetAttribute(db->pool, cudaMemPoolAttrReleaseThreshold, &keep));
+        TCH_CK(e, cudaFuncSetAttribute(query_few_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)sizeof(FewShared)));
     }
     TCH_CK(e, cudaMalloc(&d_calls, (size_t)n * L * 8));
     TCH_CK(e, cudaMemcpy(d_calls, calls, (size_t)n * L * 8, cudaMemcpyHostToDevice));

@@ -218,3 +218,41 @@ def test_results_copied_in_blocks(pkg, n, m, pinned):
         for t in threads:
             t.join()
         assert not errors, errors[0]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,L", [(2048, 2047), (2049, 2048), (2047, 2049), (16385, 40), (40961, 9), (700, 4100), (3, 1)])
+@pytest.mark.parametrize("m", [1, 3, 8])
+def test_few_profiles_at_the_clusters_edges(pkg, n, L, m):
+    """Row counts around a CTA's 2 048 and a cluster's 16 384 rows, locus counts
+    around a chunk's 2 048: rare, frequent, new and missing ids in every profile,
+    id lists of any length (none, one, thousands)."""
+    rng = np.random.default_rng(n * 3 + L + m)
+    high = rng.choice([1, 2, 6, 40, 3000], size=L)
+    A = rng.integers(0, high[None, :], size=(n, L)).astype(np.uint64) * 3
+    Q = rng.integers(0, 3 * high[None, :] + 2, size=(m, L)).astype(np.uint64)
+    Q[::2] = np.where(rng.random((len(Q[::2]), L)) < 0.6, A[rng.integers(0, n, size=len(Q[::2]))], Q[::2])
+    want = np.zeros((m, n), np.uint16)
+    for k in range(L):
+        want += (Q[:, k, None] != A[None, :, k]) & (Q[:, k, None] != 0) & (A[None, :, k] != 0)
+    with pkg.Database(A, tau=max(2, n // 9)) as db:
+        np.testing.assert_array_equal(db.query(Q)[0], want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m", [2, 31, 32, 33, 65, 200])
+@pytest.mark.parametrize("L", [1, 7, 8, 64, 513, 1030])
+def test_batch_pairs_at_tile_edges(pkg, m, L):
+    """The batch's own pairs around the tiles of 32 x 32 and the loci's eighths
+    and chunks of 64: ids that differ in one half only, missing calls."""
+    rng = np.random.default_rng(m * 11 + L)
+    low, top = (rng.integers(0, 3, size=(m, L), dtype=np.uint64) for _ in range(2))
+    Q = low | top << np.uint64(32)
+    A = Q[: max(1, m // 2)]
+    want = np.zeros((m, m), np.uint16)
+    for k in range(L):
+        want += (Q[:, k, None] != Q[None, :, k]) & (Q[:, k, None] != 0) & (Q[None, :, k] != 0)
+    with pkg.Database(A) as db:
+        got, qq = db.query(Q)
+    np.testing.assert_array_equal(np.triu(qq, 1), np.triu(want, 1))
+    np.testing.assert_array_equal(got, want[:, : len(A)])
