@@ -248,3 +248,28 @@ def test_rows_of_many_rare_pairs(pkg, n):
                 if 0 <= i < n:
                     want = (A[i + 1:] != A[i]).sum(1)
                     np.testing.assert_array_equal(d[i, i + 1:n].cpu().numpy(), want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [129, 4096, 8193, 131072, 131073, 270000])
+def test_rows_sorted_by_bit_maps(pkg, n):
+    """Groups of more rows than a warp sorts, over row counts around the words, the
+    threads' shares and the windows (131 072 rows) of the bit maps: new profiles'
+    distances read every group in its order."""
+    rng = np.random.default_rng(n)
+    L, m = 6, 9
+    top = np.array([1, 2, 3, max(1, n // 300), max(1, n // 129), min(n, 65535)])
+    A = rng.integers(1, top[None, :] + 1, size=(n, L)).astype(np.uint64)
+    Q = A[rng.integers(0, n, size=m)]
+    want = np.zeros((m, n), np.uint16)
+    for k in range(L):
+        want += Q[:, k, None] != A[None, :, k]
+    with pkg.Database(A, tau=n + 1) as db:
+        np.testing.assert_array_equal(db.query(Q)[0], want)
+        np.testing.assert_array_equal(db.query(Q[:1])[0], want[:1])
+    if n <= 8193:
+        with pkg.Solver.from_calls(A, tau=n + 1) as s:
+            H, _ = s.run(n)
+        full = (A[:, None, :] != A[None, : min(n, 600), :]).sum(2).T
+        iu = np.triu_indices(min(n, 600), 1, n)
+        np.testing.assert_array_equal(H[: min(n, 600)][iu], full[iu])
