@@ -49,27 +49,6 @@ namespace cg = cooperative_groups;
 namespace tch {
 namespace {
 
-// xq = the ids' ranks.
-__global__ void query_rank_kernel(const uint64_t* __restrict__ q, int m, int L, const uint64_t* __restrict__ cnt_off,
-                                  const uint64_t* __restrict__ slot_ids, uint32_t* xq) {
-    const size_t total = (size_t)m * L;
-    for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
-        const int k = (int)(t % L);
-        const uint64_t v = q[t];
-        uint32_t r = 0;
-        if (v) {
-            // ids of locus k ascend at slots cnt_off[k] + 1 .. cnt_off[k + 1] - 1
-            uint64_t lo = cnt_off[k] + 1, hi = cnt_off[k + 1];
-            while (lo < hi) {
-                const uint64_t mid = lo + (hi - lo) / 2;
-                if (slot_ids[mid] < v) lo = mid + 1; else hi = mid;
-            }
-            r = (lo < cnt_off[k + 1] && slot_ids[lo] == v) ? (uint32_t)(lo - cnt_off[k]) : kNovelRank;
-        }
-        xq[t] = r;
-    }
-}
-
 // Distances of one new profile (blockIdx.y) to every row of the database, straight
 // from its ids: a row differs at the loci whose bit column (that of the profile's
 // allele, DeviceEncoding::bits) has its bit, less those where the two share a rare
@@ -231,18 +210,33 @@ __device__ __forceinline__ void set_fp4_one(const KChunks& X, size_t row, size_t
     atomicOr(w, kFp4One << (4 * (col & 7)));
 }
 
-__global__ void query_pack_kernel(const uint32_t* __restrict__ xq, int m, int L, const uint64_t* __restrict__ cnt_off,
-                                  const int32_t* __restrict__ col, const uint32_t* __restrict__ base, KChunks X) {
+// The batch's ranks and operand rows (zeroed before).
+__global__ void query_pack_kernel(const uint64_t* __restrict__ q, int m, int L, const uint64_t* __restrict__ cnt_off,
+                                  const uint64_t* __restrict__ slot_ids, const int32_t* __restrict__ col,
+                                  const uint32_t* __restrict__ base, uint32_t* xq, KChunks X) {
     const size_t total = (size_t)m * L;
     for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
-        const uint32_t a = xq[t];
-        if (!a) continue;
         const size_t i = t / L;
         const int k = (int)(t % L);
-        set_fp4_one(X, i, (size_t)k);
-        if (a == kNovelRank) continue;
-        const int32_t c = col[cnt_off[k] + a];
-        if (c >= 0) set_fp4_one(X, i, (size_t)L + base[k] + (size_t)c);
+        const uint64_t v = q[t];
+        uint32_t r = 0;
+        if (v) {
+            set_fp4_one(X, i, (size_t)k);
+            // ids of locus k ascend at slots cnt_off[k] + 1 .. cnt_off[k + 1] - 1
+            const uint64_t first = cnt_off[k], end = cnt_off[k + 1];
+            uint64_t lo = first + 1, hi = end;
+            while (lo < hi) {
+                const uint64_t mid = lo + (hi - lo) / 2;
+                if (slot_ids[mid] < v) lo = mid + 1; else hi = mid;
+            }
+            r = kNovelRank;
+            if (lo < end && slot_ids[lo] == v) {
+                r = (uint32_t)(lo - first);
+                const int32_t c = col[lo];
+                if (c >= 0) set_fp4_one(X, i, (size_t)L + base[k] + (size_t)c);
+            }
+        }
+        xq[t] = r;
     }
 }
 
@@ -471,8 +465,7 @@ int db_query(tch_db* db, int m, const uint64_t* qcalls, uint16_t* h_qdb, uint16_
         if (h_qdb) {
             mark();
             if (!bits) {
-                query_rank_kernel<<<grid, 256, 0, st>>>(dq, m, L, enc.cnt_off, enc.slot_ids, xq);
-                query_pack_kernel<<<grid, 256, 0, st>>>(xq, m, L, enc.cnt_off, enc.col, enc.base, X);
+                query_pack_kernel<<<grid, 256, 0, st>>>(dq, m, L, enc.cnt_off, enc.slot_ids, enc.col, enc.base, xq, X);
                 ce = cudaGetLastError();
                 if (ce != cudaSuccess) goto done;
             }
