@@ -223,9 +223,10 @@ struct TcBatchItem {
 struct TcBatchPlan {
     void* d_jobs = nullptr;
     void* d_maps = nullptr;
-    void* d_tile_job = nullptr;  // the job of every tile
+    void* d_tiles = nullptr;  // (job, tile), by CTA pair
+    void* d_first = nullptr;  // every pair's first tile
     int njobs = 0, num_tiles = 0;
-    int grid = 0;  // CTAs of the launch (at most num_sms), each on every grid-th tile
+    int grid = 0;  // CTAs of the launch (at most num_sms)
     int* err = nullptr;
 };
 cudaError_t tc_batch_prepare(const std::vector<TcBatchItem>& items, int num_sms, TcBatchPlan* plan, int* err);

@@ -142,3 +142,20 @@ def test_batch_persistent_wide_sets(tch):
         b.run(out.data_ptr(), stream)
         b.check()
         check_all(sets, out.cpu().numpy().view(np.uint16), off, ld)
+
+
+@pytest.mark.parametrize("shapes", [[(2, 1)], [(300, 40), (2, 2600), (241, 7)], [(1500, 30), (257, 900), (1, 5), (900, 200)],
+                                    [(5, 9)] * 160 + [(700, 1200)]])
+def test_batch_tiles_spread_over_pairs(tch, shapes):
+    """Batches of one tile, of fewer tiles than CTA pairs, and of sets whose tiles
+    differ widely in K stages, so that the pairs' lists differ in length."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(len(shapes))
+    sets = [rng.integers(0, 9, size=s).astype(np.uint64) for s in shapes]
+    with tch.Batch(sets, taus=[4] * len(sets)) as b:
+        off, ld = b.layout()
+        out = torch.zeros(int(off[-1]) + 8, dtype=torch.int16, device="cuda")
+        b.set_schedule(0)
+        b.run(out.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        b.check()
+        check_all(sets, out.cpu().numpy().view(np.uint16), off, ld)
