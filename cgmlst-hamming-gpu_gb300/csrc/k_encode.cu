@@ -552,7 +552,7 @@ rare_rows_kernel(const uint16_t* __restrict__ x, int n, int L, const uint64_t* _
 // totals, which it adds up.  Reading the counts on the host, building the tables
 // there and copying them back took 1.8 of 5.7 ms for 10 007 x 1 343 profiles.
 
-constexpr int kBins = 32;  // by floor(log2(count))
+constexpr int kBins = 128;  // four to an octave of the count
 struct CountBins {
     unsigned long long n[kBins], sum[kBins], sq[kBins];  // how many, sum, sum of squares
 };
@@ -564,7 +564,8 @@ __global__ void count_bins_kernel(const uint32_t* __restrict__ cnt, uint64_t slo
     for (uint64_t q = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; q < slots; q += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t c = cnt[q];
         if (!c) continue;
-        const int b = 31 - __clz(c);
+        const int lg = 31 - __clz(c);
+        const int b = 4 * lg + (int)(((unsigned long long)c << 2 >> lg) & 3);
         atomicAdd(&mine.n[b], 1ull);
         atomicAdd(&mine.sum[b], (unsigned long long)c);
         atomicAdd(&mine.sq[b], (unsigned long long)c * c);
@@ -729,53 +730,75 @@ struct TauRow {
 
 // Analytic cost of tau on GB300: tensor-core time for the one-hot columns plus
 // the rare term (fused pair-list walk, or the dense rare-count build), subject
-// to device memory.
-std::vector<TauRow> tau_rows(const CountBins& bins, int n, int L, size_t free_bytes, const TauModel& m, bool dense) {
-    // the candidates are powers of two, so an allele is frequent at tau = 2^t
-    // exactly when floor(log2(count)) >= t: every candidate sums whole bins (the
-    // sums are integers far below 2^53, exact in double); a single row is no pair
-    double bn[kBins] = {}, bsq[kBins] = {}, br[kBins] = {}, bcells[kBins] = {};
-    for (int b = 0; b < kBins; b++) {
-        bn[b] = (double)bins.n[b];
-        bsq[b] = (double)bins.sq[b];
-        if (b) {
-            br[b] = (double)((bins.sq[b] - bins.sum[b]) / 2);
-            bcells[b] = (double)bins.sum[b];
-        }
-    }
+// to device memory.  tau is 2^(first / 4) (1 + (first % 4) / 4), a whole number: an
+// allele is frequent exactly when its bin is `first` or a later one, so every
+// candidate sums whole bins (the sums are integers far below 2^53, exact in
+// double); a single row is no pair.
+TauRow tau_row(const CountBins& bins, int first, int n, int L, size_t free_bytes, const TauModel& m, bool dense) {
     const double pairs = (double)n * (double)(n - 1) / 2.0;
     const size_t rows = up((size_t)std::max(n, 1), 256);
     const double nl = (double)n * (double)L;
-    std::vector<TauRow> out;
-    for (int t = 1; (1 << t) <= (dense ? 65536 : 4096); t++) {
-        TauRow w;
-        w.tau = 1 << t;
-        double d = 0;
-        for (int b = 0; b < kBins; b++) {
-            if (b >= t) {
-                d += bn[b];
-            } else {
-                w.sq += bsq[b];
-                w.r += br[b];
-                w.cells += bcells[b];
-            }
-        }
-        w.d = (size_t)d;
-        w.kb = (double)fp4_columns(L, w.d);  // K: MACs per pair; the two operand copies take K bytes per row
-        if (dense) {  // ranks, own positions, group members, row runs (a stripe's counts come later)
-            w.mem = (double)rows * w.kb + nl * 6.0 + 12.0 * w.cells + 12.0 * n;
-            w.t = pairs * w.kb / m.gemm_rate + w.r / m.dense_rate;
-            w.feature_t = pairs * w.kb / m.feature_gemm_rate + w.r / m.feature_dense_rate;
-            w.fits = w.mem <= (double)free_bytes && w.cells < 4.0e9;
+    TauRow w;
+    w.tau = (int)(((long long)(4 + first % 4) << (first / 4)) / 4);
+    double d = 0;
+    for (int b = 0; b < kBins; b++) {
+        if (b >= first) {
+            d += (double)bins.n[b];
         } else {
-            w.mem = (double)rows * w.kb + 4.0 * (w.r + n + 1.0) + 2.0 * (double)n * (double)up((size_t)n, 8) / 4;
-            w.t = pairs * w.kb / m.gemm_rate + w.r / m.rare_rate;
-            w.feature_t = pairs * w.kb / m.feature_gemm_rate + w.r / m.rare_rate;
-            w.fits = w.mem <= (double)free_bytes && w.r < 4.0e9;
+            w.sq += (double)bins.sq[b];
+            if (b < 4) continue;
+            w.r += (double)((bins.sq[b] - bins.sum[b]) / 2);
+            w.cells += (double)bins.sum[b];
         }
-        out.push_back(w);
     }
+    w.d = (size_t)d;
+    w.kb = (double)fp4_columns(L, w.d);  // K: MACs per pair; the two operand copies take K bytes per row
+    if (dense) {  // ranks, own positions, group members, row runs (a stripe's counts come later)
+        w.mem = (double)rows * w.kb + nl * 6.0 + 12.0 * w.cells + 12.0 * n;
+        w.t = pairs * w.kb / m.gemm_rate + w.r / m.dense_rate;
+        w.feature_t = pairs * w.kb / m.feature_gemm_rate + w.r / m.feature_dense_rate;
+        w.fits = w.mem <= (double)free_bytes && w.cells < 4.0e9;
+    } else {
+        w.mem = (double)rows * w.kb + 4.0 * (w.r + n + 1.0) + 2.0 * (double)n * (double)up((size_t)n, 8) / 4;
+        w.t = pairs * w.kb / m.gemm_rate + w.r / m.rare_rate;
+        w.feature_t = pairs * w.kb / m.feature_gemm_rate + w.r / m.rare_rate;
+        w.fits = w.mem <= (double)free_bytes && w.r < 4.0e9;
+    }
+    return w;
+}
+
+// The powers of two.
+std::vector<TauRow> tau_rows(const CountBins& bins, int n, int L, size_t free_bytes, const TauModel& m, bool dense) {
+    std::vector<TauRow> out;
+    for (int t = 1; (1 << t) <= (dense ? 65536 : 4096); t++)
+        out.push_back(tau_row(bins, 4 * t, n, L, free_bytes, m, dense));
     return out;
+}
+
+// The quarters of the octaves on either side of the best power of two, for sets
+// whose estimate is kRefineSeconds or more (below it, launches and latency that
+// the model does not know are more than the difference: 4 000 x 1 142 takes 0.0731
+// ms at 64 and 0.0753 at the model's 96) and falls to kRefineGain of it or less.
+// Whole triangles, the best power of two and the refined tau: 63 005 x 1 142
+// long-tail 8.61 (1 024) and 8.37 ms (1 280), 20 000 x 1 142 1.028 (512) and 0.999
+// (384), 20 000 x 2 794 2.055 and 1.980, 10 007 x 1 343 0.356 and 0.348; clonal
+// sets, whose rare counts are quicker than the model's rate, 20 000 x 1 343 1.149
+// (512) and 1.171 (384), 63 005 x 1 142 8.70 and 8.50.
+constexpr double kRefineSeconds = 1e-4, kRefineGain = 0.985;
+int refine_tau(const std::vector<TauRow>& rows, int best, const CountBins& bins, int n, int L, size_t free_bytes,
+               const TauModel& m) {
+    for (const TauRow& w : rows) {
+        if (w.tau != best || best < 8 || w.t < kRefineSeconds) continue;
+        int t = 0;
+        while (2 << t <= best) t++;
+        double least = kRefineGain * w.t;
+        for (int first = 4 * t - 3; first < 4 * t + 4; first++) {
+            const TauRow q = tau_row(bins, first, n, L, free_bytes, m, true);
+            if (q.fits && q.t < least) best = q.tau, least = q.t;
+        }
+        break;
+    }
+    return best;
 }
 
 int choose_tau_analytic(const std::vector<TauRow>& rows) {
@@ -861,7 +884,8 @@ constexpr int kLearnedMaxRows = 65536;
 int choose_tau_gb300(int device, const CountBins& bins, const std::vector<uint64_t>& off, int n, int L,
                      size_t free_bytes, const TauModel& m, bool dense, bool verbose, int* sub, int* group) {
     const std::vector<TauRow> rows = tau_rows(bins, n, L, free_bytes, m, dense);
-    const int analytic = choose_tau_analytic(rows);
+    int analytic = choose_tau_analytic(rows);
+    if (dense) analytic = refine_tau(rows, analytic, bins, n, L, free_bytes, m);
     int learned = 0, lsub = 0, lgroup = 0;
     std::vector<float> pred;
     TauTable t;

@@ -1,6 +1,8 @@
 """The device encoder (allele calls -> ranks, operands, rare CSR on the GPU)
 against the oracle: every cell of the upper triangle, and the encoder's sizes
 (one-hot columns, rare pairs) against the restated reference host encoder."""
+import importlib
+
 import numpy as np
 import pytest
 
@@ -273,3 +275,33 @@ def test_rows_sorted_by_bit_maps(pkg, n):
         full = (A[:, None, :] != A[None, : min(n, 600), :]).sum(2).T
         iu = np.triu_indices(min(n, 600), 1, n)
         np.testing.assert_array_equal(H[: min(n, 600)][iu], full[iu])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tau", [4, 5, 6, 7, 8, 9, 10, 12, 14, 20, 28, 40])
+def test_counts_around_quarter_octaves(pkg, tau):
+    """The sizes the tau model sums from its bins are those of the encoding: counts
+    on either side of the bins' edges, at taus on and off them."""
+    rng = np.random.default_rng(tau)
+    sizes = [1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16, 19, 20, 23, 24, 27, 28, 31, 32, 39, 40]
+    col = np.concatenate([np.full(s, a + 1) for a, s in enumerate(sizes)])
+    A = np.stack([rng.permutation(col) for _ in range(9)], axis=1).astype(np.uint64)
+    with pkg.Solver.from_calls(A, tau=tau) as s:
+        info = s.info()
+        assert info["d_onehot"] == 9 * sum(c >= tau for c in sizes)
+        assert info["n_rare"] == 9 * sum(c * (c - 1) // 2 for c in sizes if c < tau)
+
+
+@pytest.mark.gpu
+def test_refined_tau_keeps_distances(pkg):
+    """A set large enough for a tau between the powers of two: the distances are
+    those of another tau."""
+    synth = importlib.import_module(pkg.__name__ + ".synth")
+    A = synth.longtail(n=9000, L=1343, seed=3)
+    with pkg.Solver.from_calls(A) as s:
+        H, _ = s.run(4096)
+    with pkg.Solver.from_calls(A, tau=64) as s:
+        assert s.info()["tau"] == 64
+        want, _ = s.run(4096)
+    iu = np.triu_indices(9000, 1)
+    np.testing.assert_array_equal(H[iu], want[iu])
