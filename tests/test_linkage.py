@@ -290,3 +290,20 @@ def test_gpu_mst_exhausted_lists(pkg, n, nested):
     H = (H + H.T).astype(np.uint16)
     d, ld = device_matrix(torch, H)
     same_tree(pkg.mst_device(d.data_ptr(), ld, n), H)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [2, 7, 63, 64, 65, 127, 128, 129, 200, 321])
+def test_mirror_tile_edges(pkg, n):
+    """The full matrix behind the solver's neighbours, around the 64 x 64 tiles of
+    its lower half: every row's nearest columns on either side of the diagonal."""
+    rng = np.random.default_rng(n)
+    A = rng.integers(0, 5, size=(n, 33)).astype(np.uint64)
+    H = oracle.hamming(pkg.dense_ranks(A)[0])
+    H = np.triu(H, 1) + np.triu(H, 1).T
+    k = min(n - 1, 32)
+    with pkg.Solver.from_calls(A) as s:
+        idx, dist = s.neighbors(k)
+    want_i, want_d = oracle.neighbors(H, k)
+    np.testing.assert_array_equal(idx, want_i)
+    np.testing.assert_array_equal(dist, want_d)
