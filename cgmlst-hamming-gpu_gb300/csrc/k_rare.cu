@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(T, T >= 1024 ? 1 : 1536 / T)
 
 // Many sets' whole triangles in one launch (batched solves): the rows of
 // every job laid end to end (row_job: the job of every row), one CTA per row
-// as in rare_dense_kernel, each row counted in one pass (the launcher checks
+// as in rare_runs_kernel, each row counted in one pass (the launcher checks
 // that every job's width fits the counters).
 struct RareJob {
     RareGroups g;

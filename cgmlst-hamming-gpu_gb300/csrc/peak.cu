@@ -321,7 +321,7 @@ int main(int argc, char** argv) {
     // against pairs of -1.0 (0xAA)
     if (!rc && want(argc, argv, "tc_f8")) rc = run_tc<TC_F8>(pr, "tc_f8_tflops", 0x38383838u, 0xB8B8B8B8u, -1.0);
     if (!rc && want(argc, argv, "tc_f4")) rc = run_tc<TC_F4>(pr, "tc_f4_tflops", 0x22222222u, 0xAAAAAAAAu, -1.0);
-    // the tile shape of the contraction kernel (M128 N224); run alone: tch-peak tc_f4_n224
+    // a narrower tile on one CTA (M128 N224); run alone: tch-peak tc_f4_n224
     if (!rc && argc > 1 && want(argc, argv, "tc_f4_n224"))
         rc = run_tc<TC_F4, 224>(pr, "tc_f4_n224_tflops", 0x22222222u, 0xAAAAAAAAu, -1.0);
     // kind::mxf4nvf4 (not in the default set: tch-peak tc_nvf4_32 / tc_nvf4_16)
