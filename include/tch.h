@@ -141,9 +141,10 @@ int tch_solver_from_bits(int device, int n, size_t n_pad, const uint8_t* O, size
  * ranks, frequent one-hot columns, presence, rare equal pairs) runs on the
  * device.  tau <= 0 picks tau with the analytic GB300 cost model: a power of
  * two, or for sets whose estimate is 0.1 ms or more a quarter of the octaves
- * beside the best one when that is faster.  The rare term is kept
- * as groups of rows per rare allele and counted per stripe into a dense u16 block (tch_set_rare_term(1), the default), or built as the
- * reference's pair lists (tch_set_rare_term(0)).  Fails like the reference
+ * beside the best one when that is faster.  The rare term is kept as groups of
+ * rows per rare allele and counted per stripe into a dense u16 block
+ * (tch_set_rare_term(1), the default), or built as the reference's pair lists
+ * (tch_set_rare_term(0)).  Fails like the reference
  * when a locus has more than 65535 distinct ids or L > 65535; pair lists also
  * fail when the rare pairs reach 2^32, dense counts when the rare cells do. */
 int tch_solver_from_calls(int device, int n, int L, const uint64_t* calls, int tau, int kernel, tch_solver** out,
