@@ -656,7 +656,7 @@ __global__ void __launch_bounds__(256)
 
 template <class T>
 cudaError_t dalloc(T** p, size_t count, size_t* bytes) {
-    cudaError_t e = cudaMalloc((void**)p, std::max<size_t>(count, 1) * sizeof(T));
+    cudaError_t e = device_alloc((void**)p, std::max<size_t>(count, 1) * sizeof(T));
     if (e == cudaSuccess && bytes) *bytes += count * sizeof(T);
     return e;
 }
@@ -715,6 +715,19 @@ cudaError_t working_pool(int device, cudaMemPool_t* out) {
     }
     *out = pools[device];
     return cudaSuccess;
+}
+
+// cudaMalloc that gives the pool's unused memory back before it fails.
+cudaError_t device_alloc(void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaErrorMemoryAllocation) return e;
+    int device = 0;
+    cudaMemPool_t pool;
+    if (cudaGetDevice(&device) != cudaSuccess || working_pool(device, &pool) != cudaSuccess ||
+        cudaDeviceSynchronize() != cudaSuccess || cudaMemPoolTrimTo(pool, 0) != cudaSuccess)
+        return e;
+    cudaGetLastError();
+    return cudaMalloc(p, bytes);
 }
 
 // One candidate tau: its encoding sizes, device memory and analytic time.

@@ -98,7 +98,7 @@ cudaError_t alloc_fp4(Fp4Operands* X, size_t n_rows, int kb, size_t max_chunk, b
         KChunks& k = side ? X->neg : X->pos;
         for (int c = 0; c < k.n; c++) {
             const size_t b = n_rows * (size_t)k.width_of(c);
-            const cudaError_t e = cudaMalloc(&k.p[c], std::max<size_t>(b, 16));
+            const cudaError_t e = device_alloc((void**)&k.p[c], std::max<size_t>(b, 16));
             if (e != cudaSuccess) return e;
             if (bytes) *bytes += b;
         }

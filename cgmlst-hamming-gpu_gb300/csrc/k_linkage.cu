@@ -580,7 +580,7 @@ int full_matrix(tch_solver* s, int* n_out, uint16_t** H, size_t* ld, cudaStream_
     *n_out = n;
     *ld = up((size_t)std::max(n, 1), 8);
     if (n < 2) return 0;
-    if (cudaMalloc(H, (size_t)n * *ld * 2) != cudaSuccess) {
+    if (device_alloc((void**)H, (size_t)n * *ld * 2) != cudaSuccess) {
         cudaGetLastError();
         *H = nullptr;
         return e.set("the full %d x %d matrix (%.1f GB) does not fit in device memory", n, n,

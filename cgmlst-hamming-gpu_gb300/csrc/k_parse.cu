@@ -412,7 +412,7 @@ int tch_tsv_parse(int device, const char* text, size_t len, char sep, int skip_r
     TCH_CK(e, cudaSetDevice(device));
     {
         // ---- text to the device (16 bytes of slack past the end)
-        TCH_CK(e, cudaMalloc(&d_text, len + 16));
+        TCH_CK(e, device_alloc((void**)&d_text, len + 16));
         TCH_CK(e, cudaMemcpy(d_text, text, len, cudaMemcpyHostToDevice));
         TCH_CK(e, cudaMemset(d_text + len, 0, 16));
         // ---- newlines
@@ -466,7 +466,7 @@ int tch_tsv_parse(int device, const char* text, size_t len, char sep, int skip_r
         t->device = device;
         t->n = (int)n;
         t->L = (int)L;
-        TCH_CK(e, cudaMalloc(&t->calls, std::max<uint64_t>(n * L, 1) * 8));
+        TCH_CK(e, device_alloc((void**)&t->calls, std::max<uint64_t>(n * L, 1) * 8));
         TCH_CK(e, cudaMalloc(&d_rb, std::max<uint64_t>(n, 1) * 8));
         TCH_CK(e, cudaMalloc(&d_re, std::max<uint64_t>(n, 1) * 8));
         TCH_CK(e, cudaMalloc(&d_id, std::max<uint64_t>(n, 1) * 8));
@@ -570,7 +570,7 @@ int tch_tsv_filter(tch_tsv* t, double locus_pct, double sample_pct, char* err, i
             const int L2 = (int)keep.size();
             TCH_CK(e, cudaMalloc(&d_cols, std::max<size_t>(keep.size(), 1) * 4));
             if (L2) TCH_CK(e, cudaMemcpy(d_cols, keep.data(), keep.size() * 4, cudaMemcpyHostToDevice));
-            TCH_CK(e, cudaMalloc(&d_new, std::max<size_t>((size_t)n * L2, 1) * 8));
+            TCH_CK(e, device_alloc((void**)&d_new, std::max<size_t>((size_t)n * L2, 1) * 8));
             if ((size_t)n * L2)
                 gather_kernel<<<(unsigned)std::min<size_t>(((size_t)n * L2 + 255) / 256, 65535), 256>>>(
                     t->calls, L, nullptr, d_cols, n, L2, d_new);
@@ -598,7 +598,7 @@ int tch_tsv_filter(tch_tsv* t, double locus_pct, double sample_pct, char* err, i
             const int n2 = (int)keep.size();
             TCH_CK(e, cudaMalloc(&d_rows, std::max<size_t>(keep.size(), 1) * 4));
             if (n2) TCH_CK(e, cudaMemcpy(d_rows, keep.data(), keep.size() * 4, cudaMemcpyHostToDevice));
-            TCH_CK(e, cudaMalloc(&d_new, std::max<size_t>((size_t)n2 * L, 1) * 8));
+            TCH_CK(e, device_alloc((void**)&d_new, std::max<size_t>((size_t)n2 * L, 1) * 8));
             if ((size_t)n2 * L)
                 gather_kernel<<<(unsigned)std::min<size_t>(((size_t)n2 * L + 255) / 256, 65535), 256>>>(
                     t->calls, L, d_rows, nullptr, n2, L, d_new);

@@ -665,7 +665,7 @@ int tch_db_create(int device, int n, int L, const uint64_t* calls, int tau, tch_
         TCH_CK(e, cudaFuncSetAttribute(query_few_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)sizeof(FewShared)));
     }
-    TCH_CK(e, cudaMalloc(&d_calls, (size_t)n * L * 8));
+    TCH_CK(e, device_alloc((void**)&d_calls, (size_t)n * L * 8));
     TCH_CK(e, cudaMemcpy(d_calls, calls, (size_t)n * L * 8, cudaMemcpyHostToDevice));
     {
         TauModel model;

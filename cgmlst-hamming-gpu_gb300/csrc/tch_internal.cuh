@@ -381,10 +381,12 @@ struct TauTable {
 constexpr int kSchedSubs[2] = {0, 8192};
 constexpr int kSchedGroups[3] = {4, 8, 16};
 
-// With table != nullptr the encoder stops after the counts and fills it.
-// Stream-ordered working memory of the calls that build solvers.
+// Stream-ordered working memory of the calls that build solvers, and cudaMalloc
+// that gives what this pool keeps unused back before it fails.
 cudaError_t working_pool(int device, cudaMemPool_t* out);
+cudaError_t device_alloc(void** p, size_t bytes);
 
+// With table != nullptr the encoder stops after the counts and fills it.
 int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_req, const TauModel& model,
                      bool verbose, size_t max_chunk_bytes, int flags, DeviceEncoding* out, Err& e,
                      TauTable* table = nullptr);

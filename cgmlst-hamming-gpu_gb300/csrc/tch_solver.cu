@@ -166,7 +166,7 @@ struct tch_solver {
 namespace tch {
 
 static cudaError_t dmalloc(tch_solver* s, void** p, size_t bytes) {
-    cudaError_t e = cudaMalloc(p, bytes ? bytes : 16);
+    cudaError_t e = device_alloc(p, bytes ? bytes : 16);
     if (e == cudaSuccess) s->bytes += bytes;
     return e;
 }
@@ -767,7 +767,7 @@ static int solver_run(tch_solver* s, int S, tch_cb cb, void* ctx, double* gpu_se
     TCH_CK(e, cudaSetDevice(s->device));
     TCH_CK(e, pinned_acquire((size_t)S * ldo * 2, hU, &pooled));
     for (int b = 0; b < 2; b++) {
-        TCH_CK(e, cudaMalloc(&dU[b], (size_t)S * ldo * 2));
+        TCH_CK(e, device_alloc((void**)&dU[b], (size_t)S * ldo * 2));
         TCH_CK(e, cudaStreamCreateWithFlags(&st[b], cudaStreamNonBlocking));
         TCH_CK(e, cudaEventCreateWithFlags(&done[b], cudaEventDisableTiming));
     }
