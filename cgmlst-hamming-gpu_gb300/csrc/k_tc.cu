@@ -512,7 +512,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
             // columns of this tile and set: [j0, j_end)
             const int j_end = min(n, j0 + BN);
             // the rare counts, fetched while the MMAs of the tile run; a row of the
-            // block is at least up(n - c0, 8) wide, so a live 16 bytes is in bounds
+            // block is at least up(n - c0, 8) wide, so a live 16 bytes is in bounds.
+            // Plain loads: the kernel that writes the block may still run when this
+            // one starts, and the read-only path (ld.global.nc, __ldg) may only be
+            // used on what nobody writes while a kernel runs.
             uint4 r4[WARP_CHUNKS][4];
 #pragma unroll
             for (int cc = 0; cc < WARP_CHUNKS; cc++) {
@@ -522,7 +525,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
                     const int i = i0 + 8 * g + lrow;
                     r4[cc][g] = make_uint4(0, 0, 0, 0);
                     if (dense && c_begin + cc < c_end && cb >= j_min && i < iend && j < j_end)
-                        r4[cc][g] = __ldg(reinterpret_cast<const uint4*>(rdense + (size_t)(i - r0) * ldr + (j - c0)));
+                        r4[cc][g] = *reinterpret_cast<const uint4*>(rdense + (size_t)(i - r0) * ldr + (j - c0));
                 }
             }
             if (!mbar_wait(&tfull[acc], aph, abort_flag, p.err)) break;
