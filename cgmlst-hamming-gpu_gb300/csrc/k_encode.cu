@@ -35,6 +35,7 @@
 #include <vector>
 
 #include <math.h>
+#include <stdlib.h>
 
 #include "tch_internal.cuh"
 
@@ -687,6 +688,14 @@ struct Working {
     }
 };
 
+// Device memory for the hash tables of one batch of loci.  Test hook:
+// TCH_ENCODE_BATCH_BYTES, so that a few loci take several batches.
+size_t batch_bytes() {
+    const char* v = getenv("TCH_ENCODE_BATCH_BYTES");
+    const long long x = v ? atoll(v) : 0;
+    return x > 0 ? (size_t)x : (size_t)2 << 30;
+}
+
 int grid_for(size_t total, int sms) { return (int)std::min<size_t>((total + 255) / 256, (size_t)sms * 32); }
 
 }  // namespace
@@ -994,7 +1003,7 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
         lcap = (uint32_t)std::min<size_t>(std::min<int>(std::max(n, 1), (int)kMaxDistinct), C);
         // loci per batch: hash tables + id lists within ~2 GB
         nk_max = (int)std::max<size_t>(
-            1, std::min<size_t>((size_t)L, ((size_t)2 << 30) / (C * (8 + 4 + 2) + (size_t)lcap * 12)));
+            1, std::min<size_t>((size_t)L, batch_bytes() / (C * (8 + 4 + 2) + (size_t)lcap * 12)));
         TCH_CK(e, work.get(&keys, C * nk_max));
         TCH_CK(e, work.get(&cnts, C * nk_max));
         TCH_CK(e, work.get(&rank_slot, C * nk_max));
@@ -1048,8 +1057,10 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
             if (!one_batch) {
                 TCH_CK(e, cudaMemset(keys, 0, C * nk * sizeof(unsigned long long)));
                 TCH_CK(e, cudaMemset(cnts, 0, C * nk * sizeof(uint32_t)));
-                insert_kernel<<<grid_for((size_t)n * nk, sms), 256>>>(d_calls, n, L, k0, nk, keys, cnts, logC, max_probe,
-                                                                       nd, err_d);
+                // every id has a place (the first sweep gave it one), but how far it
+                // lies depends on the order in which the threads came: no limit
+                insert_kernel<<<grid_for((size_t)n * nk, sms), 256>>>(d_calls, n, L, k0, nk, keys, cnts, logC, C, nd,
+                                                                       err_d);
                 TCH_CK(e, cudaGetLastError());
             }
             rank_kernel<<<nk, 512>>>(k0, keys, cnts, logC, nd, cnt_off_d, cnt_flat, rank_slot, list_keys, list_slots,
