@@ -91,7 +91,7 @@ int ensure_rbuf(tch_batch* b, int k, size_t bytes, Err& e) {
     cudaFree(b->rbuf[k]);
     b->rbuf[k] = nullptr;
     b->rbytes[k] = 0;
-    TCH_CK(e, device_alloc((void**)&b->rbuf[k], bytes));
+    TCH_CK(e, device_alloc(&b->rbuf[k], bytes));
     b->rbytes[k] = bytes;
     return 0;
 fail:
@@ -144,11 +144,11 @@ int prepare_persistent(tch_batch* b, uint16_t* d_out, Err& e) {
         cudaFree(b->pbuf);
         b->pbuf = nullptr;
         b->pbytes = 0;
-        TCH_CK(e, device_alloc((void**)&b->pbuf, total * 2));
+        TCH_CK(e, device_alloc(&b->pbuf, total * 2));
         b->pbytes = total * 2;
     }
     if (!b->dErr) {
-        TCH_CK(e, cudaMalloc(&b->dErr, sizeof(int)));
+        TCH_CK(e, device_alloc(&b->dErr, sizeof(int)));
         TCH_CK(e, cudaMemset(b->dErr, 0, sizeof(int)));
     }
     {

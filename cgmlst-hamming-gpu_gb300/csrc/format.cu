@@ -256,7 +256,7 @@ extern "C" int tch_solver_write_tsv(tch_solver* s, const char* const* ids, const
     TCH_CK(e, cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
     TCH_CK(e, cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
     TCH_CK(e, working_pool(dev, &pool));
-    TCH_CK(e, cudaMallocFromPoolAsync((void**)&H, (size_t)n * ld * 2, pool, st));
+    TCH_CK(e, pool_alloc(&H, (size_t)n * ld * 2, pool, st));
     if (n > 1) {
         if (tch_solver_stripe(s, 0, n, H, ld, st, err, errlen)) goto fail;
         TCH_CK(e, cudaStreamSynchronize(st));
@@ -266,9 +266,9 @@ extern "C" int tch_solver_write_tsv(tch_solver* s, const char* const* ids, const
     {
         std::string all_ids;
         for (int i = 0; i < n; i++) all_ids += ids[i];
-        TCH_CK(e, cudaMallocFromPoolAsync((void**)&d_ids, std::max<size_t>(all_ids.size(), 1), pool, st));
-        TCH_CK(e, cudaMallocFromPoolAsync((void**)&d_idoff, ((size_t)n + 1) * 8, pool, st));
-        TCH_CK(e, cudaMallocFromPoolAsync((void**)&d_sep, 16, pool, st));
+        TCH_CK(e, pool_alloc(&d_ids, std::max<size_t>(all_ids.size(), 1), pool, st));
+        TCH_CK(e, pool_alloc(&d_idoff, ((size_t)n + 1) * 8, pool, st));
+        TCH_CK(e, pool_alloc(&d_sep, 16, pool, st));
         if (!all_ids.empty())
             TCH_CK(e, cudaMemcpyAsync(d_ids, all_ids.data(), all_ids.size(), cudaMemcpyHostToDevice, st));
         TCH_CK(e, cudaMemcpyAsync(d_idoff, idoff.data(), ((size_t)n + 1) * 8, cudaMemcpyHostToDevice, st));
@@ -281,11 +281,11 @@ extern "C" int tch_solver_write_tsv(tch_solver* s, const char* const* ids, const
         for (int i = 0; i < n; i++) maxid = std::max<size_t>(maxid, idoff[i + 1] - idoff[i]);
         cap_bytes = (size_t)block_rows * (maxid + (size_t)n * (seplen + 5) + 1);
     }
-    TCH_CK(e, cudaMallocFromPoolAsync((void**)&d_len, (size_t)block_rows * 8, pool, st));
+    TCH_CK(e, pool_alloc(&d_len, (size_t)block_rows * 8, pool, st));
     pooled = text_acquire(cap_bytes, h_text);
     for (int b = 0; b < 2; b++) {
-        TCH_CK(e, cudaMallocFromPoolAsync((void**)&d_off[b], ((size_t)block_rows + 1) * 8, pool, st));
-        TCH_CK(e, cudaMallocFromPoolAsync((void**)&d_text[b], cap_bytes, pool, st));
+        TCH_CK(e, pool_alloc(&d_off[b], ((size_t)block_rows + 1) * 8, pool, st));
+        TCH_CK(e, pool_alloc(&d_text[b], cap_bytes, pool, st));
         if (!pooled) TCH_CK(e, cudaMallocHost(&h_text[b], cap_bytes));
         TCH_CK(e, cudaEventCreateWithFlags(&done[b], cudaEventDisableTiming));
         TCH_CK(e, cudaEventCreateWithFlags(&ready[b], cudaEventDisableTiming));

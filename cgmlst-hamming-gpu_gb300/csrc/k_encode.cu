@@ -31,7 +31,6 @@
 // work (hashed ids included).
 
 #include <chrono>
-#include <mutex>
 #include <vector>
 
 #include <math.h>
@@ -657,7 +656,7 @@ __global__ void __launch_bounds__(256)
 
 template <class T>
 cudaError_t dalloc(T** p, size_t count, size_t* bytes) {
-    cudaError_t e = device_alloc((void**)p, std::max<size_t>(count, 1) * sizeof(T));
+    cudaError_t e = device_alloc(p, std::max<size_t>(count, 1) * sizeof(T));
     if (e == cudaSuccess && bytes) *bytes += count * sizeof(T);
     return e;
 }
@@ -668,7 +667,7 @@ struct Working {
     std::vector<void*> held;
     template <class T>
     cudaError_t get(T** p, size_t count) {
-        const cudaError_t e = cudaMallocFromPoolAsync((void**)p, std::max<size_t>(count, 1) * sizeof(T), pool, 0);
+        const cudaError_t e = pool_alloc(p, std::max<size_t>(count, 1) * sizeof(T), pool, 0);
         if (e == cudaSuccess) held.push_back(*p);
         return e;
     }
@@ -699,45 +698,6 @@ size_t batch_bytes() {
 int grid_for(size_t total, int sms) { return (int)std::min<size_t>((total + 255) / 256, (size_t)sms * 32); }
 
 }  // namespace
-
-// Working memory for building solvers, from a stream-ordered pool per device that
-// keeps up to 512 MB between calls (mapping it anew took a millisecond of a small
-// set's encoding); the driver hands back what is above that.
-cudaError_t working_pool(int device, cudaMemPool_t* out) {
-    constexpr uint64_t kKeptBytes = (uint64_t)512 << 20;
-    static std::mutex mu;
-    static cudaMemPool_t pools[kMaxDevices] = {};
-    if (device < 0 || device >= kMaxDevices) return cudaErrorInvalidDevice;
-    std::lock_guard<std::mutex> lk(mu);
-    if (!pools[device]) {
-        cudaMemPoolProps props = {};
-        props.allocType = cudaMemAllocationTypePinned;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = device;
-        cudaMemPool_t pool;
-        cudaError_t e = cudaMemPoolCreate(&pool, &props);
-        if (e != cudaSuccess) return e;
-        uint64_t keep = kKeptBytes;
-        e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-        if (e != cudaSuccess) return e;
-        pools[device] = pool;
-    }
-    *out = pools[device];
-    return cudaSuccess;
-}
-
-// cudaMalloc that gives the pool's unused memory back before it fails.
-cudaError_t device_alloc(void** p, size_t bytes) {
-    cudaError_t e = cudaMalloc(p, bytes);
-    if (e != cudaErrorMemoryAllocation) return e;
-    int device = 0;
-    cudaMemPool_t pool;
-    if (cudaGetDevice(&device) != cudaSuccess || working_pool(device, &pool) != cudaSuccess ||
-        cudaDeviceSynchronize() != cudaSuccess || cudaMemPoolTrimTo(pool, 0) != cudaSuccess)
-        return e;
-    cudaGetLastError();
-    return cudaMalloc(p, bytes);
-}
 
 // One candidate tau: its encoding sizes, device memory and analytic time.
 struct TauRow {
@@ -943,7 +903,7 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
     const bool dense_rare = (flags & (ENC_DENSE | ENC_QUERY)) != 0;
     const bool query_maps = (flags & ENC_QUERY) != 0;
     int sms = 0, hflag = 0;
-    size_t freeb = 0, totb = 0, tmp_bytes = 0;
+    size_t freeb = 0, tmp_bytes = 0;
     // Hash tables for kSmallTable ids per locus first: schemes have a few thousand
     // alleles per locus at most, and clearing and scanning tables that hold as many
     // ids as there are rows cost more than the inserts (10 007 x 1 343: 32 768 places
@@ -1089,7 +1049,7 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
     {
         int tau = tau_req;
         TCH_CK(e, cudaStreamSynchronize(0));  // the pool lets go of what it does not keep
-        TCH_CK(e, cudaMemGetInfo(&freeb, &totb));
+        TCH_CK(e, free_memory(device, &freeb));
         if (table) {  // candidates and features only
             tau_features(tau_rows(bins_h, n, L, freeb, model, dense_rare), bins_h, off_h, n, L, table);
             free_device_encoding(out);
@@ -1197,7 +1157,7 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
             TCH_CK(e, cudaGetLastError());
             // bit columns for the smallest batches, when they leave most of the memory free
             const size_t words = up((size_t)n, 1024) / 32, columns = (size_t)D + L;
-            TCH_CK(e, cudaMemGetInfo(&freeb, &totb));
+            TCH_CK(e, free_memory(device, &freeb));
             if (columns * words * 4 <= freeb / 4) {
                 TCH_CK(e, dalloc(&out->bits, columns * words, &out->bytes));
                 out->bit_words = words;

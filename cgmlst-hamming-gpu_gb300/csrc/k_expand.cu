@@ -98,7 +98,7 @@ cudaError_t alloc_fp4(Fp4Operands* X, size_t n_rows, int kb, size_t max_chunk, b
         KChunks& k = side ? X->neg : X->pos;
         for (int c = 0; c < k.n; c++) {
             const size_t b = n_rows * (size_t)k.width_of(c);
-            const cudaError_t e = device_alloc((void**)&k.p[c], std::max<size_t>(b, 16));
+            const cudaError_t e = device_alloc(&k.p[c], std::max<size_t>(b, 16));
             if (e != cudaSuccess) return e;
             if (bytes) *bytes += b;
         }
@@ -127,7 +127,7 @@ cudaError_t launch_expand_bits(const BitOperands& bits, int n, int wp, int wo, c
 cudaError_t used_bit_words(const BitOperands& bits, size_t n_pad, int* wp, int* wo, cudaStream_t st) {
     int* d = nullptr;
     int h[2] = {0, 0};
-    cudaError_t e = cudaMalloc(&d, 8);
+    cudaError_t e = device_alloc(&d, 8);
     if (e == cudaSuccess) e = cudaMemsetAsync(d, 0, 8, st);
     const size_t total = n_pad * (size_t)(bits.wP + bits.wO);
     if (e == cudaSuccess && total) {

@@ -462,7 +462,7 @@ int mst_on_device(const uint16_t* d_H, size_t ld, int n, cudaStream_t st, uint32
     // the lists' room (128 bytes a profile) serves the gathered edges afterwards
     const size_t bytes = sizeof(MstState) + n8 * (8 * kListed + 8 + 8 + 4 * 4 + 4 + 4 + 2 + 1) + 16 +
                          ((size_t)2 * kDistances + 4) * 4;
-    TCH_CK(e, cudaMallocAsync(&ws, bytes, st));
+    TCH_CK(e, pool_alloc(&ws, bytes, nullptr, st));
     lists = reinterpret_cast<unsigned long long*>(ws);
     best = lists + n8 * kListed;
     edges = best + n8;
@@ -546,7 +546,7 @@ int neighbors_on_device(const uint16_t* d_H, size_t ld, int n, int k, cudaStream
     int* derr;
     int rc = 1, herr = 0;
     const size_t cells = (size_t)n * k;
-    TCH_CK(e, cudaMallocAsync(&ws, cells * 6 + 64, st));
+    TCH_CK(e, pool_alloc(&ws, cells * 6 + 64, nullptr, st));
     d_idx = reinterpret_cast<uint32_t*>(ws);
     derr = reinterpret_cast<int*>(d_idx + cells);
     d_dist = reinterpret_cast<uint16_t*>(derr + 4);
@@ -580,7 +580,7 @@ int full_matrix(tch_solver* s, int* n_out, uint16_t** H, size_t* ld, cudaStream_
     *n_out = n;
     *ld = up((size_t)std::max(n, 1), 8);
     if (n < 2) return 0;
-    if (device_alloc((void**)H, (size_t)n * *ld * 2) != cudaSuccess) {
+    if (device_alloc(H, (size_t)n * *ld * 2) != cudaSuccess) {
         cudaGetLastError();
         *H = nullptr;
         return e.set("the full %d x %d matrix (%.1f GB) does not fit in device memory", n, n,

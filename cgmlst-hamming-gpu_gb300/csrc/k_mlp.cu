@@ -162,16 +162,16 @@ int mlp_run(int device, const float* w, const float* X, const float* y, int n, f
     float *dw = nullptr, *dX = nullptr, *dy = nullptr, *dp = nullptr, *dl = nullptr, *dg = nullptr, *ds = nullptr;
     if (n < 0 || !w || (n > 0 && !X)) return e.set("mlp: bad arguments");
     TCH_CK(e, cudaSetDevice(device));
-    TCH_CK(e, cudaMalloc(&dw, NP * 4));
-    TCH_CK(e, cudaMalloc(&dX, std::max(n, 1) * (size_t)F * 4));
-    TCH_CK(e, cudaMalloc(&dp, std::max(n, 1) * (size_t)4));
-    TCH_CK(e, cudaMalloc(&dl, 4));
-    TCH_CK(e, cudaMalloc(&dg, NP * 4));
+    TCH_CK(e, device_alloc(&dw, NP * 4));
+    TCH_CK(e, device_alloc(&dX, std::max(n, 1) * (size_t)F * 4));
+    TCH_CK(e, device_alloc(&dp, std::max(n, 1) * (size_t)4));
+    TCH_CK(e, device_alloc(&dl, 4));
+    TCH_CK(e, device_alloc(&dg, NP * 4));
     TCH_CK(e, cudaMemcpy(dw, w, NP * 4, cudaMemcpyHostToDevice));
     if (n) TCH_CK(e, cudaMemcpy(dX, X, (size_t)n * F * 4, cudaMemcpyHostToDevice));
     if (y) {
-        TCH_CK(e, cudaMalloc(&dy, std::max(n, 1) * (size_t)4));
-        TCH_CK(e, cudaMalloc(&ds, std::max(n, 1) * (size_t)SW * 4));
+        TCH_CK(e, device_alloc(&dy, std::max(n, 1) * (size_t)4));
+        TCH_CK(e, device_alloc(&ds, std::max(n, 1) * (size_t)SW * 4));
         if (n) TCH_CK(e, cudaMemcpy(dy, y, (size_t)n * 4, cudaMemcpyHostToDevice));
     }
     if (n) {
@@ -203,15 +203,15 @@ int mlp_train(int device, float* w, const float* X, const float* y, int n, int s
     cudaGraphExec_t exec = nullptr;
     if (n <= 0 || steps < 0 || !w || !X || !y || !(lr > 0)) return e.set("mlp: bad training arguments");
     TCH_CK(e, cudaSetDevice(device));
-    TCH_CK(e, cudaMalloc(&dw, NP * 4));
-    TCH_CK(e, cudaMalloc(&dg, NP * 4));
-    TCH_CK(e, cudaMalloc(&dm, NP * 4));
-    TCH_CK(e, cudaMalloc(&dv, NP * 4));
-    TCH_CK(e, cudaMalloc(&dX, (size_t)n * F * 4));
-    TCH_CK(e, cudaMalloc(&dy, (size_t)n * 4));
-    TCH_CK(e, cudaMalloc(&ds, (size_t)n * SW * 4));
-    TCH_CK(e, cudaMalloc(&dl, 4));
-    TCH_CK(e, cudaMalloc(&dstep, 4));
+    TCH_CK(e, device_alloc(&dw, NP * 4));
+    TCH_CK(e, device_alloc(&dg, NP * 4));
+    TCH_CK(e, device_alloc(&dm, NP * 4));
+    TCH_CK(e, device_alloc(&dv, NP * 4));
+    TCH_CK(e, device_alloc(&dX, (size_t)n * F * 4));
+    TCH_CK(e, device_alloc(&dy, (size_t)n * 4));
+    TCH_CK(e, device_alloc(&ds, (size_t)n * SW * 4));
+    TCH_CK(e, device_alloc(&dl, 4));
+    TCH_CK(e, device_alloc(&dstep, 4));
     TCH_CK(e, cudaMemcpy(dw, w, NP * 4, cudaMemcpyHostToDevice));
     TCH_CK(e, cudaMemcpy(dX, X, (size_t)n * F * 4, cudaMemcpyHostToDevice));
     TCH_CK(e, cudaMemcpy(dy, y, (size_t)n * 4, cudaMemcpyHostToDevice));

@@ -412,21 +412,21 @@ int tch_tsv_parse(int device, const char* text, size_t len, char sep, int skip_r
     TCH_CK(e, cudaSetDevice(device));
     {
         // ---- text to the device (16 bytes of slack past the end)
-        TCH_CK(e, device_alloc((void**)&d_text, len + 16));
+        TCH_CK(e, device_alloc(&d_text, len + 16));
         TCH_CK(e, cudaMemcpy(d_text, text, len, cudaMemcpyHostToDevice));
         TCH_CK(e, cudaMemset(d_text + len, 0, 16));
         // ---- newlines
         const size_t chunks = (len + kChunk - 1) / kChunk;
-        TCH_CK(e, cudaMalloc(&d_counts, std::max<size_t>(chunks, (len + 255) / 256 + 1) * 4));
+        TCH_CK(e, device_alloc(&d_counts, std::max<size_t>(chunks, (len + 255) / 256 + 1) * 4));
         newlines_kernel<<<(unsigned)chunks, kChunkThreads>>>(d_text, len, 0, d_counts, nullptr, nullptr);
         TCH_CK(e, cudaGetLastError());
         std::vector<uint32_t> cnt(chunks);
         TCH_CK(e, cudaMemcpy(cnt.data(), d_counts, chunks * 4, cudaMemcpyDeviceToHost));
         uint64_t nnl = 0;
         std::vector<uint64_t> base = host_scan(cnt, &nnl);
-        TCH_CK(e, cudaMalloc(&d_base, std::max<size_t>(chunks, 1) * 8));
+        TCH_CK(e, device_alloc(&d_base, std::max<size_t>(chunks, 1) * 8));
         TCH_CK(e, cudaMemcpy(d_base, base.data(), chunks * 8, cudaMemcpyHostToDevice));
-        TCH_CK(e, cudaMalloc(&d_nl, std::max<uint64_t>(nnl, 1) * 8));
+        TCH_CK(e, device_alloc(&d_nl, std::max<uint64_t>(nnl, 1) * 8));
         newlines_kernel<<<(unsigned)chunks, kChunkThreads>>>(d_text, len, 1, nullptr, d_base, d_nl);
         TCH_CK(e, cudaGetLastError());
         // str::lines: a last line without '\n' when text follows the last newline
@@ -440,7 +440,7 @@ int tch_tsv_parse(int device, const char* text, size_t len, char sep, int skip_r
         if (rblocks) {
             TCH_CK(e, cudaFree(d_counts));
             d_counts = nullptr;
-            TCH_CK(e, cudaMalloc(&d_counts, rblocks * 4));
+            TCH_CK(e, device_alloc(&d_counts, rblocks * 4));
             rows_kernel<<<(unsigned)rblocks, 256>>>(d_text, len, d_nl, nnl, nlines, 0, d_counts, nullptr, nullptr,
                                                     nullptr);
             TCH_CK(e, cudaGetLastError());
@@ -466,17 +466,17 @@ int tch_tsv_parse(int device, const char* text, size_t len, char sep, int skip_r
         t->device = device;
         t->n = (int)n;
         t->L = (int)L;
-        TCH_CK(e, device_alloc((void**)&t->calls, std::max<uint64_t>(n * L, 1) * 8));
-        TCH_CK(e, cudaMalloc(&d_rb, std::max<uint64_t>(n, 1) * 8));
-        TCH_CK(e, cudaMalloc(&d_re, std::max<uint64_t>(n, 1) * 8));
-        TCH_CK(e, cudaMalloc(&d_id, std::max<uint64_t>(n, 1) * 8));
-        TCH_CK(e, cudaMalloc(&d_bad, 4));
+        TCH_CK(e, device_alloc(&t->calls, std::max<uint64_t>(n * L, 1) * 8));
+        TCH_CK(e, device_alloc(&d_rb, std::max<uint64_t>(n, 1) * 8));
+        TCH_CK(e, device_alloc(&d_re, std::max<uint64_t>(n, 1) * 8));
+        TCH_CK(e, device_alloc(&d_id, std::max<uint64_t>(n, 1) * 8));
+        TCH_CK(e, device_alloc(&d_bad, 4));
         const int none = INT32_MAX;
         TCH_CK(e, cudaMemcpy(d_bad, &none, 4, cudaMemcpyHostToDevice));
         if (rblocks) {
             TCH_CK(e, cudaFree(d_base));
             d_base = nullptr;
-            TCH_CK(e, cudaMalloc(&d_base, rblocks * 8));
+            TCH_CK(e, device_alloc(&d_base, rblocks * 8));
             TCH_CK(e, cudaMemcpy(d_base, rbase.data(), rblocks * 8, cudaMemcpyHostToDevice));
             rows_kernel<<<(unsigned)rblocks, 256>>>(d_text, len, d_nl, nnl, nlines, 1, nullptr, d_base, d_rb, d_re);
             TCH_CK(e, cudaGetLastError());
@@ -554,7 +554,7 @@ int tch_tsv_filter(tch_tsv* t, double locus_pct, double sample_pct, char* err, i
     TCH_CK(e, cudaSetDevice(t->device));
     if (locus_pct >= 0 && t->L > 0) {  // main.rs:313-330 (no samples: 0 / 0 keeps no locus)
         const int n = t->n, L = t->L, rpb = 1024;
-        TCH_CK(e, cudaMalloc(&d_lc, (size_t)L * 8));
+        TCH_CK(e, device_alloc(&d_lc, (size_t)L * 8));
         TCH_CK(e, cudaMemset(d_lc, 0, (size_t)L * 8));
         if (n) {
             const dim3 grid((unsigned)((L + 255) / 256), (unsigned)((n + rpb - 1) / rpb));
@@ -568,9 +568,9 @@ int tch_tsv_filter(tch_tsv* t, double locus_pct, double sample_pct, char* err, i
             if (((double)lc[k] / (double)n) * 100.0 >= locus_pct) keep.push_back(k);
         if ((int)keep.size() != L) {
             const int L2 = (int)keep.size();
-            TCH_CK(e, cudaMalloc(&d_cols, std::max<size_t>(keep.size(), 1) * 4));
+            TCH_CK(e, device_alloc(&d_cols, std::max<size_t>(keep.size(), 1) * 4));
             if (L2) TCH_CK(e, cudaMemcpy(d_cols, keep.data(), keep.size() * 4, cudaMemcpyHostToDevice));
-            TCH_CK(e, device_alloc((void**)&d_new, std::max<size_t>((size_t)n * L2, 1) * 8));
+            TCH_CK(e, device_alloc(&d_new, std::max<size_t>((size_t)n * L2, 1) * 8));
             if ((size_t)n * L2)
                 gather_kernel<<<(unsigned)std::min<size_t>(((size_t)n * L2 + 255) / 256, 65535), 256>>>(
                     t->calls, L, nullptr, d_cols, n, L2, d_new);
@@ -586,7 +586,7 @@ int tch_tsv_filter(tch_tsv* t, double locus_pct, double sample_pct, char* err, i
         const int n = t->n, L = t->L;
         std::vector<uint32_t> sc(n, 0);
         if (L > 0) {
-            TCH_CK(e, cudaMalloc(&d_sc, (size_t)n * 4));
+            TCH_CK(e, device_alloc(&d_sc, (size_t)n * 4));
             sample_counts_kernel<<<(unsigned)(((size_t)n * 32 + 255) / 256), 256>>>(t->calls, n, L, d_sc);
             TCH_CK(e, cudaGetLastError());
             TCH_CK(e, cudaMemcpy(sc.data(), d_sc, (size_t)n * 4, cudaMemcpyDeviceToHost));
@@ -596,9 +596,9 @@ int tch_tsv_filter(tch_tsv* t, double locus_pct, double sample_pct, char* err, i
             if (((double)sc[i] / (double)L) * 100.0 >= sample_pct) keep.push_back(i);
         if ((int)keep.size() != n) {
             const int n2 = (int)keep.size();
-            TCH_CK(e, cudaMalloc(&d_rows, std::max<size_t>(keep.size(), 1) * 4));
+            TCH_CK(e, device_alloc(&d_rows, std::max<size_t>(keep.size(), 1) * 4));
             if (n2) TCH_CK(e, cudaMemcpy(d_rows, keep.data(), keep.size() * 4, cudaMemcpyHostToDevice));
-            TCH_CK(e, device_alloc((void**)&d_new, std::max<size_t>((size_t)n2 * L, 1) * 8));
+            TCH_CK(e, device_alloc(&d_new, std::max<size_t>((size_t)n2 * L, 1) * 8));
             if ((size_t)n2 * L)
                 gather_kernel<<<(unsigned)std::min<size_t>(((size_t)n2 * L + 255) / 256, 65535), 256>>>(
                     t->calls, L, d_rows, nullptr, n2, L, d_new);

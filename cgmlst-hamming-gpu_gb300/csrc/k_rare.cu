@@ -580,8 +580,8 @@ cudaError_t rare_batch_prepare(const std::vector<RareBatchItem>& items, RareBatc
     plan->total_rows = row0;
     plan->cwords = cwords;
     if (jobs.empty()) return cudaSuccess;
-    cudaError_t e = cudaMalloc(&plan->d_jobs, jobs.size() * sizeof(RareJob));
-    if (e == cudaSuccess) e = cudaMalloc(&plan->d_row_job, row_job.size() * sizeof(int));
+    cudaError_t e = device_alloc(&plan->d_jobs, jobs.size() * sizeof(RareJob));
+    if (e == cudaSuccess) e = device_alloc(&plan->d_row_job, row_job.size() * sizeof(int));
     if (e == cudaSuccess)
         e = cudaMemcpy(plan->d_jobs, jobs.data(), jobs.size() * sizeof(RareJob), cudaMemcpyHostToDevice);
     if (e == cudaSuccess)

@@ -794,10 +794,10 @@ cudaError_t tc_batch_prepare(const std::vector<TcBatchItem>& items, int num_sms,
     std::vector<int> first;
     spread_tiles(jobs, tiles_of, npairs, &tiles, &first);
     plan->num_tiles = num_tiles;
-    cudaError_t e = cudaMalloc(&plan->d_jobs, jobs.size() * sizeof(TcJob));
-    if (e == cudaSuccess) e = cudaMalloc(&plan->d_maps, mh.size() * sizeof(CUtensorMap));
-    if (e == cudaSuccess) e = cudaMalloc(&plan->d_tiles, tiles.size() * sizeof(int2));
-    if (e == cudaSuccess) e = cudaMalloc(&plan->d_first, first.size() * sizeof(int));
+    cudaError_t e = device_alloc(&plan->d_jobs, jobs.size() * sizeof(TcJob));
+    if (e == cudaSuccess) e = device_alloc(&plan->d_maps, mh.size() * sizeof(CUtensorMap));
+    if (e == cudaSuccess) e = device_alloc(&plan->d_tiles, tiles.size() * sizeof(int2));
+    if (e == cudaSuccess) e = device_alloc(&plan->d_first, first.size() * sizeof(int));
     if (e == cudaSuccess) e = cudaMemcpy(plan->d_jobs, jobs.data(), jobs.size() * sizeof(TcJob), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(plan->d_maps, mh.data(), mh.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice);
     if (e == cudaSuccess)

@@ -453,7 +453,7 @@ int db_query(tch_db* db, int m, const uint64_t* qcalls, uint16_t* h_qdb, uint16_
             place(&derr, 4);
             zero = bytes - zero_at;
         }
-        if (pass == 0) ce = cudaMallocFromPoolAsync((void**)&work, bytes, db->pool, st);
+        if (pass == 0) ce = pool_alloc(&work, bytes, db->pool, st);
         if (ce != cudaSuccess) goto done;
     }
     mark();
@@ -665,7 +665,7 @@ int tch_db_create(int device, int n, int L, const uint64_t* calls, int tau, tch_
         TCH_CK(e, cudaFuncSetAttribute(query_few_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)sizeof(FewShared)));
     }
-    TCH_CK(e, device_alloc((void**)&d_calls, (size_t)n * L * 8));
+    TCH_CK(e, device_alloc(&d_calls, (size_t)n * L * 8));
     TCH_CK(e, cudaMemcpy(d_calls, calls, (size_t)n * L * 8, cudaMemcpyHostToDevice));
     {
         TauModel model;
@@ -673,6 +673,7 @@ int tch_db_create(int device, int n, int L, const uint64_t* calls, int tau, tch_
             goto fail;
     }
     cudaFree(d_calls);
+    cudaStreamSynchronize(0);  // the working pool lets go of what it does not keep
     // the database's own triangle is not served: drop its ranks and positions,
     // and its A-side operand copy (queries are the A side)
     cudaFree(db->enc.x);
@@ -746,9 +747,9 @@ int tch_server_create(tch_db* db, int slots, size_t budget, tch_server** out, ch
     tch_server* sv = new tch_server();
     sv->db = db;
     if (!budget) {
-        size_t f = 0, t = 0;
+        size_t f = 0;
         cudaSetDevice(db->device);
-        cudaMemGetInfo(&f, &t);
+        free_memory(db->device, &f);
         budget = f / 2;
     }
     sv->budget = budget;

@@ -172,6 +172,26 @@ struct StripeArgs {
     bool after_counts = false;
 };
 
+// ---- memory.cpp -------------------------------------------------------------------
+// Stream-ordered working memory of the calls that build solvers, kept between them.
+cudaError_t working_pool(int device, cudaMemPool_t* out);
+// cudaMalloc, and an allocation from a stream-ordered pool (nullptr: the device's
+// own), that give back what the working pool keeps unused before they fail.  Every
+// allocation of the library is one of the two.
+cudaError_t device_alloc(void** p, size_t bytes);
+cudaError_t pool_alloc(void** p, size_t bytes, cudaMemPool_t pool, cudaStream_t st);
+template <class T>
+cudaError_t device_alloc(T** p, size_t bytes) {
+    return device_alloc(reinterpret_cast<void**>(p), bytes);
+}
+template <class T>
+cudaError_t pool_alloc(T** p, size_t bytes, cudaMemPool_t pool, cudaStream_t st) {
+    return pool_alloc(reinterpret_cast<void**>(p), bytes, pool, st);
+}
+// Free memory of the device (the current one), what the working pool keeps unused
+// included: an allocation gets it.
+cudaError_t free_memory(int device, size_t* out);
+
 // ---- k_popc.cu --------------------------------------------------------------------
 cudaError_t launch_popc_stripe(const BitOperands& ops, const RareCSR& rare, const StripeArgs& a,
                                cudaStream_t st);
@@ -380,11 +400,6 @@ struct TauTable {
 // profile sets of the GB300 sweep (and at most 2 % faster there): not offered.
 constexpr int kSchedSubs[2] = {0, 8192};
 constexpr int kSchedGroups[3] = {4, 8, 16};
-
-// Stream-ordered working memory of the calls that build solvers, and cudaMalloc
-// that gives what this pool keeps unused back before it fails.
-cudaError_t working_pool(int device, cudaMemPool_t* out);
-cudaError_t device_alloc(void** p, size_t bytes);
 
 // With table != nullptr the encoder stops after the counts and fills it.
 int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_req, const TauModel& model,

@@ -211,7 +211,7 @@ static int solver_from_bits(int device, int n, size_t n_pad, const uint8_t* O, s
     tch_solver* s = nullptr;
     int* dflag = nullptr;
     int hflag = 0;
-    size_t freeb = 0, totb = 0;
+    size_t freeb = 0;
     bool rare_gpu = true;
     *out = nullptr;
     if (n < 0) return e.set("n must be >= 0 (got %d)", n);
@@ -268,7 +268,7 @@ static int solver_from_bits(int device, int n, size_t n_pad, const uint8_t* O, s
         s->dP = s->dO = nullptr;
     }
     // rare pairs: on the device when they fit (tch.cu:104-111), else on the host
-    TCH_CK(e, cudaMemGetInfo(&freeb, &totb));
+    TCH_CK(e, free_memory(device, &freeb));
     {
         const size_t need = (n_rare + (size_t)n + 1) * 4 + (size_t)stripe_for_fit * up((size_t)n, 8) * 2 * 2 +
                             ((size_t)64 << 20);
@@ -292,7 +292,7 @@ static int solver_from_bits(int device, int n, size_t n_pad, const uint8_t* O, s
         }
         if (n_rare) TCH_CK(e, cudaMemcpy(s->dJs, js, n_rare * 4, cudaMemcpyHostToDevice));
         // ascending rows -> subtraction fused into the contraction's epilogue
-        TCH_CK(e, cudaMalloc(&dflag, sizeof(int)));
+        TCH_CK(e, device_alloc(&dflag, sizeof(int)));
         TCH_CK(e, cudaMemset(dflag, 0, sizeof(int)));
         {
             RareCSR rc;
@@ -366,12 +366,12 @@ static int solver_from_input(int device, int n, int L, const uint64_t* calls, co
     TCH_CK(e, cudaMemset(s->dErr, 0, sizeof(int)));
     TCH_CK(e, working_pool(device, &pool));
     if (!dev_calls)
-        TCH_CK(e, cudaMallocFromPoolAsync((void**)&d_calls, std::max<size_t>((size_t)n * Le, 1) * 8, pool, 0));
+        TCH_CK(e, pool_alloc(&d_calls, std::max<size_t>((size_t)n * Le, 1) * 8, pool, 0));
     if (dev_calls) {
         // read in place
     } else if (L && ranks) {
         const size_t count = (size_t)n * L;
-        TCH_CK(e, cudaMallocFromPoolAsync((void**)&d_ranks, std::max<size_t>(count, 1) * 2, pool, 0));
+        TCH_CK(e, pool_alloc(&d_ranks, std::max<size_t>(count, 1) * 2, pool, 0));
         if (count) {
             TCH_CK(e, cudaMemcpy(d_ranks, ranks, count * 2, cudaMemcpyHostToDevice));
             widen_ranks_kernel<<<(int)std::min<size_t>((count + 255) / 256, (size_t)s->num_sms * 32), 256>>>(
@@ -390,6 +390,7 @@ static int solver_from_input(int device, int n, int L, const uint64_t* calls, co
         goto fail;
     if (d_calls) cudaFreeAsync(d_calls, 0);
     d_calls = nullptr;
+    TCH_CK(e, cudaStreamSynchronize(0));  // the pool lets go of what it does not keep
     if (enc.dense) {  // the solver takes the rare groups
         s->dense = true;
         s->gL = Le;
@@ -431,6 +432,7 @@ static int solver_from_input(int device, int n, int L, const uint64_t* calls, co
 fail:
     if (d_calls) cudaFreeAsync(d_calls, 0);
     if (d_ranks) cudaFreeAsync(d_ranks, 0);
+    cudaStreamSynchronize(0);
     solver_free(s);
     return 1;
 }
@@ -522,7 +524,7 @@ int solver_stripe(tch_solver* s, int r0, int rows, uint16_t* d_out, size_t ldo, 
         const size_t ldr = up((size_t)(s->n - q0), kRareDenseAlign);
         const size_t rbytes = (size_t)qrows * ldr * 2;
         uint16_t* R = nullptr;
-        ce = cudaMallocFromPoolAsync((void**)&R, rbytes, pool, st);
+        ce = pool_alloc(&R, rbytes, pool, st);
         if (ce != cudaSuccess)
             return e.set("rare counts of the stripe (%zu bytes): %s", rbytes, cudaGetErrorString(ce));
         StripeArgs qa = a;
@@ -767,7 +769,7 @@ static int solver_run(tch_solver* s, int S, tch_cb cb, void* ctx, double* gpu_se
     TCH_CK(e, cudaSetDevice(s->device));
     TCH_CK(e, pinned_acquire((size_t)S * ldo * 2, hU, &pooled));
     for (int b = 0; b < 2; b++) {
-        TCH_CK(e, device_alloc((void**)&dU[b], (size_t)S * ldo * 2));
+        TCH_CK(e, device_alloc(&dU[b], (size_t)S * ldo * 2));
         TCH_CK(e, cudaStreamCreateWithFlags(&st[b], cudaStreamNonBlocking));
         TCH_CK(e, cudaEventCreateWithFlags(&done[b], cudaEventDisableTiming));
     }
@@ -908,8 +910,8 @@ int tch_device_count(void) {
 }
 
 size_t tch_free_vram(int device) {
-    size_t f = 0, t = 0;
-    if (cudaSetDevice(device) != cudaSuccess || cudaMemGetInfo(&f, &t) != cudaSuccess) return 0;
+    size_t f = 0;
+    if (cudaSetDevice(device) != cudaSuccess || free_memory(device, &f) != cudaSuccess) return 0;
     return f;
 }
 
@@ -998,12 +1000,13 @@ int tch_tau_features(int device, int n, int L, const uint64_t* calls, int max_ro
     if (L > 65535) return e.set("more than 65535 loci (u16 distances)");
     if (!calls || !taus || !feats || !rows || max_rows < 0) return e.set("null buffer");
     TCH_CK(e, cudaSetDevice(device));
-    TCH_CK(e, cudaMalloc(&d_calls, (size_t)n * L * 8));
+    TCH_CK(e, device_alloc(&d_calls, (size_t)n * L * 8));
     TCH_CK(e, cudaMemcpy(d_calls, calls, (size_t)n * L * 8, cudaMemcpyHostToDevice));
     if (encode_on_device(device, n, L, d_calls, 0, g_tau_model, false, 0, rare_dense_default() ? ENC_DENSE : 0, &enc,
                          e, &table))
         goto fail;
     cudaFree(d_calls);
+    cudaStreamSynchronize(0);
     *rows = (int)std::min<size_t>(table.taus.size(), (size_t)max_rows);
     for (int r = 0; r < *rows; r++) {
         taus[r] = table.taus[r];
