@@ -1146,24 +1146,31 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
             TCH_CK(e, cudaGetLastError());
         }
 
-        if (query_maps) {  // groups as the new profiles' rare counts read them
+        if (query_maps) {
+            // groups as the new profiles' rare counts read them, and bit columns for
+            // the smallest batches, each when it takes at most a quarter of the free
+            // memory: a set of many alleles and windows may have tables of gigabytes,
+            // and every batch can go without (k_rare.cu, the tile pass)
+            const char* force = getenv("TCH_FORCE_GROUP_SEARCH");  // test hook: as if the tables did not fit
             const int windows = query_windows(n);
             const size_t entries = off_h[L] * (size_t)windows + 1;
-            TCH_CK(e, dalloc(&wpos, entries, &out->bytes));
-            window_kernel<<<grid_for(entries, sms), 256>>>(goff_d, sorted, off_h[L], windows, wpos);
-            TCH_CK(e, cudaGetLastError());
-            TCH_CK(e, dalloc(&sorted16, n_members + 8, &tmp_bytes));  // the last piece is loaded whole
-            narrow_members_kernel<<<grid_for(std::max<size_t>(n_members, 1), sms), 256>>>(sorted, n_members, sorted16);
-            TCH_CK(e, cudaGetLastError());
-            // bit columns for the smallest batches, when they leave most of the memory free
-            const size_t words = up((size_t)n, 1024) / 32, columns = (size_t)D + L;
             TCH_CK(e, free_memory(device, &freeb));
-            if (columns * words * 4 <= freeb / 4) {
-                TCH_CK(e, dalloc(&out->bits, columns * words, &out->bytes));
-                out->bit_words = words;
-                bit_columns_kernel<<<dim3((unsigned)((words + 7) / 8), (unsigned)((L + 31) / 32)), 256>>>(
-                    out->x, n, L, cnt_off_d, col_d, base_d, words, out->bits);
+            if (entries * 4 + (n_members + 8) * 2 <= freeb / 4 && !(force && force[0] == '1')) {
+                TCH_CK(e, dalloc(&wpos, entries, &out->bytes));
+                window_kernel<<<grid_for(entries, sms), 256>>>(goff_d, sorted, off_h[L], windows, wpos);
                 TCH_CK(e, cudaGetLastError());
+                TCH_CK(e, dalloc(&sorted16, n_members + 8, &tmp_bytes));  // the last piece is loaded whole
+                narrow_members_kernel<<<grid_for(std::max<size_t>(n_members, 1), sms), 256>>>(sorted, n_members, sorted16);
+                TCH_CK(e, cudaGetLastError());
+                TCH_CK(e, free_memory(device, &freeb));
+                const size_t words = up((size_t)n, 1024) / 32, columns = (size_t)D + L;
+                if (columns * words * 4 <= freeb / 4) {
+                    TCH_CK(e, dalloc(&out->bits, columns * words, &out->bytes));
+                    out->bit_words = words;
+                    bit_columns_kernel<<<dim3((unsigned)((words + 7) / 8), (unsigned)((L + 31) / 32)), 256>>>(
+                        out->x, n, L, cnt_off_d, col_d, base_d, words, out->bits);
+                    TCH_CK(e, cudaGetLastError());
+                }
             }
         }
         mark("rare groups");
@@ -1195,7 +1202,7 @@ int encode_on_device(int device, int n, int L, const uint64_t* d_calls, int tau_
             out->n_rare = (size_t)n_rare_pairs;
             out->cnt_off = cnt_off_d;
             out->goff = goff_d;
-            out->members = query_maps ? nullptr : sorted;  // freed with the rest
+            out->members = query_maps && wpos ? nullptr : sorted;  // in two bytes: freed with the rest
             out->members16 = sorted16;
             out->mpos = mpos;
             out->bytes += ((size_t)L + 1) * 8 + (off_h[L] + 1) * 8 + n_members * (sorted16 ? 2 : 4) + (size_t)n * L * 4;

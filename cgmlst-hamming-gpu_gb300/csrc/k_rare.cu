@@ -452,7 +452,12 @@ __global__ void __launch_bounds__(T, 1024 / T)
 // the windows' CTAs overlap: five of them on an SM.  701 profiles against 200 000
 // x 1 142 (tau 4 096): 0.35 ms; one CTA per profile with four passes of 65 536
 // columns, two binary searches per locus in each, took 0.67.
+// Databases without the window entries (they did not fit) keep the members in four
+// bytes, and a run's ends are found by binary search (WINDOWS false): 64 profiles
+// against 20 000 x 3 016 and 200 000 x 1 142 take 0.304 and 0.500 ms in the call,
+// with the entries 0.230 and 0.437.
 constexpr int QT = 256;
+template <bool WINDOWS>
 __global__ void __launch_bounds__(QT, 5)
     rare_query_kernel(const RareGroups g, const uint32_t* __restrict__ xq, uint16_t* __restrict__ R, size_t ldr,
                       int cend) {
@@ -464,7 +469,8 @@ __global__ void __launch_bounds__(QT, 5)
     const int wb = w * kQueryWindow, nq = (min(cend, wb + kQueryWindow) - wb) >> 3;
     for (int q = tid; q < nq; q += QT) counters[q] = make_uint4(0, 0, 0, 0);
     __syncthreads();
-    const Counters c = window_counters(counters);
+    const Counters c = WINDOWS ? window_counters(counters) : counters_at(counters, wb);
+    constexpr uint32_t G = WINDOWS ? kPiece<uint16_t> : kPiece<uint32_t>;
     uint2* run = runs[warp];
     for (int k0 = 32 * warp; k0 < g.L; k0 += QT) {
         const int k = k0 + lane;
@@ -472,12 +478,20 @@ __global__ void __launch_bounds__(QT, 5)
         if (k < g.L) {
             const uint32_t a = __ldg(xq + (size_t)r * g.L + k);
             if (a && a != kNovelRank) {  // empty for an allele that is frequent in the set
-                const uint32_t* e = g.wpos + (__ldg(g.cnt_off + k) + a) * (uint64_t)g.windows + w;
-                lo = __ldg(e);
-                hi = __ldg(e + 1);
+                const uint64_t slot = __ldg(g.cnt_off + k) + a;
+                if (WINDOWS) {
+                    const uint32_t* e = g.wpos + slot * (uint64_t)g.windows + w;
+                    lo = __ldg(e);
+                    hi = __ldg(e + 1);
+                } else {
+                    const uint64_t end = __ldg(g.goff + slot + 1);
+                    const uint64_t first = lower_bound_m(g.members, __ldg(g.goff + slot), end, (uint32_t)wb);
+                    lo = (uint32_t)first;
+                    hi = (uint32_t)lower_bound_m(g.members, first, end, (uint32_t)wb + kQueryWindow);
+                }
             }
         }
-        const uint32_t pieces = hi > lo ? (hi - 1) / 8 - lo / 8 + 1 : 0;
+        const uint32_t pieces = hi > lo ? (hi - 1) / G - lo / G + 1 : 0;
         uint32_t inc = pieces;  // inclusive scan
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
@@ -487,10 +501,11 @@ __global__ void __launch_bounds__(QT, 5)
         const uint32_t total = __shfl_sync(FULL, inc, 31);
         const unsigned has = __ballot_sync(FULL, pieces > 0);
         __syncwarp();  // the previous runs' readers
-        if (pieces) run[__popc(has & ((1u << lane) - 1u))] = make_uint2((inc - pieces) << 3 | ((hi - 1) & 7u), lo);
+        if (pieces) run[__popc(has & ((1u << lane) - 1u))] = make_uint2((inc - pieces) << 3 | ((hi - 1) % G), lo);
         if (lane == 0) run[__popc(has)] = make_uint2(total << 3, 0);
         __syncwarp();
-        walk_pieces<uint16_t>(c, run, __popc(has), 0, total, g.members16, lane);
+        if (WINDOWS) walk_pieces<uint16_t>(c, run, __popc(has), 0, total, g.members16, lane);
+        else walk_pieces<uint32_t>(c, run, __popc(has), 0, total, g.members, lane);
     }
     __syncthreads();
     uint4* dst = reinterpret_cast<uint4*>(R + (size_t)r * ldr + wb);
@@ -716,11 +731,12 @@ cudaError_t launch_rare_dense(const RareGroups& g, int r0, int rows, uint16_t* R
 cudaError_t launch_rare_query(const RareGroups& g, const uint32_t* xq, int m, uint16_t* R, size_t ldr,
                               cudaStream_t st) {
     const size_t width = up((size_t)std::max(g.n, 1), kRareDenseAlign);
-    if (ldr < width || (ldr & 7) || ((uintptr_t)R & 15) || !g.wpos || g.windows != query_windows(g.n))
-        return cudaErrorInvalidValue;
+    if (ldr < width || (ldr & 7) || ((uintptr_t)R & 15)) return cudaErrorInvalidValue;
+    if (g.wpos ? g.windows != query_windows(g.n) || !g.members16 : !g.goff || !g.members) return cudaErrorInvalidValue;
+    const auto kernel = g.wpos ? rare_query_kernel<true> : rare_query_kernel<false>;
     for (int r0 = 0; r0 < m; r0 += 65535) {  // the grid's second dimension
-        const dim3 grid(g.windows, std::min(65535, m - r0));
-        rare_query_kernel<<<grid, QT, 0, st>>>(g, xq + (size_t)r0 * g.L, R + (size_t)r0 * ldr, ldr, (int)width);
+        const dim3 grid(query_windows(g.n), std::min(65535, m - r0));
+        kernel<<<grid, QT, 0, st>>>(g, xq + (size_t)r0 * g.L, R + (size_t)r0 * ldr, ldr, (int)width);
     }
     return cudaGetLastError();
 }

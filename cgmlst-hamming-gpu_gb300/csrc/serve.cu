@@ -471,6 +471,8 @@ int db_query(tch_db* db, int m, const uint64_t* qcalls, uint16_t* h_qdb, uint16_
             }
             RareGroups g;
             g.cnt_off = enc.cnt_off;
+            g.goff = enc.goff;
+            g.members = enc.members;
             g.members16 = enc.members16;
             g.wpos = enc.wpos;
             g.windows = query_windows(n);

@@ -294,6 +294,7 @@ struct RareGroups {
     // For new profiles (databases; members16 modulo 65 536): wpos[q * windows + w] =
     // the first member of slot q's group at or after row w * kQueryWindow, and the
     // next entry where the window's members end (slot q + 1's first for the last).
+    // Null when the table did not fit: the groups are searched in members.
     const uint32_t* wpos = nullptr;
     int windows = 0;
 };
