@@ -79,9 +79,11 @@ __device__ __forceinline__ uint32_t lane16(const uint4& h, int e) {
 //
 // Bound by the one read of the matrix.  40 009 profiles, k = 10: 0.84 ms
 // for the call; the radix select before it (a CTA per row, three reads of the
-// row, a warp match per value in two of them) took 9.5 ms.  A row whose
-// distances fall from column to column makes every value a hit: 32 values then
-// cost one merge of about 200 instructions, still below that.
+// row, a warp match per value in two of them) took 9.5 ms.  In a row whose
+// distances fall from column to column every value is a hit, and 32 of them cost a
+// merge of about 200 instructions, so a block after a crowded one is bounded by
+// its own values first: 60 000 such rows take 5.0 ms, 28.4 without that bound, 10.9
+// in the radix select.
 
 constexpr int kNbrWarps = kNbrThreads / 32;
 
@@ -124,7 +126,8 @@ __device__ __forceinline__ unsigned long long nearest_keys(const uint4* __restri
                                                            uint32_t thr, unsigned long long* buf, int lane) {
     const int nq = (n + 7) >> 3;
     unsigned long long list = kNoEdge;
-    uint32_t held = 0;  // keys in the buffer
+    uint32_t held = 0;    // keys in the buffer
+    bool crowded = true;  // bound the next block by its own values first
     for (int q0 = 0; q0 < nq; q0 += 128) {
         uint4 h[4];
 #pragma unroll
@@ -132,14 +135,15 @@ __device__ __forceinline__ unsigned long long nearest_keys(const uint4* __restri
             const int q = q0 + 32 * u + lane;
             h[u] = q < nq ? __ldcs(row + q) : make_uint4(FULL, FULL, FULL, FULL);
         }
-        if (q0 == 0) {
-            // a first bound: the k-th smallest of the 32 lanes' smallest valid values
+        if (crowded) {
+            // a bound from the block alone, in the first one and after one of many
+            // hits: the k-th smallest of the 32 lanes' smallest valid values
             uint32_t m = 0xFFFFu;
 #pragma unroll
             for (int u = 0; u < 4; u++)
 #pragma unroll
                 for (int e = 0; e < 8; e++) {
-                    const int j = 8 * (32 * u + lane) + e;
+                    const int j = 8 * (q0 + 32 * u + lane) + e;
                     const uint32_t w = lane16(h[u], e);
                     if (w < m && j < n && j != i && (!OUT || __ldg(comp + j) != own)) m = w;
                 }
@@ -149,6 +153,7 @@ __device__ __forceinline__ unsigned long long nearest_keys(const uint4* __restri
         // every key in the list or the buffer comes from smaller columns, except
         // those of this block: a later value at the k-th distance is no hit
         const uint32_t start = thr;
+        int merges = 0;
 #pragma unroll
         for (int u = 0; u < 4; u++) {
             const uint32_t m2 = __vminu2(__vminu2(h[u].x, h[u].y), __vminu2(h[u].z, h[u].w));
@@ -173,6 +178,7 @@ __device__ __forceinline__ unsigned long long nearest_keys(const uint4* __restri
                 held += __popc(who);
                 if (held >= 32) {
                     held -= 32;
+                    merges++;
                     __syncwarp();
                     list = merge_keys(list, buf[held + lane], lane);
                     __syncwarp();
@@ -183,6 +189,7 @@ __device__ __forceinline__ unsigned long long nearest_keys(const uint4* __restri
         }
         const uint32_t kth = key_distance(__shfl_sync(FULL, list, k - 1));
         thr = min(thr, kth);
+        crowded = merges > 1;
     }
     if (held) {
         __syncwarp();

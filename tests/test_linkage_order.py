@@ -1,0 +1,88 @@
+"""Rows whose distances fall from column to column: nearly every value is nearer
+than all before it, so the running bound of the nearest-column pass must come
+from the columns at hand, not only from the list so far."""
+import numpy as np
+import oracle
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def fill(torch, H):
+    n = len(H)
+    ld = (n + 7) // 8 * 8
+    full = np.zeros((n, ld), np.uint16)
+    full[:, :n] = H
+    return torch.from_numpy(full.view(np.int16)).cuda(), ld
+
+
+@pytest.mark.parametrize("n", [1025, 2500, 4100])
+@pytest.mark.parametrize("shape", ["steps", "saw", "valley", "lanes", "low", "mixed"])
+def test_neighbors_of_falling_rows(pkg, n, shape):
+    """Falling in steps (ties), in teeth that restart at odd columns, towards the
+    diagonal, in some lanes' columns only, below a low first block, and with
+    random rows between; k at both ends of its range and between."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(n)
+    j, i = np.arange(n)[None, :], np.arange(n)[:, None]
+    if shape == "steps":
+        H = 60000 - j // 7 * 5 + 0 * i
+    elif shape == "saw":
+        H = 60000 - (j + 37 * i) % 1237
+    elif shape == "valley":
+        H = np.abs(i - j) * 9
+    elif shape == "lanes":
+        H = np.where(j // 8 % 32 < 9, 60000 - j, 65535) + 0 * i
+    elif shape == "low":
+        H = np.where(j < 1024, 30, 60000 - j * 14) + 0 * i
+    else:
+        H = np.where(i % 2 == 0, 60000 - j * 13, rng.integers(0, 65536, size=(n, n)))
+    H = np.clip(H, 0, 65535).astype(np.uint16)
+    d, ld = fill(torch, H)
+    for k in (1, 9, 10, 32):
+        idx, dist = pkg.neighbors_device(d.data_ptr(), ld, n, k)
+        wi, wd = oracle.neighbors(H, k)
+        np.testing.assert_array_equal(idx, wi)
+        np.testing.assert_array_equal(dist, wd)
+
+
+@pytest.mark.parametrize("n", [1025, 2049])
+@pytest.mark.parametrize("shape", ["last", "first", "far"])
+def test_tree_of_falling_rows(pkg, n, shape):
+    """Distances that fall with the larger index, with the smaller, and with the
+    gap between the two."""
+    torch = pytest.importorskip("torch")
+    j, i = np.arange(n)[None, :], np.arange(n)[:, None]
+    H = 40000 - {"last": np.maximum(i, j), "first": np.minimum(i, j), "far": np.abs(i - j)}[shape]
+    H = H.astype(np.uint16)
+    d, ld = fill(torch, H)
+    u, v, w = pkg.mst_device(d.data_ptr(), ld, n)
+    eu, ev, ew = oracle.mst(H)
+    np.testing.assert_array_equal(u, eu)
+    np.testing.assert_array_equal(v, ev)
+    np.testing.assert_array_equal(w, ew)
+
+
+def test_falling_rows_cost_little_more(pkg):
+    """20 000 profiles: falling rows took 8 times as long as random ones when every
+    value of theirs was merged, and as long in the radix select before it."""
+    torch = pytest.importorskip("torch")
+    n = 20000
+    st = torch.cuda.Stream()
+    best = []
+    for falling in (False, True):
+        if falling:
+            H = (-1 - torch.arange(n, device="cuda")).to(torch.int16)[None, :].expand(n, n).contiguous()
+        else:
+            H = torch.randint(-32768, 32767, (n, n), dtype=torch.int16, device="cuda")
+        times = []
+        for _ in range(7):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            torch.cuda.synchronize()
+            a.record(st)
+            pkg.neighbors_device(H.data_ptr(), n, n, 10, st.cuda_stream)
+            b.record(st)
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        best.append(min(times))
+    assert best[1] < 5 * best[0], best
