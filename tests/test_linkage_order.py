@@ -1,6 +1,8 @@
-"""Rows whose distances fall from column to column: nearly every value is nearer
-than all before it, so the running bound of the nearest-column pass must come
-from the columns at hand, not only from the list so far."""
+"""Orders that the kernels behind the tree and the neighbours find hard: rows whose
+distances fall from column to column (nearly every value is nearer than all
+before it, so the running bound of the nearest-column pass must come from the
+columns at hand, not only from the list so far), and many tree edges of one
+distance."""
 import numpy as np
 import oracle
 import pytest
@@ -86,3 +88,30 @@ def test_falling_rows_cost_little_more(pkg):
             times.append(a.elapsed_time(b))
         best.append(min(times))
     assert best[1] < 5 * best[0], best
+
+
+@pytest.mark.parametrize("sizes", [[4096], [4097], [5000, 4096, 700], [300, 9000, 1, 4097, 20]])
+def test_edges_of_one_distance_in_order(pkg, sizes):
+    """Trees that are paths through the profiles in random order, so that many edges
+    of one distance come in no order: numbers of them around the chunks that are
+    sorted and the count from which they are, several such distances beside one
+    another."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(sum(sizes))
+    m = sum(sizes)
+    n = m + 1
+    perm = rng.permutation(n)
+    w = np.repeat(np.arange(1, len(sizes) + 1) * 3, sizes).astype(np.int64)
+    ld = (n + 7) // 8 * 8
+    d = torch.full((n, ld), 900, dtype=torch.int16, device="cuda")
+    a, b = torch.from_numpy(perm[:-1]).cuda(), torch.from_numpy(perm[1:]).cuda()
+    wt = torch.from_numpy(w).to(torch.int16).cuda()
+    d[a, b] = wt
+    d[b, a] = wt
+    torch.cuda.synchronize()
+    lo, hi = np.minimum(perm[:-1], perm[1:]), np.maximum(perm[:-1], perm[1:])
+    order = np.lexsort((hi, lo, w))
+    u, v, got = pkg.mst_device(d.data_ptr(), ld, n)
+    np.testing.assert_array_equal(u, lo[order])
+    np.testing.assert_array_equal(v, hi[order])
+    np.testing.assert_array_equal(got, w[order])
