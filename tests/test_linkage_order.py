@@ -90,12 +90,13 @@ def test_falling_rows_cost_little_more(pkg):
     assert best[1] < 5 * best[0], best
 
 
-@pytest.mark.parametrize("sizes", [[4096], [4097], [5000, 4096, 700], [300, 9000, 1, 4097, 20]])
+@pytest.mark.parametrize("sizes", [[4096], [4097], [5000, 4096, 700], [300, 9000, 1, 4097, 20], [1022], [1023], [1024],
+                                   [1025], [2, 1030]])
 def test_edges_of_one_distance_in_order(pkg, sizes):
     """Trees that are paths through the profiles in random order, so that many edges
     of one distance come in no order: numbers of them around the chunks that are
     sorted and the count from which they are, several such distances beside one
-    another."""
+    another, and around the size up to which the host orders them."""
     torch = pytest.importorskip("torch")
     rng = np.random.default_rng(sum(sizes))
     m = sum(sizes)
