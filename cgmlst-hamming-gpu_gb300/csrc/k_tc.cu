@@ -56,9 +56,9 @@
 //     through vector registers;
 // raster groups of 16 and the smaller shared-memory configuration did the rest.
 //
-// Every mbarrier wait is bounded (about 2 s of %globaltimer); on a timeout the
-// CTA records DEVERR_TIMEOUT, stops issuing work, drains what it issued,
-// frees its TMEM and returns.
+// Every mbarrier wait is bounded (about 2 s of %globaltimer, none of it spent on the
+// launch before); on a timeout the CTA records DEVERR_TIMEOUT, stops issuing work,
+// drains what it issued, frees its TMEM and returns.
 
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -350,7 +350,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
             uint32_t issued_ph[STAGES];
             for (int q = 0; q < STAGES; q++) issued[q] = 0, issued_ph[q] = 0;
             int last_job = -1;  // MULTI: the job whose maps this thread has acquired
-            for (int t = t_begin; ok && t < t_end; t += t_step) {
+            for (int t = t_begin, nth = 0; ok && t < t_end; t += t_step, nth++) {
+                if (nth == 2) grid_wait();  // as the issuer
                 int bi, bj, y_a, y_b, kblocks;
                 const CUtensorMap* ma = maps.a;
                 const CUtensorMap* mb = maps.b;
@@ -422,7 +423,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
             bool ready = false;  // stage s is known to hold its operands
             bool ok = mbar_wait(scales, 0, abort_flag, p.err);
             tc_fence_after();
-            for (int t = t_begin; ok && t < t_end; t += t_step) {
+            for (int t = t_begin, nth = 0; ok && t < t_end; t += t_step, nth++) {
+                // the first two tiles have an accumulator each; the third waits for
+                // the epilogue, and so for the launch before, however long that
+                // takes: the bound of the waits begins when it is done
+                if (nth == 2) grid_wait();
                 const int kblocks = MULTI ? p.jobs[__ldg(&p.tiles[t].x)].kblocks : p.kblocks;
                 if (!mbar_wait(&tempty[acc], aph ^ 1, abort_flag, p.err)) { ok = false; break; }
                 tc_fence_after();

@@ -23,6 +23,43 @@ def test_rare_counts_are_not_read_through_the_read_only_path():
     assert not re.search(r"__restrict__\s+rdense|ld\.global\.nc", text)
 
 
+def test_bounded_waits_do_not_cover_the_launch_before():
+    """The epilogue waits for the counts' launch, without a limit; the roles whose
+    limited waits hang on the epilogue (producer and issuer, from their third
+    tile on) wait for that launch first, so that a long one is no timeout."""
+    with open(os.path.join(ROOT, PKG_NAME, "csrc", "k_tc.cu")) as f:
+        text = re.sub(r"//[^\n]*", "", f.read())
+    body = text[text.index("tc_stripe_kernel("):text.index("cuTensorMapEncodeTiled", text.index("tc_stripe_kernel("))]
+    loops = body.split("for (int t = t_begin")[1:]
+    assert len(loops) == 3  # producer, issuer, epilogue
+    for loop in loops[:2]:
+        head = loop[:loop.index("mbar_wait")]
+        assert re.search(r"if \(nth == 2\) grid_wait\(\);", head)
+    assert "grid_wait();" in body[:body.index("for (int t = t_begin; t < t_end")]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [1, 32, 300])
+def test_few_rows_against_long_counts(pkg, rows):
+    """Stripes of fewer rows than SMs, whose tile pass starts at once beside the
+    counts and takes several tiles per CTA pair while it waits for them."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(rows)
+    n, L = 60000, 60
+    A = rng.integers(0, 4, size=(n, L)).astype(np.uint64)
+    ld = (n + 7) // 8 * 8
+    with pkg.Solver.from_calls(A, tau=65536) as s:
+        for r0 in (0, 3000):
+            out = torch.zeros((rows, ld), dtype=torch.int16, device="cuda:0")
+            s.stripe(r0, rows, out.data_ptr(), ld, torch.cuda.current_stream().cuda_stream)
+            s.check()
+            got = out.cpu().numpy().view(np.uint16)
+            for r in range(0, rows, max(1, rows // 5)):
+                i = r0 + r
+                want = ((A[i + 1:] != A[i]) & (A[i + 1:] != 0) & (A[i] != 0)).sum(1)
+                np.testing.assert_array_equal(got[r, r + 1:n - r0], want)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("n", [300, 1301])
 def test_solves_in_turn_through_one_block(pkg, n):
