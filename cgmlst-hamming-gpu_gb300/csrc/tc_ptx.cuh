@@ -112,6 +112,14 @@ __device__ __forceinline__ void tma_load_2d_pair(const CUtensorMap* map, uint32_
         "l"((uint64_t)map), "r"(x), "r"(y), "r"(bar)
         : "memory");
 }
+// The same for a CTA by itself.
+__device__ __forceinline__ void tma_load_2d(const CUtensorMap* map, uint32_t bar, void* dst, int x, int y) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+            smem_u32(dst)),
+        "l"((uint64_t)map), "r"(x), "r"(y), "r"(bar)
+        : "memory");
+}
 // The MMAs issued so far by this thread done: one arrival on `bar` of this CTA ...
 __device__ __forceinline__ void tc_commit_pair_local(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))

@@ -243,10 +243,14 @@ struct TcBatchItem {
 struct TcBatchPlan {
     void* d_jobs = nullptr;
     void* d_maps = nullptr;
-    void* d_tiles = nullptr;  // (job, tile), by CTA pair
-    void* d_first = nullptr;  // every pair's first tile
+    // Two launches, either of which may be empty: tiles on CTA pairs, and tiles of
+    // sets of one row block on CTAs by themselves.
+    struct Part {
+        void* d_tiles = nullptr;  // (job, tile), list by list
+        void* d_first = nullptr;  // every list's first tile
+        int lists = 0;            // pairs, or CTAs
+    } part[2];
     int njobs = 0, num_tiles = 0;
-    int grid = 0;  // CTAs of the launch (at most num_sms)
     int* err = nullptr;
 };
 cudaError_t tc_batch_prepare(const std::vector<TcBatchItem>& items, int num_sms, TcBatchPlan* plan, int* err);
