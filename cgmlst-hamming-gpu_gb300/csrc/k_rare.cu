@@ -14,9 +14,9 @@
 // partner adds 1 with a shared atomic, and the finished row is written out with
 // coalesced 16-byte stores.  Triangle solves read the rows' partner runs as the
 // encoder laid them out (rare_runs_kernel); where there are none (stripes wider
-// than one pass) the runs of up to 2048 loci are found per locus,
-// laid end to end by a block-wide scan of their lengths and cut into 32 equal
-// parts, one per warp (rare_dense_kernel).
+// than one pass) or the groups are too crowded for them (launch_rare_dense), the
+// runs of two loci per thread are found at a time, laid end to end by a block-wide
+// scan of their lengths and cut into equal parts, one per warp (rare_dense_kernel).
 //
 // What bounds rare_runs_kernel: the shared atomics.  Random columns put 3.4
 // lanes of a warp on one bank, so an atomic takes 3.4 of the L1's data cycles,
@@ -636,6 +636,11 @@ void rare_batch_release(RareBatchPlan* plan) {
 // system's).
 constexpr int runs_room(int per_sm) { return (227 * 1024) / per_sm - 1024; }
 
+// Narrow rows, in columns: a CTA of NT (128) threads each, so that many rows' chains
+// of dependent steps overlap (5 000 profiles, tau 64: 0.039 ms, with 512 threads
+// 0.060; from 8 192 columns on the two are alike).
+constexpr int kNarrow = 8192;
+
 // One launch of rare_runs_kernel over rows [ra, rb) of the stripe: `per_sm` CTAs
 // of T threads on an SM, as many of them as hold the widest row's counters; the
 // runs staged at a time take what is left, up to a row's most.
@@ -661,10 +666,6 @@ static cudaError_t launch_rare_runs(const RareGroups& g, int r0, int rows, uint1
     const int width = (int)up((size_t)(g.n - r0), kRareDenseAlign), cend = r0 + width;
     // widest row that leaves room for two CTAs on an SM
     constexpr int kWide = (runs_room(2) - runs_smem<512>(0, kMinCap)) / 2 / kRareDenseAlign * kRareDenseAlign;
-    // narrow rows: a CTA of NT (128) threads each, so that many rows' chains of
-    // dependent steps overlap (5 000 profiles, tau 64: 0.039 ms, with 512 threads
-    // 0.060; from 8 192 columns on the two are alike)
-    constexpr int kNarrow = 8192;
     // sets with more than 32 768 rare pairs per row keep many warps per row busy:
     // 256 threads a row, a CTA each, up to 20 480 columns (10 000 x 1 142, tau 1 024,
     // 91 000 pairs per row: 0.552 ms, with 512 and 128 threads 0.658; 12 011
@@ -710,21 +711,31 @@ cudaError_t launch_rare_dense(const RareGroups& g, int r0, int rows, uint16_t* R
     if (rows <= 0) return cudaSuccess;
     const size_t width = up((size_t)(g.n - r0), kRareDenseAlign);
     if (ldr < width || (ldr & 7) || ((uintptr_t)R & 15)) return cudaErrorInvalidValue;
-    // every row's precomputed runs, where the widest row fits one counter pass
-    if (g.roff && width <= (size_t)2 * RD_WORDS)
+    // Every row's precomputed runs, where the widest row fits one counter pass.  Not
+    // with four-byte members in groups so large that a row has more than eight rare
+    // pairs per column: lanes on consecutive members of such runs meet fewer banks
+    // twice than lanes on pieces of four (70 001 x 200, tau 65 536, 13 pairs per
+    // column: the last 8 192 rows 0.48 and 0.59 ms, 20 480 3.35 and 3.48; x 1 142, tau
+    // 4 096, 4.7 pairs: 0.36 and 0.29, 1.95 and 1.46).
+    const bool crowded = !g.members16 && g.pairs / 8 > (size_t)g.n * g.n;
+    if (g.roff && width <= (size_t)2 * RD_WORDS && !crowded)
         return g.members16 ? launch_rare_runs<uint16_t>(g, r0, rows, R, ldr, sms, st)
                            : launch_rare_runs<uint32_t>(g, r0, rows, R, ldr, sms, st);
     static bool attrs[kMaxDevices] = {};  // once per device (also keeps it out of graph captures)
     bool& attr = attrs[current_device()];
     if (!attr) {
-        const cudaError_t e = cudaFuncSetAttribute(rare_dense_kernel<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   rd_smem<1024>(RD_WORDS));
+        const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
+        cudaError_t e = cudaFuncSetAttribute(rare_dense_kernel<1024>, at, rd_smem<1024>(RD_WORDS));
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(rare_dense_kernel<NT>, at, rd_smem<NT>(kNarrow / 2));
         if (e != cudaSuccess) return e;
         attr = true;
     }
     const int cwords = counter_words(width);
-    rare_dense_kernel<1024><<<std::max(1, std::min(rows, sms)), 1024, rd_smem<1024>(cwords), st>>>(
-        g, r0, rows, R, ldr, r0 + (int)width, cwords);
+    if (width <= (size_t)kNarrow)  // a CTA of 128 threads per row, as in bands of runs
+        rare_dense_kernel<NT><<<rows, NT, rd_smem<NT>(cwords), st>>>(g, r0, rows, R, ldr, r0 + (int)width, cwords);
+    else
+        rare_dense_kernel<1024><<<std::max(1, std::min(rows, sms)), 1024, rd_smem<1024>(cwords), st>>>(
+            g, r0, rows, R, ldr, r0 + (int)width, cwords);
     return cudaGetLastError();
 }
 
