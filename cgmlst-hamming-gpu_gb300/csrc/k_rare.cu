@@ -27,6 +27,7 @@
 // 1 024-thread CTA per SM took every row; 0.6 ms of it is the 4 GB block.
 
 #include <climits>
+#include <cstdlib>
 
 #include "rare_walk.cuh"
 #include "tch_internal.cuh"
@@ -640,6 +641,14 @@ constexpr int runs_room(int per_sm) { return (227 * 1024) / per_sm - 1024; }
 // of dependent steps overlap (5 000 profiles, tau 64: 0.039 ms, with 512 threads
 // 0.060; from 8 192 columns on the two are alike).
 constexpr int kNarrow = 8192;
+// TCH_RARE_SMALL_ROWS: only for stripes of fewer rows than this.
+static bool narrow_rows(int rows) {
+    static const int limit = [] {
+        const char* v = getenv("TCH_RARE_SMALL_ROWS");
+        return v ? std::max(0, atoi(v)) : INT_MAX;
+    }();
+    return rows < limit;
+}
 
 // One launch of rare_runs_kernel over rows [ra, rb) of the stripe: `per_sm` CTAs
 // of T threads on an SM, as many of them as hold the widest row's counters; the
@@ -694,7 +703,7 @@ static cudaError_t launch_rare_runs(const RareGroups& g, int r0, int rows, uint1
             e = launch_runs<1024, M>(g, r0, ra, rb, R, ldr, cend, 1, true, sms, st);
         } else if ((rb = wider(28672)) > ra) {
             e = launch_runs<512, M>(g, r0, ra, rb, R, ldr, cend, 2, true, sms, st);
-        } else if ((rb = wider(heavy ? kHeavyWidth : kNarrow)) > ra) {
+        } else if ((rb = wider(heavy ? kHeavyWidth : narrow_rows(rows) ? kNarrow : 0)) > ra) {
             e = launch_runs<512, M>(g, r0, ra, rb, R, ldr, cend, 3, true, sms, st);
         } else {
             rb = rows;
@@ -731,7 +740,7 @@ cudaError_t launch_rare_dense(const RareGroups& g, int r0, int rows, uint16_t* R
         attr = true;
     }
     const int cwords = counter_words(width);
-    if (width <= (size_t)kNarrow)  // a CTA of 128 threads per row, as in bands of runs
+    if (width <= (size_t)kNarrow && narrow_rows(rows))  // a CTA of 128 threads per row, as in bands of runs
         rare_dense_kernel<NT><<<rows, NT, rd_smem<NT>(cwords), st>>>(g, r0, rows, R, ldr, r0 + (int)width, cwords);
     else
         rare_dense_kernel<1024><<<std::max(1, std::min(rows, sms)), 1024, rd_smem<1024>(cwords), st>>>(
