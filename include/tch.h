@@ -45,8 +45,9 @@ typedef void (*tch_cb)(void* ctx, int r0, int rows, size_t w, const uint16_t* st
 /* Number of CUDA devices; 0 on error.  Replaces tch.cu:68-71. */
 int tch_device_count(void);
 
-/* Free device memory in bytes after making `device` current; 0 on error.
- * Replaces tch.cu:73-77. */
+/* Free device memory in bytes after making `device` current, with what the library
+ * keeps unused and gives back when it is needed; 0 on error.  Replaces
+ * tch.cu:73-77. */
 size_t tch_free_vram(int device);
 
 /* The whole distance matrix, upper triangle, in stripes of S rows.
