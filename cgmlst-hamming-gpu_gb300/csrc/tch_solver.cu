@@ -433,6 +433,7 @@ fail:
     if (d_calls) cudaFreeAsync(d_calls, 0);
     if (d_ranks) cudaFreeAsync(d_ranks, 0);
     cudaStreamSynchronize(0);
+    free_device_encoding(&enc);
     solver_free(s);
     return 1;
 }
